@@ -33,7 +33,7 @@ __device__ __forceinline__ uint64_t le64_of(uint32_t be_lo, uint32_t be_hi) {
 
 // one keystream block of the CPU mapping from round keys in global memory (rare paths)
 __device__ __noinline__ void ctr_block_g(uint32_t (&W)[4], uint32_t ctr, const uint32_t *__restrict__ rkg,
-                                         const AesCtx &c) {
+                                         AesCtx c) {
   uint32_t rk[60];
 #pragma unroll
   for (int i = 0; i < 60; ++i) rk[i] = __ldg(rkg + i);
@@ -46,7 +46,7 @@ __device__ __noinline__ void ctr_block_g(uint32_t (&W)[4], uint32_t ctr, const u
 // src/gauss.c:578-703, regenerating blocks as needed
 template <int SIG>
 __device__ __noinline__ void uniform_slow(uint32_t *y, int ystride, uint32_t cb, const uint32_t *__restrict__ rkg,
-                                          const AesCtx &c, uint32_t *status) {
+                                          AesCtx c, uint32_t *status) {
   int w = 0, have_blk = -1;
   uint32_t W[4] = {0, 0, 0, 0};
   for (int j = 0; j < 8; ++j) {
@@ -71,49 +71,76 @@ __device__ __noinline__ void uniform_slow(uint32_t *y, int ystride, uint32_t cb,
   }
 }
 
-// 126-bit CDT compare of the CPU S3 for one lane whose high word ties a table entry: the
-// low word (bytes 8 lane.. of r, or of r + 100 for lanes 4..7) is regenerated here
-__device__ __noinline__ uint32_t cdt_full_slow(int lane, uint64_t r2, uint32_t cb, const uint32_t *__restrict__ rkg,
-                                               const AesCtx &c) {
-  const int off = (lane < 4 ? 0 : 100) + 8 * (lane & 3);
-  uint32_t W[4], lo, hi;
-  ctr_block_g(W, cb + (uint32_t)(off >> 4), rkg, c);
-  const int w0 = (off >> 2) & 3;
-  lo = w0 == 0 ? W[0] : w0 == 1 ? W[1] : w0 == 2 ? W[2] : W[3];
-  const int off2 = off + 4;
-  if ((off2 >> 4) != (off >> 4)) ctr_block_g(W, cb + (uint32_t)(off2 >> 4), rkg, c);
-  const int w1 = (off2 >> 2) & 3;
-  hi = w1 == 0 ? W[0] : w1 == 1 ? W[1] : w1 == 2 ? W[2] : W[3];
-  return cdt_sample<true>(r2, (uint64_t)bswap32(lo) | ((uint64_t)bswap32(hi) << 32));
+// keystream word w (bytes 4w..4w+3, little-endian) of a refill
+__device__ __forceinline__ uint32_t refill_word(int w, uint32_t cb, const uint32_t *__restrict__ rkg,
+                                                AesCtx c) {
+  uint32_t W[4];
+  ctr_block_g(W, cb + (uint32_t)(w >> 2), rkg, c);
+  const int i = w & 3;
+  return bswap32(i == 0 ? W[0] : i == 1 ? W[1] : i == 2 ? W[2] : W[3]);
 }
 
-template <bool FULL>
-__device__ __forceinline__ uint32_t cdt_lane(int lane, uint64_t r2, uint32_t cb, const uint32_t *rkg,
-                                             const AesCtx &c) {
-  bool tie;
-  const uint32_t x = cdt_sample_hi(r2, tie);
-  if (FULL && tie) return cdt_full_slow(lane, r2, cb, rkg, c);
-  return x;
+// What a refill keeps of candidate ln beside z's low word: its accept bit (bit ln), bit 32 of z (bit
+// 8 + ln; |value| = z < 8K < 2^33), and bit 16 if an accepted z ever reaches 2^33.
+__device__ __forceinline__ uint32_t candidate_bits(int ln, bool b, uint64_t z, uint32_t k8) {
+  const uint32_t a = accept_final(b, z, (k8 >> ln) & 1u);
+  return (a << ln) | ((uint32_t)((z >> 32) & 1u) << (8 + ln)) | ((a & (uint32_t)((z >> 33) != 0)) << 16);
+}
+
+// The candidates of a refill that its top words left undecided (bits of `open`), again from their
+// full words: CDT words 8 + 2 lane, 9 + 2 lane and, for the 126-bit compare of the CPU S3, 2 lane, 1
+// + 2 lane; Bernoulli words 16 + 2 lane, 17 + 2 lane; exponent bytes in word 24 (all 25 words
+// further for lanes 4..7).  Rewrites their low words in cand[8] and returns `bits` with theirs
+// corrected.
+template <int SIG, bool FULL, int VAR>
+__device__ __noinline__ uint32_t refill_slow(uint32_t open, uint32_t k8, uint32_t cb,
+                                             const uint32_t *__restrict__ rkg, AesCtx c, double kinv,
+                                             uint32_t *cand, uint32_t bits, uint32_t *status) {
+  uint32_t y[8];
+  uniform_slow<SIG>(y, 1, cb, rkg, c, status);
+  for (; open; open &= open - 1) {
+    const int ln = __ffs(open) - 1, w = (ln < 4 ? 0 : 25) + 2 * (ln & 3);
+    uint64_t v[3];  // r1, r2, rm
+#pragma unroll 1
+    for (int i = 0; i < 3; ++i)
+      v[i] = refill_word(w + 8 * i, cb, rkg, c) | ((uint64_t)refill_word(w + 8 * i + 1, cb, rkg, c) << 32);
+    const uint32_t rexp = (refill_word(ln < 4 ? 24 : 49, cb, rkg, c) >> (8 * (ln & 3))) & 0xffu;
+    uint64_t z;
+    const bool b = candidate<SIG, VAR>(cdt_sample<FULL>(v[1], v[0]), y[ln], v[2], rexp, kinv, z);
+    cand[ln] = (uint32_t)z;
+    bits = (bits & ~(0x101u << ln)) | candidate_bits(ln, b, z, k8);
+  }
+  return bits;
 }
 
 // Blocks of one refill that the fast path reads (16-byte block b = bytes 16b..16b+15, word w
-// = bytes 4w..4w+3): 2, 3 (CDT high words of lanes 0..3, words 8..15), 4, 5, 6 (Bernoulli
-// words 16..24), 8..12 (CDT high words and Bernoulli words of lanes 4..7, words 33..49),
-// 12..14 (the first 10 uniform words from byte 200, words 50..59) and 17 (sign byte 280,
-// word 70): 13 of the refill's 24 blocks.  Blocks 0, 1, 7 hold only the low CDT words, which
-// S1/S2 never use and S3 uses only on ties; blocks 15 and 16 hold uniform words 60..67, needed
-// only when fewer than 8 of the first 10 words are accepted.  Both rare cases regenerate what
-// they need on their slow paths.
+// = bytes 4w..4w+3): 2, 3 (CDT words of lanes 0..3, words 8..15), 4, 5, 6 (Bernoulli words
+// 16..24), 8..12 (CDT and Bernoulli words of lanes 4..7, words 33..49), 12..14 (the first 10
+// uniform words from byte 200, words 50..59) and 17 (sign byte 280, word 70): 13 of the refill's
+// 24 blocks.  Of each 64-bit CDT and Bernoulli word the fast path needs the top half only (the
+// odd words of blocks 2..5, the even words of blocks 8..11), so 10 of the 13 blocks leave half of
+// their final round out: 80 of the refill's 2,576 table lookups.  The low halves, and blocks 0,
+// 1, 7 (the second CDT words, which only S3 uses), matter on ties; blocks 15 and 16 hold uniform
+// words 60..67, needed only when fewer than 8 of the first 10 words are accepted.  The rare
+// cases regenerate what they need on their slow paths.
 //
 // The blocks are computed in the order below and each is consumed as soon as it exists, so a
-// refill never buffers its keystream: the uniform words and the sign byte first (every
-// candidate needs its y and sign bit), then the exponent word of lanes 0..3, and from there
-// every CDT sample and every candidate the moment its last word arrives.  All live values
-// (the 8 y, the packed CDT samples, a few words carried to the next block, the outputs) are
-// registers; a buffered keystream had to live in local memory, whose traffic took 6% of the
-// L1 data pipe that the table lookups saturate and missed L1 on a third of its loads.
+// refill never buffers its keystream: the sign byte, the uniform words and the CDT words first,
+// then the Bernoulli words, two candidates at a time.  All live values (the 8 y, the packed CDT
+// samples, a few words carried to a later block, the outputs) are registers; a buffered
+// keystream had to live in local memory, whose traffic took 6% of the L1 data pipe that the
+// table lookups saturate and missed L1 on a third of its loads.
+//
+// The order also keeps the recomputations of the counter cache (aes.cuh) rare.  The 32 refills of a
+// warp start 24 counters apart from a multiple of 768, so in one lane the upper counter bits
+// change between blocks 15 and 16, in one between blocks 7 and 8, and in no other inside the
+// refill; a recomputation costs the whole warp 15 lookups.  Block 17 first and blocks 8..14 before
+// blocks 2..6 makes 3 of them per refill (5 to 7 in other orders).
 constexpr int kRefillBlocks = 13;
-__constant__ uint8_t c_refill_order[kRefillBlocks] = {12, 13, 14, 17, 6, 2, 3, 4, 5, 8, 9, 10, 11};
+__constant__ uint8_t c_refill_order[kRefillBlocks] = {17, 12, 13, 14, 8, 9, 10, 11, 6, 2, 3, 4, 5};
+// by step: bit s of kEvenWords / kOddWords -- words 0, 2 / words 1, 3 of that block are read
+constexpr uint32_t kEvenWords = 0x01ffu;  // blocks 17, 12, 13, 14, 8..11 and 6
+constexpr uint32_t kOddWords = 0x1e0eu;   // blocks 12, 13, 14 and 2..5
 
 constexpr int kCandThreads = 512;  // 1 CTA (128 KiB of tables) per SM; 128 registers per thread
 
@@ -134,38 +161,24 @@ __device__ __forceinline__ void uniform_step(uint32_t (&y)[8], uint32_t &rej, ui
   rej += ok ? 0u : 1u;
 }
 
-// Candidate ln of the refill (src/gauss.c:836-890): CDT sample x (packed 4 bits per lane in
-// xp), uniform y, Bernoulli words rm (bytes 64 + 8 li + 100 h) and exponent byte, sign bit ln
-// of k8.  |value| = z < 8K < 2^33 is kept as its low word (returned) and, in `bits`, its accept
-// bit (bit ln), its bit 32 (bit 8 + ln) and bit 16 if an accepted z ever reaches 2^33.
-template <int SIG, int VAR>
-__device__ __forceinline__ uint32_t refill_candidate(int ln, uint32_t xp, uint32_t y, uint32_t rm_lo,
-                                                     uint32_t rm_hi, uint32_t ewrd, uint32_t k8, double kinv,
-                                                     uint32_t &bits) {
-  const uint32_t x = (xp >> (4 * ln)) & 15u;
-  const uint32_t rexp = (ewrd >> (24 - 8 * (ln & 3))) & 0xffu;
-  uint64_t z;
-  const bool b = candidate<SIG, VAR>(x, y, le64_of(rm_lo, rm_hi), rexp, kinv, z);
-  const uint32_t a = accept_final(b, z, (k8 >> ln) & 1u);
-  bits |= (a << ln) | ((uint32_t)((z >> 32) & 1u) << (8 + ln)) | ((a & (uint32_t)((z >> 33) != 0)) << 16);
-  return (uint32_t)z;
-}
-
 template <int SIG, bool FULL, int VAR>
 __global__ void __launch_bounds__(kCandThreads, 1)
     k_cand_cpu(const uint32_t *__restrict__ rkeys, SegDev sg, double kinv, uint32_t *__restrict__ cand_lo,
                uint8_t *__restrict__ amask, uint16_t *__restrict__ chs, uint32_t *__restrict__ status) {
-  extern __shared__ __align__(128) uint8_t smem[];
-  aes_fill_tables(smem);
+  aes_fill_tables();
   __syncthreads();
-  const AesCtx c{smem, (threadIdx.x & 31u) * 4u};
+  const AesCtx c = aes_ctx();
   // the host keeps the flattened refill count below 2^32 - 2^24 (no wrap of g)
   const uint32_t total = (uint32_t)__ldg(sg.roff + sg.nstreams);
   uint32_t rk[60];
   uint32_t st = 0;
   uint32_t lo = 1, hi = 0;  // refill range of stream st (empty: forces the first lookup)
   CtrCache cc;
-  for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x) {
+  // a contiguous run of refills per warp: the counter cache's upper part lasts 2,730 refills
+  const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+  const uint32_t run = ((total + warps - 1) / warps + 31u) & ~31u;
+  const uint32_t g0 = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * run, g1 = min(total, g0 + run);
+  for (uint32_t g = g0 + (threadIdx.x & 31u); g < g1; g += 32u) {
     if (g < lo || g >= hi) {
       st = seg_find(sg.roff, sg.nstreams, g);
       lo = (uint32_t)__ldg(sg.roff + st);
@@ -180,86 +193,92 @@ __global__ void __launch_bounds__(kCandThreads, 1)
     uint32_t y[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) y[j] = 0;
-    uint32_t rej = 0, k8 = 0, xp = 0, w24 = 0, w48 = 0, w49 = 0, carry = 0, lo0 = 0, lo1 = 0;
+    uint32_t rej = 0, k8 = 0, xp = 0, w34 = 0, w42 = 0, w48 = 0, ew = 0, lo0 = 0, lo1 = 0;
     uint32_t bits = 0;  // accept mask, bits 32 (<< 8), wide flag (bit 16)
-    // one AES body for all 13 blocks (keeps the loop inside the instruction cache); the
-    // consumer of each block is selected by the (warp-uniform) step
+    uint32_t open = 0;  // candidates that their top words do not decide
+    uint32_t ln = 4;    // the next two candidates: ln, ln + 1 (lanes 4..7, then 0..3)
+    // One AES body for all 13 blocks, one body for two CDT samples and one for two candidates
+    // (src/gauss.c:836-890): the loop has to stay inside the instruction cache.  What is done with
+    // a block is selected by the (warp-uniform) step.
 #pragma unroll 1
     for (int step = 0; step < kRefillBlocks; ++step) {
       uint32_t W[4];
-      aes256_ctr_block_cached(W, cb + c_refill_order[step], rk, rkg, c, cc);
-      switch (step) {
-        case 0:  // block 12: words 48 (rm high word of lane 7), 49 (exponents of lanes 4..7), 50, 51
-          w48 = W[0];
-          w49 = W[1];
-          uniform_step<SIG, 0>(y, rej, W[2]);
-          uniform_step<SIG, 1>(y, rej, W[3]);
-          break;
-        case 1:  // block 13: uniform words 52..55
-          uniform_step<SIG, 2>(y, rej, W[0]);
-          uniform_step<SIG, 3>(y, rej, W[1]);
-          uniform_step<SIG, 4>(y, rej, W[2]);
-          uniform_step<SIG, 5>(y, rej, W[3]);
-          break;
-        case 2:  // block 14: uniform words 56..59; fewer than 8 of the 10 accepted: slow path
-          uniform_step<SIG, 6>(y, rej, W[0]);
-          uniform_step<SIG, 7>(y, rej, W[1]);
-          uniform_step<SIG, 8>(y, rej, W[2]);
-          uniform_step<SIG, 9>(y, rej, W[3]);
-          if (rej > 2) {
-            uint32_t ys[8];
-            uniform_slow<SIG>(ys, 1, cb, rkg, c, status);
+      aes256_ctr_block_cached(W, cb + c_refill_order[step], rk, rkg, c, cc, (kEvenWords >> step) & 1u,
+                              (kOddWords >> step) & 1u);
+      if (step == 0) {  // block 17: word 70 holds the sign byte 280
+        k8 = bswap32(W[2]) & 0xffu;
+      } else if (step == 1) {  // block 12: words 48 (top Bernoulli word of lane 7), 49 (exponents of lanes 4..7), 50, 51
+        w48 = W[0];
+        ew = W[1];
+        uniform_step<SIG, 0>(y, rej, W[2]);
+        uniform_step<SIG, 1>(y, rej, W[3]);
+      } else if (step == 2) {  // block 13: uniform words 52..55
+        uniform_step<SIG, 2>(y, rej, W[0]);
+        uniform_step<SIG, 3>(y, rej, W[1]);
+        uniform_step<SIG, 4>(y, rej, W[2]);
+        uniform_step<SIG, 5>(y, rej, W[3]);
+      } else if (step == 3) {  // block 14: uniform words 56..59; fewer than 8 of the 10 accepted: slow path
+        uniform_step<SIG, 6>(y, rej, W[0]);
+        uniform_step<SIG, 7>(y, rej, W[1]);
+        uniform_step<SIG, 8>(y, rej, W[2]);
+        uniform_step<SIG, 9>(y, rej, W[3]);
+        if (rej > 2) {
+          uint32_t ys[8];
+          uniform_slow<SIG>(ys, 1, cb, rkg, c, status);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) y[j] = ys[j];
-          }
-          break;
-        case 3:  // block 17: word 70 holds the sign byte 280
-          k8 = bswap32(W[2]) & 0xffu;
-          break;
-        case 4:  // block 6: word 24, the exponent bytes of lanes 0..3
-          w24 = W[0];
-          break;
-        case 5:  // block 2: CDT high words of lanes 0 (words 8, 9) and 1 (10, 11)
-          xp |= cdt_lane<FULL>(0, le64_of(W[0], W[1]), cb, rkg, c);
-          xp |= cdt_lane<FULL>(1, le64_of(W[2], W[3]), cb, rkg, c) << 4;
-          break;
-        case 6:  // block 3: lanes 2 (12, 13) and 3 (14, 15)
-          xp |= cdt_lane<FULL>(2, le64_of(W[0], W[1]), cb, rkg, c) << 8;
-          xp |= cdt_lane<FULL>(3, le64_of(W[2], W[3]), cb, rkg, c) << 12;
-          break;
-        case 7:  // block 4: Bernoulli words of lanes 0 (16, 17) and 1 (18, 19)
-          lo0 = refill_candidate<SIG, VAR>(0, xp, y[0], W[0], W[1], w24, k8, kinv, bits);
-          lo1 = refill_candidate<SIG, VAR>(1, xp, y[1], W[2], W[3], w24, k8, kinv, bits);
-          break;
-        case 8: {  // block 5: lanes 2 (20, 21) and 3 (22, 23); candidates 0..3 complete
-          const uint32_t lo2 = refill_candidate<SIG, VAR>(2, xp, y[2], W[0], W[1], w24, k8, kinv, bits);
-          const uint32_t lo3 = refill_candidate<SIG, VAR>(3, xp, y[3], W[2], W[3], w24, k8, kinv, bits);
-          reinterpret_cast<uint4 *>(cand_lo + (size_t)g * 8)[0] = make_uint4(lo0, lo1, lo2, lo3);
-          break;
+          for (int j = 0; j < 8; ++j) y[j] = ys[j];
         }
-        case 9:  // block 8: CDT words of lane 4 (33, 34); word 35 starts lane 5
-          xp |= cdt_lane<FULL>(4, le64_of(W[1], W[2]), cb, rkg, c) << 16;
-          carry = W[3];
-          break;
-        case 10:  // block 9: lanes 5 (35, 36) and 6 (37, 38); word 39 starts lane 7
-          xp |= cdt_lane<FULL>(5, le64_of(carry, W[0]), cb, rkg, c) << 20;
-          xp |= cdt_lane<FULL>(6, le64_of(W[1], W[2]), cb, rkg, c) << 24;
-          carry = W[3];
-          break;
-        case 11:  // block 10: lane 7 CDT (39, 40); Bernoulli words of lane 4 (41, 42); 43 starts lane 5
-          xp |= cdt_lane<FULL>(7, le64_of(carry, W[0]), cb, rkg, c) << 28;
-          lo0 = refill_candidate<SIG, VAR>(4, xp, y[4], W[1], W[2], w49, k8, kinv, bits);
-          carry = W[3];
-          break;
-        default: {  // block 11: Bernoulli words of lanes 5 (43, 44), 6 (45, 46), 7 (47, 48)
-          const uint32_t lo5 = refill_candidate<SIG, VAR>(5, xp, y[5], carry, W[0], w49, k8, kinv, bits);
-          const uint32_t lo6 = refill_candidate<SIG, VAR>(6, xp, y[6], W[1], W[2], w49, k8, kinv, bits);
-          const uint32_t lo7 = refill_candidate<SIG, VAR>(7, xp, y[7], W[3], w48, w49, k8, kinv, bits);
-          reinterpret_cast<uint4 *>(cand_lo + (size_t)g * 8)[1] = make_uint4(lo0, lo5, lo6, lo7);
-          break;
+      } else if (step == 4) {  // block 8: top CDT word of lane 4 (34)
+        w34 = W[2];
+      } else if (step == 8) {  // block 6: word 24, the exponent bytes of lanes 0..3
+        ew = W[0];
+      } else if (step == 5 || step == 6 || step == 9 || step == 10) {
+        // top CDT words, two lanes each: blocks 9 (lanes 5: 36, 6: 38), 10 (4: 34, 7: 40), 2 (0: 9, 1:
+        // 11), 3 (2: 13, 3: 15); block 10 also has the top Bernoulli word of lane 4 (42).  xp holds the
+        // samples of the next four candidates, 4 bits each.
+        const uint32_t la = step == 5 ? 1u : step == 10 ? 2u : 0u, lb = step == 6 ? 3u : la + 1u;
+        const uint32_t wa = step == 5 ? W[0] : step == 6 ? w34 : W[1];
+        const uint32_t wb = step == 5 ? W[2] : step == 6 ? W[0] : W[3];
+        if (step == 6) w42 = W[2];
+        bool ta, tb;
+        xp |= (cdt_sample_top(bswap32(wa), ta) << (4u * la)) | (cdt_sample_top(bswap32(wb), tb) << (4u * lb));
+        open |= (((uint32_t)ta << la) | ((uint32_t)tb << lb)) << (step < 9 ? 4 : 0);
+      } else {
+        // top Bernoulli words: blocks 11 (lanes 4: 42, 5: 44 and 6: 46, 7: 48), 4 (0: 17, 1: 19), 5 (2:
+        // 21, 3: 23).  Each pair of candidates takes its y, CDT samples and exponent bytes from the
+        // head of their queues: y[4..7], y[0..3] in that order, xp and ew.
+        uint32_t ra = step == 7 ? w42 : W[1], rb = step == 7 ? W[0] : W[3];
+#pragma unroll 1
+        for (;;) {
+          uint64_t za, zb;
+          bool ta, tb;
+          const uint64_t va = candidate_input<SIG>(xp & 15u, y[4], za);
+          const uint64_t vb = candidate_input<SIG>((xp >> 4) & 15u, y[5], zb);
+          const bool ba = bernoulli_accept_top<SIG, VAR>(va, bswap32(ra), ew >> 24, kinv, ta);
+          const bool bb = bernoulli_accept_top<SIG, VAR>(vb, bswap32(rb), (ew >> 16) & 0xffu, kinv, tb);
+          bits |= candidate_bits(ln, ba, za, k8) | candidate_bits(ln + 1u, bb, zb, k8);
+          open |= ((uint32_t)ta | ((uint32_t)tb << 1)) << ln;
+          if (ln & 2u)
+            reinterpret_cast<uint4 *>(cand_lo + (size_t)g * 8)[ln >> 2] = make_uint4(lo0, lo1, (uint32_t)za, (uint32_t)zb);
+          lo0 = (uint32_t)za;
+          lo1 = (uint32_t)zb;
+          xp >>= 8;
+          ew <<= 16;
+          y[4] = y[6];
+          y[5] = y[7];
+          y[6] = y[0];
+          y[7] = y[1];
+          y[0] = y[2];
+          y[1] = y[3];
+          ln = (ln + 2u) & 7u;
+          if (ln != 6u) break;
+          ra = W[2];
+          rb = w48;
         }
       }
     }
+    if (open)
+      bits = refill_slow<SIG, FULL, VAR>(open, k8, cb, rkg, c, kinv, cand_lo + (size_t)g * 8, bits, status);
     amask[g] = (uint8_t)bits;
     chs[g] = (uint16_t)(((bits >> 8) & 0xffu) | (k8 << 8));
     if (bits & 0x10000u) atomicOr(status, kStatusWideSample);
@@ -636,7 +655,7 @@ __global__ void k_seg_uniform(uint32_t nstreams, uint32_t calls, uint32_t n, uin
 // into buf; blocks 18..23 only when a uniform draw needs them.
 __device__ __forceinline__ void chain_blocks(uint32_t *buf, int from, int to, uint32_t &s0, uint32_t &s1,
                                              uint32_t &s2, uint32_t &s3, const uint32_t (&rk)[60],
-                                             const AesCtx &c) {
+                                             AesCtx c) {
   for (int m = from; m < to; ++m) {
     aes256_rounds(s0, s1, s2, s3, rk, c);
     buf[4 * m] = s0;
@@ -653,10 +672,9 @@ template <int SIG>
 __global__ void __launch_bounds__(kGpuMapThreads, 1)
     k_gauss_gpu_map(const uint32_t *__restrict__ rkey, uint32_t poly0, uint32_t npolys, uint32_t n, double kinv,
                     ModArgs m, uint32_t *__restrict__ out, uint32_t *__restrict__ status) {
-  extern __shared__ __align__(128) uint8_t smem[];
-  aes_fill_tables(smem);
+  aes_fill_tables();
   __syncthreads();
-  const AesCtx c{smem, (threadIdx.x & 31u) * 4u};
+  const AesCtx c = aes_ctx();
   uint32_t rk[60];
 #pragma unroll
   for (int i = 0; i < 60; ++i) rk[i] = __ldg(rkey + i);
@@ -751,10 +769,9 @@ __global__ void __launch_bounds__(kGpuMapThreads, 1)
 // sample_polya (src/sample.c:56-128): AES-CTR (nonce 0) bytes, a_i = le64(bytes 8i..8i+7) mod q_j
 __global__ void __launch_bounds__(256) k_polya(const uint32_t *__restrict__ rkey, uint32_t n, ModArgs m,
                                                uint32_t *__restrict__ a) {
-  extern __shared__ __align__(128) uint8_t smem[];
-  aes_fill_tables(smem);
+  aes_fill_tables();
   __syncthreads();
-  const AesCtx c{smem, (threadIdx.x & 31u) * 4u};
+  const AesCtx c = aes_ctx();
   uint32_t rk[60];
 #pragma unroll
   for (int i = 0; i < 60; ++i) rk[i] = __ldg(rkey + i);

@@ -63,19 +63,21 @@ __device__ __forceinline__ uint32_t cdt_sample(uint64_t r2, uint64_t r1) {
   }
   return x;
 }
-// The high-word compare of cdt_sample<false> from the constant high words, and whether r2
-// ties one of them (the FULL compare needs the low words only then), from the same
-// differences.
-__device__ __forceinline__ uint32_t cdt_sample_hi(uint64_t r2, bool &tie) {
-  r2 &= 0x7fffffffffffffffull;
-  uint32_t x = 0;
-  tie = false;
+// x of cdt_sample from the top 32 bits of r2 alone: entry i counts when r2 < cdt_hi(i), which the
+// top words settle unless they are equal, and a nonzero top word is above entries 5..8.  `open`
+// is set when the top word ties an entry's (or is 0): about 6 in 2^31 draws, which need r2's low
+// word, and a tie of all 63 bits the second word too.
+__device__ __forceinline__ uint32_t cdt_sample_top(uint32_t r2_top, bool &open) {
+  static_assert((cdt_hi(4) >> 32) != 0 && (cdt_hi(5) >> 32) == 0, "entries 0..4 have nonzero top words");
+  const uint32_t h = r2_top & 0x7fffffffu;
+  uint32_t x = 0, near = h;
 #pragma unroll
-  for (int i = 0; i < 9; ++i) {
-    const uint64_t d = r2 - cdt_hi(i);
-    x += (uint32_t)(d >> 63);
-    tie |= d == 0;
+  for (int i = 0; i < 5; ++i) {
+    const uint32_t d = h - (uint32_t)(cdt_hi(i) >> 32);  // both below 2^31: bit 31 is the borrow
+    x += d >> 31;
+    near = min(near, d);
   }
+  open = near == 0;
   return x;
 }
 
@@ -123,29 +125,68 @@ __device__ __forceinline__ bool bernoulli_accept(uint64_t xin, uint64_t rm, uint
   return eq1 || ((((uint64_t)(r_mant - rmant) & (uint64_t)(r_exp - rp)) >> 63) != 0);
 }
 
+// bernoulli_accept from the top 32 bits of rm: the exponent test needs only those, and so does
+// the mantissa test unless the top 21 bits of the two 53-bit mantissas are equal (`open`, about
+// 2^-21 of the calls, which need the low word).  The shift of vtu by 52 leaves 12 bits of it, so
+// the low word of vres is the low word of the polynomial s.
+template <int SIG, int VAR>
+__device__ __forceinline__ bool bernoulli_accept_top(uint64_t xin, uint32_t rm_top, uint32_t rexp, double kinv,
+                                                     bool &open) {
+  const uint64_t x = xin | 0x4330000000000000ull;
+  double vx = (SIG == 0) ? __ull2double_rn(x - 0x4330000000000000ull)
+                         : __dsub_rn(__longlong_as_double((long long)x), 4503599627370496.0);
+  vx = __dmul_rn(vx, kinv);
+  const double fl = floor(vx);  // vx <= 0
+  const double t = __dadd_rn(fl, 6755399441055744.0);
+  // the low 12 bits of (long long)t: for sigma_1 (|vx| < 19) and by the AVX form they are t's own
+  // low mantissa bits; t <= 1.5 2^52 here, and below -2^63 the conversion saturates as x86 does
+  const uint32_t ti = (VAR == 1 || SIG == 0) ? (uint32_t)__double2loint(t) : (uint32_t)__double2ll_rz(t);
+  const double f = __dsub_rn(vx, fl);
+  double s = __fma_rn(__longlong_as_double((long long)c_expc[0]), f, __longlong_as_double((long long)c_expc[1]));
+#pragma unroll
+  for (int c = 2; c < 10; ++c) s = __fma_rn(s, f, __longlong_as_double((long long)c_expc[c]));
+  const uint32_t vtop = (uint32_t)__double2hiint(s) + (ti << 20);
+  const int32_t rexpo = (VAR == 1 ? (int32_t)(vtop >> 20) : ((int32_t)vtop >> 20)) + (19 - 1023 + 1);
+  const uint32_t r_exp = (rm_top >> 21) | (rexp << 11);  // 19 bits
+  bool below;  // r_exp < 2^rexpo, with the out-of-range shifts of bernoulli_accept
+  if (VAR != 0)
+    below = (uint32_t)rexpo < 64u && __funnelshift_rc(r_exp, 0u, (uint32_t)rexpo) == 0;
+  else if (SIG == 0)
+    below = __funnelshift_rc(r_exp, 0u, (uint32_t)rexpo & 63u) == 0;
+  else
+    below = rexpo >= 0 && __funnelshift_rc(r_exp, 0u, (uint32_t)rexpo & 63u) == 0;
+  const uint32_t m = (vtop & 0xfffffu) | 0x100000u, r = rm_top & 0x1fffffu;
+  const bool eq1 = vtop == 0x3ff00000u && __double2loint(s) == 0;
+  open = below && r == m && !eq1;
+  return eq1 || (below && r < m);
+}
+
 // uniform y in [0, K): 32-bit rejection then Barrett (src/gauss.c:578-703)
 template <int SIG>
 __device__ __forceinline__ bool uniform_ok(uint32_t x) {
   constexpr uint64_t K = sigma_k(SIG), BF = (1ull << 32) / K, UQ = K * BF;
   return (uint64_t)x < UQ;
 }
+// x - (floor(x BF / 2^32) + 1) K, plus K if that is negative; it lies in [-K, K), so 32 bits hold
+// it and the correction is the unsigned minimum of r and r + K
 template <int SIG>
-__device__ __forceinline__ uint32_t uniform_reduce(uint32_t x32) {
-  constexpr uint64_t K = sigma_k(SIG), BF = (1ull << 32) / K;
-  uint64_t x = x32;
-  x = x - ((((x * BF) >> 32) + 1) * K);
-  x = x + (x >> 63) * K;
-  return (uint32_t)x;
+__device__ __forceinline__ uint32_t uniform_reduce(uint32_t x) {
+  constexpr uint32_t K = (uint32_t)sigma_k(SIG), BF = (uint32_t)((1ull << 32) / K);
+  const uint32_t r = x - __umulhi(x, BF) * K - K;
+  return __viaddmin_u32(r, K, r);
 }
 
 // one candidate: z = K x + y, Bernoulli input (uint32)(z + K x) * y (src/gauss.c:836-850)
+template <int SIG>
+__device__ __forceinline__ uint64_t candidate_input(uint32_t x, uint32_t y, uint64_t &z) {
+  constexpr uint32_t K = (uint32_t)sigma_k(SIG);
+  z = (uint64_t)x * K + y;
+  return (uint64_t)(2u * K * x + y) * y;
+}
 template <int SIG, int VAR>
 __device__ __forceinline__ bool candidate(uint32_t x, uint32_t y, uint64_t rm, uint32_t rexp, double kinv,
                                           uint64_t &z) {
-  constexpr uint64_t K = sigma_k(SIG);
-  const uint64_t kx = (uint64_t)x * K;
-  z = kx + y;
-  const uint64_t vb = (uint64_t)(uint32_t)(z + kx) * (uint64_t)y;
+  const uint64_t vb = candidate_input<SIG>(x, y, z);
   return bernoulli_accept<SIG, VAR>(vb, rm, rexp, kinv);
 }
 
