@@ -76,6 +76,11 @@ int ctx_encrypt_cpu_map(Ctx &c, int batch, const uint32_t *d_x, const uint32_t *
                         const uint8_t *seeds3, uint32_t *d_ct, cudaStream_t s);
 int ctx_encrypt_gpu_map(Ctx &c, int batch, const uint32_t *d_x, const uint32_t *d_mpk, const uint8_t *seed2,
                         uint32_t *d_ct, cudaStream_t s);
+// out[z][k][3][n] = sum_i y[k][i] v[z][i] mod q (mac.cu); v: nz blocks of l residue-polynomial
+// triples, vstride words apart; keys y[k][l]
+struct SchemeArgs;
+int mac_launch(Ctx &c, const SchemeArgs &sa, const uint32_t *d_v, size_t vstride, int nz, const uint32_t *d_y,
+               int y_signed, int nkeys, uint32_t *d_out, cudaStream_t s);
 int ctx_keygen(Ctx &c, int nkeys, const uint32_t *d_y, int y_signed, const uint32_t *d_msk, uint32_t *d_sky,
                cudaStream_t s);
 int ctx_decrypt(Ctx &c, int nct, const uint32_t *d_ct, int nkeys, const uint32_t *d_y, int y_signed,

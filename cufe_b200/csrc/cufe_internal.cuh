@@ -32,6 +32,15 @@ struct RingArgs {
   int pp_fwd, pp_inv;  // NTT kernel variant per direction (1..CUFE_NTT_VARIANTS), set by the tuner
 };
 
+// bits of the device status word that a context's calls set (cufe_sync reports them)
+enum : uint32_t {
+  kStatusUniformOverrun = 1u,   // a uniform draw ran past the 384-byte refill (reference UB)
+  kStatusRefillsExhausted = 2u, // mode A: the precomputed refills did not cover all calls
+  kStatusRefillCap = 4u,        // GPU mapping: a thread exceeded kMaxRefillsPerThread refills
+  kStatusWideSample = 8u,       // an accepted candidate at or above 2^33 (z = K x + y < 8K keeps it below)
+  kStatusMmaTimeout = 16u,      // a wait for the tensor core gave up (mac.cu)
+};
+
 // ------------------------------------------------------------------ arithmetic
 // All residues are kept canonical in [0, q) with q < 2^31.
 

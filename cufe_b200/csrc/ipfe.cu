@@ -515,86 +515,14 @@ __global__ void __launch_bounds__(NttPlan<LOGN>::T * ppc<LOGN>(), MINB)
   }
 }
 
-// sk_y = sum_i (y_i mod q_m) msk_i (src/rlwe_sife.c:215-245); KCH keys per pass over msk
-template <int KCH>
-__global__ void __launch_bounds__(256) k_keygen(const uint32_t *__restrict__ y, int y_signed, int nkeys,
-                                                const uint32_t *__restrict__ msk, uint32_t *__restrict__ sky, int n,
-                                                SchemeArgs sa) {
-  extern __shared__ uint32_t smem_u32[];
-  const int l = sa.l, m = blockIdx.y, k0 = blockIdx.z * KCH;
-  const uint32_t q = sa.ra.q[m];
-  uint32_t *yq = smem_u32, *ys = smem_u32 + KCH * l;
-  for (int t = threadIdx.x; t < KCH * l; t += blockDim.x) {
-    const int kk = t / l, i = t - kk * l;
-    uint32_t v = 0;
-    if (k0 + kk < nkeys) v = y_residue(y[(size_t)(k0 + kk) * l + i], y_signed, q, sa.mu[m]);
-    yq[t] = v;
-    ys[t] = (uint32_t)(((uint64_t)v << 32) / q);
-  }
-  __syncthreads();
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n) return;
-  uint64_t acc[KCH];
-#pragma unroll
-  for (int kk = 0; kk < KCH; ++kk) acc[kk] = 0;
-  for (int i = 0; i < l; ++i) {
-    const uint32_t v = __ldg(msk + ((size_t)i * 3 + m) * n + j);
-#pragma unroll
-    for (int kk = 0; kk < KCH; ++kk) acc[kk] += shoup_lazy(v, yq[kk * l + i], ys[kk * l + i], q);
-  }
-#pragma unroll
-  for (int kk = 0; kk < KCH; ++kk)
-    if (k0 + kk < nkeys) sky[((size_t)(k0 + kk) * 3 + m) * n + j] = mod_u64(acc[kk], sa.mu[m], q);
-}
-
-// Decryption (src/rlwe_sife.c:248-278), d_y = sum_i y_i c_i - INTT(NTT(c_l) NTT(sk_y)), in
-// two kernels.  k_dec_mac streams the ciphertexts: thread = 4 consecutive coefficients of one
-// (ciphertext, key, residue), 16-byte loads, Shoup products accumulated in 64 bits; the
-// l-sum is optionally split into S chunks (small batches) with canonical partial sums.
-// k_dec_tail adds the chunks and subtracts the negacyclic product c_l * sk_y.
-__global__ void __launch_bounds__(256) k_dec_mac(const uint32_t *__restrict__ ct, const uint32_t *__restrict__ y,
-                                                 int y_signed, int nkeys, int nsplit, uint32_t *__restrict__ part,
-                                                 SchemeArgs sa) {
-  extern __shared__ uint32_t smem_u32[];
-  const int n = sa.ra.n, l = sa.l;
-  const int per_poly = n / 4 / blockDim.x;  // CTAs per residue polynomial
-  const int s = blockIdx.x / per_poly, sub = blockIdx.x - s * per_poly;
-  const int w = blockIdx.y;  // (c * nkeys + key) * 3 + m
-  const int m = w % 3, ck = w / 3, key = ck % nkeys, c = ck / nkeys;
-  const uint32_t q = sa.ra.q[m];
-  const int i0 = (int)((long long)l * s / nsplit), i1 = (int)((long long)l * (s + 1) / nsplit);
-  uint32_t *yq = smem_u32, *ys = smem_u32 + (i1 - i0);
-  for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
-    const uint32_t v = y_residue(y[(size_t)key * l + i], y_signed, q, sa.mu[m]);
-    yq[i - i0] = v;
-    ys[i - i0] = (uint32_t)(((uint64_t)v << 32) / q);
-  }
-  __syncthreads();
-  const int j = 4 * (sub * blockDim.x + threadIdx.x);
-  const uint32_t *cb = ct + (size_t)c * (l + 1) * 3 * n + (size_t)m * n + j;
-  uint64_t a0 = 0, a1 = 0, a2 = 0, a3 = 0;
-#pragma unroll 4
-  for (int i = i0; i < i1; ++i) {
-    const uint4 v = __ldg(reinterpret_cast<const uint4 *>(cb + (size_t)i * 3 * n));
-    const uint32_t yv = yq[i - i0], yh = ys[i - i0];
-    a0 += shoup_lazy(v.x, yv, yh, q);
-    a1 += shoup_lazy(v.y, yv, yh, q);
-    a2 += shoup_lazy(v.z, yv, yh, q);
-    a3 += shoup_lazy(v.w, yv, yh, q);
-  }
-  uint4 o;
-  o.x = mod_u64(a0, sa.mu[m], q);
-  o.y = mod_u64(a1, sa.mu[m], q);
-  o.z = mod_u64(a2, sa.mu[m], q);
-  o.w = mod_u64(a3, sa.mu[m], q);
-  *reinterpret_cast<uint4 *>(part + ((size_t)w * nsplit + s) * n + j) = o;
-}
-
+// Decryption (src/rlwe_sife.c:248-278), d_y = sum_i y_i c_i - INTT(NTT(c_l) NTT(sk_y)): the
+// l-sums come from mac_launch; k_dec_tail subtracts the negacyclic product c_l * sk_y from them,
+// in place.
 template <int LOGN>
 __global__ void __launch_bounds__(512)
-    k_dec_tail(const uint32_t *__restrict__ part, int nsplit, const uint32_t *__restrict__ clhat,
-               const uint32_t *__restrict__ skhat, const uint32_t *__restrict__ skhat_sh, int nkeys,
-               uint32_t *__restrict__ dy, long long nwork, SchemeArgs sa) {
+    k_dec_tail(const uint32_t *__restrict__ clhat, const uint32_t *__restrict__ skhat,
+               const uint32_t *__restrict__ skhat_sh, int nkeys, uint32_t *__restrict__ dy, long long nwork,
+               SchemeArgs sa) {
   using P = NttPlan<LOGN>;
   extern __shared__ uint32_t smem_u32[];
   const int th = threadIdx.x;
@@ -615,14 +543,11 @@ __global__ void __launch_bounds__(512)
   ntt_inv_core<LOGN>(a, sm, th, q, sa.ra.ipsi2 + (size_t)m * P::N, sa.ra.ninv[m],
                      sa.ra.ninv_sh[m], sa.ra.w1n[m], sa.ra.w1n_sh[m]);
   if (act) {
-    const uint32_t *pp = part + (size_t)ww * nsplit * P::N;
     uint32_t *o = dy + ww * P::N;
 #pragma unroll
     for (int e = 0; e < 16; ++e) {
       const int j = P::template idx<0>(th, e);
-      uint32_t mac = pp[j];
-      for (int s = 1; s < nsplit; ++s) mac = mod_add(mac, pp[(size_t)s * P::N + j], q);
-      o[j] = mod_sub(mac, a[e], q);
+      o[j] = mod_sub(o[j], a[e], q);
     }
   }
 }
@@ -919,6 +844,7 @@ int Ctx::check_status(cudaStream_t s) {
     if (st & 2u) why += " precomputed refill range exhausted;";
     if (st & 4u) why += " GPU-mapping refill cap reached;";
     if (st & 8u) why += " candidate at or above 2^33;";
+    if (st & 16u) why += " a wait for the tensor core gave up;";
     set_last_error(std::string("sampler status ") + std::to_string(st) + ":" + why);
     return CUFE_ERR_SAMPLER;
   }
@@ -1148,55 +1074,39 @@ int ctx_encrypt_gpu_map(Ctx &c, int batch, const uint32_t *d_x, const uint32_t *
 
 int ctx_keygen(Ctx &c, int nkeys, const uint32_t *d_y, int y_signed, const uint32_t *d_msk, uint32_t *d_sky,
                cudaStream_t s) {
-  if (nkeys < 1) return CUFE_ERR_INVALID;
-  constexpr int KCH = 4;
-  const SchemeArgs sa = scheme_args(c);
-  const size_t smem = (size_t)2 * KCH * c.l * 4;
-  if (smem > 200 * 1024) return CUFE_ERR_INVALID;
-  CUFE_CUDA(cudaFuncSetAttribute(k_keygen<KCH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  dim3 grid((c.n + 255) / 256, 3, (nkeys + KCH - 1) / KCH);
+  if (nkeys < 1 || c.l > 6400) return CUFE_ERR_INVALID;
   ProfScope ps("keygen", s);
-  note_launch(), k_keygen<KCH><<<grid, 256, smem, s>>>(d_y, y_signed, nkeys, d_msk, d_sky, c.n, sa);
-  CUFE_CUDA(cudaGetLastError());
-  return CUFE_OK;
+  return mac_launch(c, scheme_args(c), d_msk, 0, 1, d_y, y_signed, nkeys, d_sky, s);
 }
 
-int ctx_decrypt(Ctx &c, int nct, const uint32_t *d_ct, int nkeys, const uint32_t *d_y, int y_signed,
-                const uint32_t *d_sky, uint32_t *d_dy, cudaStream_t s) {
-  if (nct < 1 || nkeys < 1) return CUFE_ERR_INVALID;
-  const int n = c.n, l = c.l;
-  const size_t poly = (size_t)3 * n;
-  const long long nwork = (long long)nct * nkeys * 3;
-  // split the l-sum until about two waves of MAC threads are resident
-  const long long base_threads = nwork * (n / 4);
-  const long long want = (long long)c.num_sms * 2048 * 2;
+// the vector lengths that decryption takes: 25,599 slots per chunk of the l-sum, and as many
+// chunks as it takes to fill the device, max_split at most
+static bool decrypt_length_ok(const Ctx &c, long long nwork, int max_split) {
   int nsplit = 1;
-  while (nsplit < 32 && base_threads * nsplit < want && l / (nsplit * 2) >= 8) nsplit *= 2;
-  int rc = c.ensure_ws(((size_t)nct * poly + 2 * (size_t)nkeys * poly + (size_t)nwork * nsplit * n) * 4 + 8 * 256);
-  if (rc) return rc;
-  Arena ar(c.ws);
-  uint32_t *clhat = ar.take<uint32_t>((size_t)nct * poly);
-  uint32_t *skhat = ar.take<uint32_t>((size_t)nkeys * poly);
-  uint32_t *skhat_sh = ar.take<uint32_t>((size_t)nkeys * poly);
-  uint32_t *part = ar.take<uint32_t>((size_t)nwork * nsplit * n);
-  CUFE_CUDA(cudaMemcpy2DAsync(clhat, poly * 4, d_ct + (size_t)l * poly, (size_t)(l + 1) * poly * 4, poly * 4, nct,
+  while (nsplit < max_split && nwork * (c.n / 4) * nsplit < (long long)c.num_sms * 2048 * 2 && c.l / (nsplit * 2) >= 8)
+    nsplit *= 2;
+  return (c.l + nsplit - 1) / nsplit + 1 <= 25600;
+}
+
+// the decryption of nct ciphertexts under nkeys keys with its scratch: clhat [nct][3][n], skhat
+// and skhat_sh [nkeys][3][n]
+static int decrypt_with(Ctx &c, int nct, const uint32_t *d_ct, int nkeys, const uint32_t *d_y, int y_signed,
+                        const uint32_t *d_sky, uint32_t *d_dy, uint32_t *clhat, uint32_t *skhat, uint32_t *skhat_sh,
+                        cudaStream_t s) {
+  const size_t poly = (size_t)3 * c.n, ct_words = (size_t)(c.l + 1) * poly;
+  const long long nwork = (long long)nct * nkeys * 3;
+  const SchemeArgs sa = scheme_args(c);
+  CUFE_CUDA(cudaMemcpy2DAsync(clhat, poly * 4, d_ct + (size_t)c.l * poly, ct_words * 4, poly * 4, nct,
                               cudaMemcpyDeviceToDevice, s));
-  rc = ntt_launch(c.ring.args, clhat, (long long)nct * 3, false, s);
+  int rc = ntt_launch(c.ring.args, clhat, (long long)nct * 3, false, s);
   if (rc) return rc;
   CUFE_CUDA(cudaMemcpyAsync(skhat, d_sky, (size_t)nkeys * poly * 4, cudaMemcpyDeviceToDevice, s));
   rc = ntt_fwd_shoup_launch(c.ring.args, skhat, skhat_sh, (long long)nkeys * 3, s);
   if (rc) return rc;
-  const SchemeArgs sa = scheme_args(c);
   {
-    const int threads = std::min(256, n / 4);
-    const int per_poly = n / 4 / threads;
-    const size_t smem = (size_t)2 * ((l + nsplit - 1) / nsplit + 1) * 4;
-    if (smem > 200 * 1024) return CUFE_ERR_INVALID;
-    CUFE_CUDA(cudaFuncSetAttribute(k_dec_mac, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     ProfScope ps("decrypt_mac", s);
-    note_launch(), k_dec_mac<<<dim3(per_poly * nsplit, (unsigned)nwork), threads, smem, s>>>(d_ct, d_y, y_signed, nkeys, nsplit,
-                                                                             part, sa);
-    CUFE_CUDA(cudaGetLastError());
+    rc = mac_launch(c, sa, d_ct, ct_words, nct, d_y, y_signed, nkeys, d_dy, s);
+    if (rc) return rc;
   }
   return dispatch_logn(c.ring.logn, [&](auto L) {
     constexpr int LOGN = decltype(L)::value;
@@ -1205,10 +1115,24 @@ int ctx_decrypt(Ctx &c, int nct, const uint32_t *d_ct, int nkeys, const uint32_t
     CUFE_CUDA(cudaFuncSetAttribute(k_dec_tail<LOGN>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
     ProfScope ps("decrypt_tail", s);
     note_launch(), k_dec_tail<LOGN><<<(unsigned)((nwork + G - 1) / G), dim3(NttPlan<LOGN>::T, G), smem, s>>>(
-        part, nsplit, clhat, skhat, skhat_sh, nkeys, d_dy, nwork, sa);
+        clhat, skhat, skhat_sh, nkeys, d_dy, nwork, sa);
     CUFE_CUDA(cudaGetLastError());
     return (int)CUFE_OK;
   });
+}
+
+int ctx_decrypt(Ctx &c, int nct, const uint32_t *d_ct, int nkeys, const uint32_t *d_y, int y_signed,
+                const uint32_t *d_sky, uint32_t *d_dy, cudaStream_t s) {
+  if (nct < 1 || nkeys < 1) return CUFE_ERR_INVALID;
+  if (!decrypt_length_ok(c, (long long)nct * nkeys * 3, 32)) return CUFE_ERR_INVALID;
+  const size_t poly = (size_t)3 * c.n;
+  int rc = c.ensure_ws(((size_t)nct * poly + 2 * (size_t)nkeys * poly) * 4 + 8 * 256);
+  if (rc) return rc;
+  Arena ar(c.ws);
+  uint32_t *clhat = ar.take<uint32_t>((size_t)nct * poly);
+  uint32_t *skhat = ar.take<uint32_t>((size_t)nkeys * poly);
+  uint32_t *skhat_sh = ar.take<uint32_t>((size_t)nkeys * poly);
+  return decrypt_with(c, nct, d_ct, nkeys, d_y, y_signed, d_sky, d_dy, clhat, skhat, skhat_sh, s);
 }
 
 // ------------------------------------------------------------------ decryption without allocation
@@ -1219,13 +1143,12 @@ int ctx_decrypt(Ctx &c, int nct, const uint32_t *d_ct, int nkeys, const uint32_t
 // ctx_decrypt_noalloc runs the same decryption kernels as ctx_decrypt with every scratch
 // buffer carved from the file-scope array below instead of the context workspace.  The
 // array is a fixed part of the library image: every GPU that loads the library holds its
-// 2 MiB until the process exits.
+// 432 KiB until the process exits.
 constexpr int kNoAllocMaxN = 4096;    // ring degree
 constexpr int kNoAllocMaxKeys = 4;    // keys per call (one ciphertext per call)
-constexpr int kNoAllocMaxSplit = 8;   // chunks of the l-sum
+constexpr int kNoAllocMaxSplit = 8;   // chunks of the l-sum that bound its length
 constexpr size_t kNoAllocWords = (size_t)3 * kNoAllocMaxN                       // NTT(c_l)
                                  + (size_t)2 * kNoAllocMaxKeys * 3 * kNoAllocMaxN  // NTT(sk_y), Shoup
-                                 + (size_t)3 * kNoAllocMaxKeys * kNoAllocMaxSplit * kNoAllocMaxN  // partials
                                  + 4 * 64;                                          // region padding
 static __device__ __align__(256) uint32_t g_noalloc_scratch[kNoAllocWords];
 
@@ -1254,7 +1177,7 @@ static int noalloc_scratch(int device, uint32_t **out) {
 
 int ctx_decrypt_noalloc(Ctx &c, const uint32_t *d_ct, int nkeys, const uint32_t *d_y, int y_signed,
                         const uint32_t *d_sky, uint32_t *d_dy, cudaStream_t s) {
-  const int n = c.n, l = c.l;
+  const int n = c.n;
   if (n > kNoAllocMaxN || nkeys < 1 || nkeys > kNoAllocMaxKeys) {
     set_last_error("cufe_decrypt_noalloc supports n <= " + std::to_string(kNoAllocMaxN) + " and 1.." +
                    std::to_string(kNoAllocMaxKeys) + " keys per call (got n = " + std::to_string(n) +
@@ -1264,45 +1187,14 @@ int ctx_decrypt_noalloc(Ctx &c, const uint32_t *d_ct, int nkeys, const uint32_t 
   uint32_t *base = nullptr;
   int rc = noalloc_scratch(c.device, &base);
   if (rc) return rc;
+  if (!decrypt_length_ok(c, (long long)nkeys * 3, kNoAllocMaxSplit)) return CUFE_ERR_INVALID;
   const size_t poly = (size_t)3 * n;
-  const long long nwork = (long long)nkeys * 3;
-  const long long base_threads = nwork * (n / 4);
-  const long long want = (long long)c.num_sms * 2048 * 2;
-  int nsplit = 1;
-  while (nsplit < kNoAllocMaxSplit && base_threads * nsplit < want && l / (nsplit * 2) >= 8) nsplit *= 2;
   auto round64 = [](size_t w) { return (w + 63) & ~(size_t)63; };
   uint32_t *clhat = base;
   uint32_t *skhat = clhat + round64(poly);
   uint32_t *skhat_sh = skhat + round64((size_t)nkeys * poly);
-  uint32_t *part = skhat_sh + round64((size_t)nkeys * poly);
-  // every scratch word read below is written first by this call (no zeroing needed)
-  CUFE_CUDA(cudaMemcpyAsync(clhat, d_ct + (size_t)l * poly, poly * 4, cudaMemcpyDeviceToDevice, s));
-  rc = ntt_launch(c.ring.args, clhat, 3, false, s);
-  if (rc) return rc;
-  CUFE_CUDA(cudaMemcpyAsync(skhat, d_sky, (size_t)nkeys * poly * 4, cudaMemcpyDeviceToDevice, s));
-  rc = ntt_fwd_shoup_launch(c.ring.args, skhat, skhat_sh, (long long)nkeys * 3, s);
-  if (rc) return rc;
-  const SchemeArgs sa = scheme_args(c);
-  {
-    const int threads = std::min(256, n / 4);
-    const int per_poly = n / 4 / threads;
-    const size_t smem = (size_t)2 * ((l + nsplit - 1) / nsplit + 1) * 4;
-    if (smem > 200 * 1024) return CUFE_ERR_INVALID;
-    CUFE_CUDA(cudaFuncSetAttribute(k_dec_mac, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    note_launch(), k_dec_mac<<<dim3(per_poly * nsplit, (unsigned)nwork), threads, smem, s>>>(d_ct, d_y, y_signed, nkeys, nsplit,
-                                                                             part, sa);
-    CUFE_CUDA(cudaGetLastError());
-  }
-  return dispatch_logn(c.ring.logn, [&](auto L) {
-    constexpr int LOGN = decltype(L)::value;
-    constexpr int G = ppc<LOGN>();
-    const size_t smem = (size_t)G * NttPlan<LOGN>::SMEM_WORDS * 4;
-    CUFE_CUDA(cudaFuncSetAttribute(k_dec_tail<LOGN>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
-    note_launch(), k_dec_tail<LOGN><<<(unsigned)((nwork + G - 1) / G), dim3(NttPlan<LOGN>::T, G), smem, s>>>(
-        part, nsplit, clhat, skhat, skhat_sh, nkeys, d_dy, nwork, sa);
-    CUFE_CUDA(cudaGetLastError());
-    return (int)CUFE_OK;
-  });
+  // every scratch word read is written first by this call (no zeroing needed)
+  return decrypt_with(c, 1, d_ct, nkeys, d_y, y_signed, d_sky, d_dy, clhat, skhat, skhat_sh, s);
 }
 
 static DecodeArgs decode_args(const Ctx &c) {

@@ -130,7 +130,7 @@ int cufe_decrypt(cufe_ctx *ctx, int nct, const uint32_t *d_ct, int nkeys, const 
  * that must not take cudaMalloc's implicit device synchronisation).  No counterpart in the
  * reference.  Same result as cufe_decrypt for one ciphertext d_ct[l+1][3][n] and nkeys
  * keys: d_dy[nkeys][3][n].  Limits: n <= 4096 and 1 <= nkeys <= 4, else CUFE_ERR_INVALID.
- * Its scratch is a fixed array of about 2 MiB inside the library image, held on every GPU
+ * Its scratch is a fixed array of 432 KiB inside the library image, held on every GPU
  * that loads the library until the process exits.  The first call on a device looks up the
  * array's device address (make that first call before any stream capture).  All calls share
  * the array: calls that overlap on the GPU (different streams, threads or contexts without
