@@ -100,6 +100,13 @@ int svm_predict(Ctx &c, SvmModel &m, int nct, const uint32_t *d_ct, int *d_label
 int svm_tune(Ctx &c, SvmModel &m, int nct, const uint32_t *d_ct, int *choice, float *ms, cudaStream_t s);
 SvmModel *svm_new();
 void svm_delete(SvmModel *m);
+// the coefficient-0 product on the tensor cores (coef0.cu): whether the sizes allow it, its
+// workspace, and the launch
+struct DecodeArgs;
+bool coef0_mma_ok(const Ctx &c);
+size_t coef0_mma_bytes(const Ctx &c, int nct, int nkeys);
+int coef0_mma_launch(Ctx &c, const SchemeArgs &sa, const DecodeArgs &dd, int nct, const uint32_t *d_ct, int nkeys,
+                     const uint32_t *d_y, int y_signed, const uint32_t *d_sky, void *ws, uint32_t *d_out, cudaStream_t s);
 int ctx_decrypt_coef0(Ctx &c, int nct, const uint32_t *d_ct, int nkeys, const uint32_t *d_y, int y_signed,
                       const uint32_t *d_sky, uint32_t *d_d0, uint32_t *d_out, cudaStream_t s);
 int ctx_decrypt_coef0_form(Ctx &c, int form, int nct, const uint32_t *d_ct, int nkeys, const uint32_t *d_y,

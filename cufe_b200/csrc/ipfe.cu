@@ -613,10 +613,10 @@ __global__ void __launch_bounds__(256)
 // XOR-swizzled in steps of the vector width so that the staging stores spread over the banks.
 // Products are exact: a, b < 2^31, so four products sum below 2^64 in one wide multiply-add
 // chain, folded into a 64 + 32-bit accumulator (K < 2^34 products); one reduction per pair.
-// Tile shapes (ciphertexts x keys): 64 x 32 (the default), 64 x 64, 32 x 32, 32 x 64; the
-// context's tuner picks per (ciphertexts, keys).
+// Tile shapes (ciphertexts x keys): 64 x 32, 64 x 64, 32 x 32, 32 x 64; the context's tuner picks per
+// (ciphertexts, keys).  The first gives way to the tensor-core product (coef0.cu) where that can run.
 constexpr int kC0Kc = 32;
-constexpr int kCoef0TiledMinKeys = 32;  // fewer keys: one CTA per pair (untuned rule)
+constexpr int kCoef0TiledMinKeys = 32;  // fewer keys never take the integer tiles untuned
 constexpr int kCoef0Forms = 5;          // 0 per pair, 1..4 the tile shapes below
 template <int TM, int R>
 __device__ __forceinline__ int c0_swz(int kk, int i) {
@@ -1238,8 +1238,9 @@ static int launch_coef0_tiled(Ctx &c, int nct, const uint32_t *d_ct, int nkeys, 
   return CUFE_OK;
 }
 
-// form 0: one CTA per (ciphertext, key) pair; 1..4: the tiled product at 64x32, 64x64, 32x32,
-// 32x64 (ciphertexts x keys) then the decode of every pair
+// form 0: one CTA per (ciphertext, key) pair; 1: the tensor-core product, or where it cannot run the
+// tiled product at 64x32; 2..4: the tiled product at 64x64, 32x32, 32x64 (ciphertexts x keys), then the
+// decode of every pair
 int ctx_decrypt_coef0_form(Ctx &c, int form, int nct, const uint32_t *d_ct, int nkeys, const uint32_t *d_y,
                            int y_signed, const uint32_t *d_sky, uint32_t *d_d0, uint32_t *d_out, cudaStream_t s) {
   if (nct < 1 || nkeys < 1 || (long long)nct * nkeys > 0x7fffffffLL || !d_out || form < 0 || form >= kCoef0Forms)
@@ -1253,6 +1254,18 @@ int ctx_decrypt_coef0_form(Ctx &c, int form, int nct, const uint32_t *d_ct, int 
   }
   // many keys per ciphertext: the tiled product, then the decode of every pair
   const long long npairs = (long long)nct * nkeys;
+  // form 1 runs on the tensor cores where its workspace may be taken: not with d_d0 (those calls use
+  // none, so that they may overlap others of the context), nor in a capture that would have to grow it
+  bool mma = form == 1 && !d_d0 && coef0_mma_ok(c);
+  if (mma && coef0_mma_bytes(c, nct, nkeys) > c.ws_bytes) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    CUFE_CUDA(cudaStreamIsCapturing(s, &cap));
+    mma = cap == cudaStreamCaptureStatusNone && c.ensure_ws(coef0_mma_bytes(c, nct, nkeys)) == CUFE_OK;
+  }
+  if (mma) {
+    ProfScope ps("decrypt_coef0", s);
+    return coef0_mma_launch(c, scheme_args(c), decode_args(c), nct, d_ct, nkeys, d_y, y_signed, d_sky, c.ws, d_out, s);
+  }
   uint32_t *d0 = d_d0;
   if (!d0) {
     const int rc = c.ensure_ws((size_t)npairs * 3 * 4);
@@ -1340,7 +1353,12 @@ int ctx_tune_decrypt_coef0(Ctx &c, int nct, const uint32_t *d_ct, int nkeys, con
 int ctx_decrypt_coef0(Ctx &c, int nct, const uint32_t *d_ct, int nkeys, const uint32_t *d_y, int y_signed,
                       const uint32_t *d_sky, uint32_t *d_d0, uint32_t *d_out, cudaStream_t s) {
   const auto it = c.coef0_form.find({nct, nkeys});
-  const int form = it != c.coef0_form.end() ? it->second : (nkeys < kCoef0TiledMinKeys ? 0 : 1);
+  // untuned: one CTA per pair for few pairs.  us on a B200 (per pair | tensor cores | integer tiles),
+  // n = 2048, l = 124: 64 x 8 pairs 18 | 23 | 185, 1,000 x 1 28 | 35 | 213, 64 x 32 43 | 23 | 218, 200 x 64
+  // 219 | 26 | 223, 1,000 x 500 8178 | 88 | 1261; n = 4096, l = 784: 64 x 8 33 | 30 | 411
+  const long long pairs = (long long)nct * nkeys;
+  int form = !d_d0 && coef0_mma_ok(c) ? (pairs >= 1024 ? 1 : 0) : (nkeys >= kCoef0TiledMinKeys && pairs >= 12800 ? 1 : 0);
+  if (it != c.coef0_form.end()) form = it->second;
   return ctx_decrypt_coef0_form(c, form, nct, d_ct, nkeys, d_y, y_signed, d_sky, d_d0, d_out, s);
 }
 

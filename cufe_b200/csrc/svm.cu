@@ -22,61 +22,87 @@ namespace {
 
 constexpr int kMaxClasses = 64;
 
-// One term loop of the vote, `for (k = 0; k < cnt; k++) sum += coef[k] * kvalue[k]`
-// (main.c:359-362), with the arithmetic gcc -O3 gives it on an AVX2 + FMA host (the
-// reference's Makefile builds with -O3 -march=native -mavx2): the loop is vectorised as an
-// in-order reduction, 4 products at a time (vmulpd: each product rounded) added to the sum one
-// after another (vaddsd), then a 2-wide epilogue the same way, and an odd last term in the
-// scalar remainder, where the multiply-add is contracted to one fused multiply-add.  So every
-// product is rounded before its addition except the last one of an odd-length loop.
-template <class F>
-__device__ double vote_terms(double sum, const double *__restrict__ coef, F value, int first, int cnt) {
-  const int paired = cnt & ~1;
-  for (int k = 0; k < paired; ++k) sum = __dadd_rn(sum, __dmul_rn(coef[first + k], value(first + k)));
-  if (cnt & 1) sum = __fma_rn(coef[first + paired], value(first + paired), sum);
-  return sum;
-}
-
-// One thread per test vector: the vote of main.c:331-379, in its order, the term loops as
-// vote_terms computes them.  kvalue is the decoded coefficient 0 in [0, p]; for signed support
-// vectors it is centred into (-p/2, p/2] (the reference only has unsigned y and uses the value
-// as decoded).
-__global__ void k_svm_vote(const uint32_t *__restrict__ kval, int nct, int lsv, uint32_t p, int centre,
-                           int nr_class, const double *__restrict__ coef, const double *__restrict__ rho,
-                           const int *__restrict__ nsv, const int *__restrict__ label, int *__restrict__ out,
-                           double *__restrict__ dec) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nct) return;
-  const uint32_t *kv = kval + (size_t)t * lsv;
-  auto value = [&](int i) -> double {
-    const uint32_t v = kv[i];
+// The vote of main.c:331-379 for 16 test vectors per CTA, in its order.
+//
+// One term loop, `for (k = 0; k < cnt; k++) sum += coef[k] * kvalue[k]` (main.c:359-362), with the
+// arithmetic gcc -O3 gives it on an AVX2 + FMA host (the reference's Makefile builds with -O3
+// -march=native -mavx2): the loop is vectorised as an in-order reduction, 4 products at a time
+// (vmulpd: each product rounded) added to the sum one after another (vaddsd), then a 2-wide
+// epilogue the same way, and an odd last term in the scalar remainder, where the multiply-add is
+// contracted to one fused multiply-add.  So every product is rounded before its addition except
+// the last one of an odd-length loop.
+//
+// Only the additions form a chain: warps 1.. compute the rounded products of 128 terms (coalesced
+// reads of kvalue), while warp 0, one lane per vector, adds the 128 before them in order.  One
+// thread per vector for all of it waited for a scattered load per term (500 terms, 1,000 vectors
+// on a B200: 75 us against 11).
+//
+// kvalue is the decoded coefficient 0 in [0, p]; for signed support vectors it is centred into
+// (-p/2, p/2] (the reference only has unsigned y and uses the value as decoded).
+constexpr int kVoteThreads = 256, kVoteVecs = 16, kVoteTerms = 128;
+__global__ void __launch_bounds__(kVoteThreads)
+    k_svm_vote(const uint32_t *__restrict__ kval, int nct, int lsv, uint32_t p, int centre, int nr_class,
+               const double *__restrict__ coef, const double *__restrict__ rho, const int *__restrict__ nsv,
+               const int *__restrict__ label, int *__restrict__ out, double *__restrict__ dec) {
+  __shared__ double prod[2][kVoteTerms][kVoteVecs];
+  const int t0 = blockIdx.x * kVoteVecs, tid = threadIdx.x;
+  const int t = t0 + tid;  // the vector of a lane of warp 0
+  const bool chain = tid < kVoteVecs && t < nct;
+  const auto value = [&](int vec, int i) -> double {
+    const uint32_t v = __ldg(kval + (size_t)vec * lsv + i);
     if (centre) {
       const uint32_t r = v % p;
       return r > p / 2 ? (double)r - (double)p : (double)r;
     }
     return (double)v;
   };
-  int start[kMaxClasses], vote[kMaxClasses];
-  start[0] = 0;
-  for (int i = 1; i < nr_class; ++i) start[i] = start[i - 1] + nsv[i - 1];
-  for (int i = 0; i < nr_class; ++i) vote[i] = 0;
-  int pp = 0;
+  int vote[kMaxClasses];
+  if (chain)
+    for (int i = 0; i < nr_class; ++i) vote[i] = 0;
+  int buf = 0, pair = 0, si = 0;
   const int npairs = nr_class * (nr_class - 1) / 2;
-  for (int i = 0; i < nr_class; ++i)
-    for (int j = i + 1; j < nr_class; ++j) {
+  for (int i = 0; i < nr_class; si += nsv[i], ++i) {
+    int sj = si + nsv[i];
+    for (int j = i + 1; j < nr_class; sj += nsv[j], ++j) {
       double sum = 0;
-      const int si = start[i], sj = start[j], ci = nsv[i], cj = nsv[j];
-      const double *coef1 = coef + (size_t)(j - 1) * lsv, *coef2 = coef + (size_t)i * lsv;
-      sum = vote_terms(sum, coef1, value, si, ci);
-      sum = vote_terms(sum, coef2, value, sj, cj);
-      sum -= rho[pp];
-      if (dec) dec[(size_t)t * npairs + pp] = sum;
-      if (sum > 0)
-        ++vote[i];
-      else
-        ++vote[j];
-      ++pp;
+      for (int side = 0; side < 2; ++side) {
+        const double *cf = coef + (size_t)(side ? i : j - 1) * lsv;
+        const int first = side ? sj : si, cnt = nsv[side ? j : i], paired = cnt & ~1;
+        for (int b = 0; b < paired; b += kVoteTerms, buf ^= 1) {
+          const int terms = min(kVoteTerms, paired - b);
+          if (tid >= 32) {
+            constexpr int W = kVoteThreads - 32, IT = (kVoteVecs * kVoteTerms + W - 1) / W;
+#pragma unroll
+            for (int it = 0; it < IT; ++it) {  // unrolled: the reads of all products in flight
+              const int e = it * W + tid - 32, k = e % kVoteTerms, v = e / kVoteTerms;
+              if (v < kVoteVecs && k < terms && t0 + v < nct)
+                prod[buf][k][v] = __dmul_rn(cf[first + b + k], value(t0 + v, first + b + k));
+            }
+          }
+          __syncthreads();  // also: warp 0 has finished with the other buffer
+          if (chain) {
+            int k = 0;
+            for (; k + 8 <= terms; k += 8) {  // eight reads ahead of their additions
+              double x[8];
+#pragma unroll
+              for (int u = 0; u < 8; ++u) x[u] = prod[buf][k + u][tid];
+#pragma unroll
+              for (int u = 0; u < 8; ++u) sum = __dadd_rn(sum, x[u]);
+            }
+            for (; k < terms; ++k) sum = __dadd_rn(sum, prod[buf][k][tid]);
+          }
+        }
+        if ((cnt & 1) && chain) sum = __fma_rn(cf[first + paired], value(t, first + paired), sum);
+      }
+      if (chain) {
+        sum -= rho[pair];
+        if (dec) dec[(size_t)t * npairs + pair] = sum;
+        ++vote[sum > 0 ? i : j];
+      }
+      ++pair;
     }
+  }
+  if (!chain) return;
   int best = 0;
   for (int i = 1; i < nr_class; ++i)
     if (vote[i] > vote[best]) best = i;
@@ -173,7 +199,7 @@ int svm_predict(Ctx &c, SvmModel &m, int nct, const uint32_t *d_ct, int *d_label
   int rc = ctx_decrypt_coef0(c, nct, d_ct, m.lsv, m.d_y, m.y_signed, m.d_sky, nullptr, kv, s);
   if (rc) return rc;
   ProfScope ps("svm_vote", s);
-  note_launch(), k_svm_vote<<<(nct + 127) / 128, 128, 0, s>>>(kv, nct, m.lsv, c.p, m.y_signed, m.nr_class, m.d_coef, m.d_rho,
+  note_launch(), k_svm_vote<<<(nct + kVoteVecs - 1) / kVoteVecs, kVoteThreads, 0, s>>>(kv, nct, m.lsv, c.p, m.y_signed, m.nr_class, m.d_coef, m.d_rho,
                                                m.d_nsv, m.d_label, d_label, d_dec);
   CUFE_CUDA(cudaGetLastError());
   return CUFE_OK;

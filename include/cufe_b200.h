@@ -155,9 +155,11 @@ int cufe_decrypt_coef0(cufe_ctx *ctx, int nct, const uint32_t *d_ct, int nkeys, 
  * for that shape; later calls of the same shape use it (other shapes keep the fixed rules).
  *   cufe_tune_encrypt: one or two instances per thread group in the encryption kernel, for this
  *     batch size (fixed rule: two from batch 2); choice = 1 or 2, ms[2];
- *   cufe_tune_decrypt_coef0: for (nct, nkeys), form 0 = one CTA per (ciphertext, key) pair, 1..4
- *     = the tiled product at 64x32, 64x64, 32x32, 32x64 ciphertexts x keys per CTA (fixed rule:
- *     form 0 below 32 keys, else 1); choice = the form, ms[5];
+ *   cufe_tune_decrypt_coef0: for (nct, nkeys), form 0 = one CTA per (ciphertext, key) pair, 1 = the
+ *     product on the tensor cores (with d_d0, rings below 64 or n + l above 8192: the tiled product at
+ *     64x32), 2..4 = the tiled product at 64x64, 32x32, 32x64 ciphertexts x keys per CTA (fixed rule:
+ *     1 from 1024 pairs, or 12800 where it is the tiled product and there are 32 keys; else form 0);
+ *     choice = the form, ms[5];
  *   cufe_decrypt_coef0_form: cufe_decrypt_coef0 in the given form (tests, comparisons). */
 int cufe_tune_encrypt(cufe_ctx *ctx, int batch, const uint32_t *d_x, const uint32_t *d_mpk, const uint8_t *seeds2,
                       const uint8_t *seeds3, uint32_t *d_ct, int *choice, float *ms, void *stream);
