@@ -6,7 +6,7 @@
 // Two kernels.  k_mac_few streams v once per KCH keys and is bound by memory; k_mac_mma is the
 // product of many keys with v on the tensor cores.  Before, every product was three integer
 // instructions and v was read once per 4 keys (key generation) or per key (decryption).  B200,
-// us per call, before -> now: 1 key at n = 4096, l = 784 277 -> 16; 591 keys at l = 785 2034 -> 70;
+// us per call, before -> now: 1 key at n = 4096, l = 784 277 -> 13; 591 keys at l = 785 2034 -> 70;
 // the decryption of one ciphertext under 591 keys at n = 2048, l = 124 254 -> 100.
 #include <algorithm>
 
@@ -52,75 +52,80 @@ __device__ __forceinline__ void store4(uint32_t *p, uint4 v, bool vec) {
   }
 }
 
+// x mod q for |x| < 2^63
+__device__ __forceinline__ uint32_t mod_s64(int64_t x, uint64_t mu, uint32_t q) {
+  const uint32_t r = mod_u64((uint64_t)(x < 0 ? -x : x), mu, q);
+  return x < 0 && r ? q - r : r;
+}
+
 // A CTA sums 4 * lanes coefficients of one (z, modulus) for KCH keys: thread (slice, lane) takes 4
 // coefficients (16-byte loads) of the rows slice, slice + slices, ..., eight rows in flight, and
-// the slices are added in shared memory, so no partial sums go through memory.  Keys whose
-// entries are all below 2^15 in magnitude (every quantised weight is) take one 64-bit
-// multiply-add per product: with y + 2^15 in place of a signed y the sums stay below
-// 2^32 2^16 l <= 2^64, and 2^15 times the sum of the words comes off at the end.  Others take
-// their residues and the 96-bit sum.
+// the slices are added in shared memory, one thread per coefficient, so no partial sums go
+// through memory.
+struct FewArgs {
+  const uint32_t *v, *y;
+  size_t vstride;
+  uint32_t *out;
+  int y_signed, nkeys, lanes, vec;
+};
 template <int KCH>
-__global__ void __launch_bounds__(kFewThreads)
-    k_mac_few(const uint32_t *__restrict__ v, size_t vstride, const uint32_t *__restrict__ y, int y_signed, int nkeys,
-              uint32_t *__restrict__ out, int lanes, int vec, SchemeArgs sa) {
-  __shared__ uint32_t ys[KCH][kFewRows];
-  __shared__ uint64_t red[kFewThreads][4];
-  __shared__ uint32_t redh[kFewThreads][4];
-  const int n = sa.ra.n, l = sa.l, tid = threadIdx.x;
+struct FewSmem {
+  uint32_t ys[KCH][kFewRows];
+  uint64_t red[4 * kFewThreads];
+  uint32_t redh[4 * kFewThreads];
+};
+
+// WIDE: 96-bit sums of the words by the residues of y.  Otherwise signed 64-bit sums, one
+// multiply-add per product, for |y| < 2^15 (2^31 2^15 l <= 2^62) and words below 2^31; returns
+// false, and stores nothing, where a word is not.  staged: the first rows of y are in sm.ys.
+template <int KCH, bool WIDE>
+__device__ __forceinline__ bool few_sums(const FewArgs &a, const SchemeArgs &sa, FewSmem<KCH> &sm, bool staged) {
+  const int n = sa.ra.n, l = sa.l, tid = threadIdx.x, lanes = a.lanes;
   const int lane = tid & (lanes - 1), slice = tid / lanes, slices = kFewThreads / lanes;
   const int tiles = n / (4 * lanes);  // per residue polynomial
-  const int m = blockIdx.x / tiles, j = 4 * ((blockIdx.x - m * tiles) * lanes + lane);
-  const int z = blockIdx.y, k0 = blockIdx.z * KCH;
-  const uint32_t q = sa.ra.q[m], bias = y_signed ? 32768u : 0u;
+  const int m = blockIdx.x / tiles, j0 = 4 * (blockIdx.x - m * tiles) * lanes;
+  const int z = blockIdx.y, k0 = blockIdx.z * KCH, keys = min(KCH, a.nkeys - k0);
+  const uint32_t q = sa.ra.q[m];
   const uint64_t mu = sa.mu[m];
-  const uint32_t *vb = v + z * vstride + (size_t)m * n + j;
+  const uint32_t *vb = a.v + z * a.vstride + (size_t)m * n + j0 + 4 * lane;
   const size_t row = (size_t)3 * n;
-  bool big = false;
-  for (int t = tid; t < KCH * l; t += kFewThreads) {
-    const int kk = t / l;
-    if (k0 + kk < nkeys) big |= y[(size_t)(k0 + kk) * l + (t - kk * l)] + bias > 65535u;
-  }
-  big = __syncthreads_or(big);
-  uint64_t acc[KCH][4], sx[4];
-  uint32_t hi[KCH][4];
+  uint64_t acc[KCH][4];
+  uint32_t hi[KCH][4], any = 0;
 #pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    sx[e] = 0;
+  for (int kk = 0; kk < KCH; ++kk)
 #pragma unroll
-    for (int kk = 0; kk < KCH; ++kk) acc[kk][e] = 0, hi[kk][e] = 0;
-  }
+    for (int e = 0; e < 4; ++e) acc[kk][e] = 0, hi[kk][e] = 0;
   for (int r0 = 0; r0 < l; r0 += kFewRows) {
     const int rows = min(kFewRows, l - r0);
-    if (r0) __syncthreads();
-    for (int t = tid; t < KCH * kFewRows; t += kFewThreads) {
-      const int kk = t / kFewRows, i = t % kFewRows;
-      uint32_t w = 0;
-      if (i < rows && k0 + kk < nkeys) {
-        w = y[(size_t)(k0 + kk) * l + r0 + i];
-        w = big ? y_residue(w, y_signed, q, mu) : w + bias;
-      }
-      ys[kk][i] = w;
+    if (r0 || !staged) {
+      __syncthreads();
+#pragma unroll
+      for (int kk = 0; kk < KCH; ++kk)
+        for (int i = tid; i < rows; i += kFewThreads) {
+          const uint32_t w = kk < keys ? a.y[(size_t)(k0 + kk) * l + r0 + i] : 0u;
+          sm.ys[kk][i] = WIDE ? y_residue(w, a.y_signed, q, mu) : w;
+        }
+      __syncthreads();
     }
-    __syncthreads();
     const uint32_t *vr = vb + (size_t)r0 * row;
     for (int i = slice; i < rows; i += 8 * slices) {
       uint4 x[8];
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
         const int r = i + u * slices;
-        x[u] = r < rows ? load4(vr + (size_t)r * row, vec) : make_uint4(0, 0, 0, 0);
+        x[u] = r < rows ? load4(vr + (size_t)r * row, a.vec) : make_uint4(0, 0, 0, 0);
       }
-      if (!big) {
+      if (!WIDE) {
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
-          sx[0] += x[u].x, sx[1] += x[u].y, sx[2] += x[u].z, sx[3] += x[u].w;
+          any |= x[u].x | x[u].y | x[u].z | x[u].w;
 #pragma unroll
           for (int kk = 0; kk < KCH; ++kk) {
-            const uint32_t yv = ys[kk][min(i + u * slices, kFewRows - 1)];
-            acc[kk][0] += (uint64_t)x[u].x * yv;
-            acc[kk][1] += (uint64_t)x[u].y * yv;
-            acc[kk][2] += (uint64_t)x[u].z * yv;
-            acc[kk][3] += (uint64_t)x[u].w * yv;
+            const int32_t yv = (int32_t)sm.ys[kk][min(i + u * slices, kFewRows - 1)];
+            acc[kk][0] += (uint64_t)((int64_t)(int32_t)x[u].x * yv);
+            acc[kk][1] += (uint64_t)((int64_t)(int32_t)x[u].y * yv);
+            acc[kk][2] += (uint64_t)((int64_t)(int32_t)x[u].z * yv);
+            acc[kk][3] += (uint64_t)((int64_t)(int32_t)x[u].w * yv);
           }
         }
       } else {
@@ -128,8 +133,8 @@ __global__ void __launch_bounds__(kFewThreads)
         for (int kk = 0; kk < KCH; ++kk)
 #pragma unroll
           for (int u = 0; u < 8; u += 2) {
-            const uint32_t y0 = ys[kk][min(i + u * slices, kFewRows - 1)];
-            const uint32_t y1 = ys[kk][min(i + (u + 1) * slices, kFewRows - 1)];
+            const uint32_t y0 = sm.ys[kk][min(i + u * slices, kFewRows - 1)];
+            const uint32_t y1 = sm.ys[kk][min(i + (u + 1) * slices, kFewRows - 1)];
             const uint64_t t[4] = {(uint64_t)x[u].x * y0 + (uint64_t)x[u + 1].x * y1,
                                    (uint64_t)x[u].y * y0 + (uint64_t)x[u + 1].y * y1,
                                    (uint64_t)x[u].z * y0 + (uint64_t)x[u + 1].z * y1,
@@ -143,30 +148,54 @@ __global__ void __launch_bounds__(kFewThreads)
       }
     }
   }
-  // add the slices of one key at a time (the bias first); the first `lanes` threads finish
+  if (!WIDE && __syncthreads_or((int32_t)any < 0)) return false;
+  const int cols = 4 * lanes;
 #pragma unroll
   for (int kk = 0; kk < KCH; ++kk) {
-    if (kk) __syncthreads();
+    if (kk >= keys) break;
+    __syncthreads();
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      red[tid][e] = big ? acc[kk][e] : (uint64_t)mod_u64(acc[kk][e], mu, q) + (q - mod_u64(sx[e] * bias, mu, q));
-      if (big) redh[tid][e] = hi[kk][e];
+      sm.red[slice * cols + 4 * lane + e] = acc[kk][e];
+      if (WIDE) sm.redh[slice * cols + 4 * lane + e] = hi[kk][e];
     }
     __syncthreads();
-    if (tid < lanes && k0 + kk < nkeys) {
-      uint32_t o[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
+    uint32_t *o = a.out + ((size_t)(z * (size_t)a.nkeys + k0 + kk) * 3 + m) * n + j0;
+    for (int i = tid; i < cols; i += kFewThreads) {
+      if (WIDE) {
         WideSum w;
         for (int s = 0; s < slices; ++s) {
-          w.add(red[s * lanes + tid][e]);
-          if (big) w.hi += redh[s * lanes + tid][e];
+          w.add(sm.red[s * cols + i]);
+          w.hi += sm.redh[s * cols + i];
         }
-        o[e] = w.mod(mu, q);
+        o[i] = w.mod(mu, q);
+      } else {
+        uint64_t t = 0;
+        for (int s = 0; s < slices; ++s) t += sm.red[s * cols + i];
+        o[i] = mod_s64((int64_t)t, mu, q);
       }
-      store4(out + ((size_t)(z * (size_t)nkeys + k0 + kk) * 3 + m) * n + j, make_uint4(o[0], o[1], o[2], o[3]), vec);
     }
   }
+  return true;
+}
+
+template <int KCH>
+__global__ void __launch_bounds__(kFewThreads, KCH == 4 ? 2 : KCH == 2 ? 3 : 4)
+    k_mac_few(const __grid_constant__ FewArgs a, const __grid_constant__ SchemeArgs sa) {
+  __shared__ FewSmem<KCH> sm;
+  const int l = sa.l, k0 = blockIdx.z * KCH, keys = min(KCH, a.nkeys - k0);
+  // y of the first rows staged and checked at once, the rows beyond them checked
+  bool big = false;
+#pragma unroll
+  for (int kk = 0; kk < KCH; ++kk)
+    for (int i = threadIdx.x; i < l; i += kFewThreads) {
+      const uint32_t w = kk < keys ? a.y[(size_t)(k0 + kk) * l + i] : 0u;
+      if (i < kFewRows) sm.ys[kk][i] = w;
+      big |= a.y_signed ? w + 32767u > 65534u : w > 32767u;
+    }
+  big = __syncthreads_or(big);
+  if (!big && few_sums<KCH, false>(a, sa, sm, true)) return;
+  few_sums<KCH, true>(a, sa, sm, false);
 }
 
 // ------------------------------------------------------------------ many keys
@@ -373,8 +402,10 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
       // through the free stages, so that rows of 256 bytes are stored whole
       uint32_t *row = reinterpret_cast<uint32_t *>(smem + (smem_b - smem_a)) + ((warp & 3) * 32 + lane) * kMmaPitch +
                       (warp >> 2) * 16;
+      const bool any = key0 + (warp & 3) * 32 < a.nkeys;  // whole warps
 #pragma unroll
       for (int h = 0; h < 16; h += 8) {
+        if (!any) break;
         uint32_t d[4][8];
 #pragma unroll
         for (int b = 0; b < 4; ++b)
@@ -417,17 +448,27 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
 
 }  // namespace
 
-// From this many keys on the tensor-core kernel is used; its time does not depend on their number up to
-// 128.  us on a B200 (n, l: streamed with 1, 2, 3, 4, 8 keys | tensor cores with 3): 4096, 784: 16.7,
-// 20.6, 29.6, 30.9, 49.4 | 26.8; 2048, 200: 9.0, 10.4, 14.4, 15.6, 18.6 | 8.6; 1024, 40: 6.1, 8.4,
-// 12.4, 14.2, 14.5 | 7.5.
-constexpr int kMmaMinKeys = 3;
+// Which kernel: estimated us on a B200, fitted to the measurements below.  Tensor cores: the CTAs walk
+// their coefficient tiles, 1.25 us per 128 slots and 1.5 per epilogue, whatever the number of keys
+// up to 128 per tile; streamed: v read at about 3.5 TB/s per 4 keys.  One or two keys are always
+// streamed.  us (streamed | tensor cores) at n, l, ciphertexts, keys: 4096, 37, 21, 3: 21 | 78; 2048, 53,
+// 26, 3: 22 | 52; 4096, 123, 36, 4: 70 | 127; 4096, 65, 17, 8: 43 | 66; 4096, 784, 4, 4: 60 | 65; 1024, 100, 30,
+// 6: 32 | 33; 4096, 100, 8, 16: 54 | 36; 4096, 784, 1, 8: 49 | 27; 1024, 40, 1, 32: 26 | 8.
+static bool use_mma(const Ctx &c, int nz, int nkeys) {
+  if (nkeys <= 2 || c.n < kMmaCols || c.l > kMmaMaxL) return false;
+  const int key_tiles = (nkeys + kMmaKeys - 1) / kMmaKeys;
+  const long long tiles = (long long)nz * (3 * c.n / kMmaCols);
+  const long long ctas = std::max(1LL, (long long)c.num_sms / key_tiles), rounds = (tiles + ctas - 1) / ctas;
+  const double mma = 6.0 + (double)rounds * (1.25 * ((c.l + kMmaK - 1) / kMmaK) + 1.5);
+  const double few = ((nkeys + 3) / 4) * (5.0 + (double)nz * c.l * 12.0 * c.n / 3.5e6);
+  return mma < few;
+}
 
 int mac_launch(Ctx &c, const SchemeArgs &sa, const uint32_t *d_v, size_t vstride, int nz, const uint32_t *d_y,
                int y_signed, int nkeys, uint32_t *d_out, cudaStream_t s) {
   const int n = c.n, l = c.l;
   const int vec = ((reinterpret_cast<uintptr_t>(d_v) | reinterpret_cast<uintptr_t>(d_out)) & 15u) == 0 && vstride % 4 == 0;
-  if (nkeys >= kMmaMinKeys && n >= kMmaCols && l <= kMmaMaxL) {
+  if (use_mma(c, nz, nkeys)) {
     MmaArgs a{d_v, vstride, d_y, y_signed, nkeys, nz, (nkeys + kMmaKeys - 1) / kMmaKeys, vec, d_out, {}};
     for (int j = 0; j < 3; ++j) {
       const uint64_t q = sa.ra.q[j];
@@ -445,17 +486,21 @@ int mac_launch(Ctx &c, const SchemeArgs &sa, const uint32_t *d_v, size_t vstride
   }
   const int kch = nkeys >= 3 ? 4 : nkeys;
   const int groups = (nkeys + kch - 1) / kch;
-  // 1 KB of a row per CTA where that leaves 8 CTAs per SM, else 256 bytes
-  int lanes = std::min(n / 4, 64);
-  if ((long long)nz * groups * 3 * n / (4 * lanes) < 8LL * c.num_sms) lanes = std::min(lanes, 16);
+  // About 64 rows or more per slice; fewer, and so more slices and CTAs, while there are not two CTAs
+  // per SM (1 key at n = 4096, l = 784: 12.5 us with 384 CTAs, 16.6 with 192).
+  int lanes = 256;
+  while (lanes > 16 && l / (kFewThreads / lanes) >= 128) lanes /= 2;
+  lanes = std::min(lanes, n / 4);
+  while (lanes > 8 && (long long)nz * groups * 3 * n / (4 * lanes) < 2LL * c.num_sms) lanes /= 2;
   const dim3 grid((unsigned)(3 * n / (4 * lanes)), (unsigned)nz, (unsigned)groups);
+  const FewArgs a{d_v, d_y, vstride, d_out, y_signed, nkeys, lanes, vec};
   note_launch();
   if (kch == 1)
-    k_mac_few<1><<<grid, kFewThreads, 0, s>>>(d_v, vstride, d_y, y_signed, nkeys, d_out, lanes, vec, sa);
+    k_mac_few<1><<<grid, kFewThreads, 0, s>>>(a, sa);
   else if (kch == 2)
-    k_mac_few<2><<<grid, kFewThreads, 0, s>>>(d_v, vstride, d_y, y_signed, nkeys, d_out, lanes, vec, sa);
+    k_mac_few<2><<<grid, kFewThreads, 0, s>>>(a, sa);
   else
-    k_mac_few<4><<<grid, kFewThreads, 0, s>>>(d_v, vstride, d_y, y_signed, nkeys, d_out, lanes, vec, sa);
+    k_mac_few<4><<<grid, kFewThreads, 0, s>>>(a, sa);
   CUFE_CUDA(cudaGetLastError());
   return CUFE_OK;
 }
