@@ -240,53 +240,86 @@ struct MmaArgs {
   int sh[3];
 };
 
-// The same tiles for keys with entries outside a signed byte: 96-bit sums of residue products,
-// 16 keys per thread, y staged 32 slots at a time.
-__device__ __noinline__ void mac_tiles_general(const MmaArgs &a, const SchemeArgs &sa, uint32_t *ystage, int key0,
+// The same tiles where a key has an entry outside a signed byte: Shoup products of the residues of y
+// (three 32-bit multiplications; a 64-bit multiply-add takes as long as four), two coefficients and
+// 8 keys per thread.  The 16 warps take the groups of 8 keys that hold keys, times slices of the
+// rows, 16 of them at a time each; the slices' residues are added at the end.
+__device__ __noinline__ void mac_tiles_general(const MmaArgs &a, const SchemeArgs &sa, uint8_t *smem, int key0,
                                                int first, int stride, int tiles) {
-  constexpr int KS = 32, PITCH = kMmaKeys + 4;
-  const int n = sa.ra.n, l = sa.l, per_z = 3 * n / kMmaCols;
-  const int c = threadIdx.x & (kMmaCols - 1), kg = threadIdx.x / kMmaCols;
+  constexpr int ROWS = 16, KT = 8, WARPS = kMmaThreads / 32, PER = ROWS * KT * WARPS / kMmaThreads;
+  uint2 *ystage = reinterpret_cast<uint2 *>(smem);      // (y, floor(y 2^32 / q)) of [row][key]
+  uint32_t *part = reinterpret_cast<uint32_t *>(smem);  // [slice][key][coefficient]
+  const int n = sa.ra.n, l = sa.l, per_z = 3 * n / kMmaCols, tid = threadIdx.x;
+  const int c = tid & 31, g = tid >> 5;
+  const int live = min(kMmaKeys, a.nkeys - key0);
+  int groups = 1;
+  while (groups * KT < live) groups *= 2;
+  const int slices = WARPS / groups, keys = KT * groups, pitch = keys + 2, rows = ROWS * slices;
+  const int kg = g % groups, sl = g / groups;
   for (int tile = first; tile < tiles; tile += stride) {
     const int z = tile / per_z, col = (tile - z * per_z) * kMmaCols, m = col / n;
     const uint32_t q = sa.ra.q[m];
     const uint64_t mu = sa.mu[m];
     const uint32_t *vb = a.v + z * a.vstride + col + c;
-    WideSum s[16];
-    for (int i0 = 0; i0 < l; i0 += KS) {
-      __syncthreads();
-      for (int t = threadIdx.x; t < KS * kMmaKeys; t += kMmaThreads) {
-        const int i = t % KS, k = t / KS;
-        ystage[i * PITCH + k] =
-            i0 + i < l && key0 + k < a.nkeys ? y_residue(a.y[(size_t)(key0 + k) * l + i0 + i], a.y_signed, q, mu) : 0u;
+    uint64_t s[KT][2];
+#pragma unroll
+    for (int k = 0; k < KT; ++k) s[k][0] = s[k][1] = 0;
+    uint32_t yn[PER];  // the y of the next rows, loaded while these are multiplied
+    const auto load_y = [&](int i0) {
+#pragma unroll
+      for (int u = 0; u < PER; ++u) {
+        const int t = tid + u * kMmaThreads, r = i0 + t % rows, k = t / rows;
+        yn[u] = r < l && k < live ? __ldg(a.y + (size_t)(key0 + k) * l + r) : 0u;
+      }
+    };
+    load_y(0);
+    for (int i0 = 0; i0 < l; i0 += rows) {
+      uint32_t x[ROWS][2];
+#pragma unroll
+      for (int i = 0; i < ROWS; ++i) {
+        const int r = i0 + sl * ROWS + i;
+        x[i][0] = r < l ? __ldg(vb + (size_t)r * 3 * n) : 0u;
+        x[i][1] = r < l ? __ldg(vb + (size_t)r * 3 * n + 32) : 0u;
       }
       __syncthreads();
-      for (int i = 0; i < KS; i += 4) {
-        uint32_t x[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) x[u] = i0 + i + u < l ? __ldg(vb + (size_t)(i0 + i + u) * 3 * n) : 0u;
+      for (int u = 0; u < PER; ++u) {
+        const int t = tid + u * kMmaThreads, i = t % rows, k = t / rows;
+        const uint32_t w = y_residue(yn[u], a.y_signed, q, mu);
+        const uint64_t ws = (uint64_t)w << 32, qe = __umul64hi(ws, mu);  // floor(ws / q) or one less
+        ystage[i * pitch + k] = make_uint2(w, (uint32_t)qe + (uint32_t)(ws - qe * q >= q));
+      }
+      __syncthreads();
+      load_y(i0 + rows);
 #pragma unroll
-        for (int g = 0; g < 4; ++g) {
+      for (int i = 0; i < ROWS; ++i)
 #pragma unroll
-          for (int u = 0; u < 4; u += 2) {
-            const uint4 w0 = *reinterpret_cast<const uint4 *>(ystage + (i + u) * PITCH + kg * 16 + 4 * g);
-            const uint4 w1 = *reinterpret_cast<const uint4 *>(ystage + (i + u + 1) * PITCH + kg * 16 + 4 * g);
-            s[4 * g].add((uint64_t)x[u] * w0.x + (uint64_t)x[u + 1] * w1.x);
-            s[4 * g + 1].add((uint64_t)x[u] * w0.y + (uint64_t)x[u + 1] * w1.y);
-            s[4 * g + 2].add((uint64_t)x[u] * w0.z + (uint64_t)x[u + 1] * w1.z);
-            s[4 * g + 3].add((uint64_t)x[u] * w0.w + (uint64_t)x[u + 1] * w1.w);
+        for (int e = 0; e < KT; e += 2) {
+          const uint4 w = *reinterpret_cast<const uint4 *>(ystage + (sl * ROWS + i) * pitch + kg * KT + e);
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            s[e][h] += shoup_lazy(x[i][h], w.x, w.y, q);
+            s[e + 1][h] += shoup_lazy(x[i][h], w.z, w.w, q);
           }
         }
-      }
     }
+    __syncthreads();
 #pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      const int key = key0 + kg * 16 + k;
-      if (key < a.nkeys)
-        a.out[(size_t)(z * (size_t)a.nkeys + key) * 3 * n + col + c] = s[k].mod(mu, q);
+    for (int k = 0; k < KT; ++k)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) part[(sl * keys + kg * KT + k) * kMmaCols + c + 32 * h] = mod_u64(s[k][h], mu, q);
+    __syncthreads();
+    for (int t = tid; t < live * kMmaCols; t += kMmaThreads) {
+      uint64_t sum = 0;
+      for (int u = 0; u < slices; ++u) sum += part[u * keys * kMmaCols + t];
+      a.out[(size_t)(z * (size_t)a.nkeys + key0 + t / kMmaCols) * 3 * n + col + t % kMmaCols] = mod_u64(sum, mu, q);
     }
+    __syncthreads();
   }
 }
+static_assert(16 * 16 * (8 + 2) * 8 <= 2 * kMmaStage && 16 * (128 + 2) * 8 <= 2 * kMmaStage &&
+                  128 * kMmaCols * 4 <= 2 * kMmaStage,
+              "the general tiles' staging");
 
 __global__ void __launch_bounds__(kMmaThreads, 1) 
     k_mac_mma(const __grid_constant__ MmaArgs a, const __grid_constant__ SchemeArgs sa, uint32_t *__restrict__ status) {
@@ -361,7 +394,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
   uint32_t tmem;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(slot));
   if (bad) {
-    mac_tiles_general(a, sa, reinterpret_cast<uint32_t *>(smem + (smem_b - smem_a)), key0, first, stride, tiles);
+    mac_tiles_general(a, sa, smem + (smem_b - smem_a), key0, first, stride, tiles);
   } else {
     bool live = true;
     int tile = first, ch = 0;
