@@ -29,14 +29,17 @@ __device__ __forceinline__ uint32_t xtime_u8(uint32_t b) {
   return ((b << 1) ^ ((b & 0x80u) ? 0x1bu : 0u)) & 0xffu;
 }
 
-// fill the replicated tables (all threads of the CTA; caller syncs)
+// fill the replicated tables (all threads of the CTA, a multiple of 16; caller syncs): 16 threads
+// write the 256 bytes of one entry of a pair of tables, 16 bytes each
 __device__ __forceinline__ void aes_fill_tables() {
-  for (uint32_t i = threadIdx.x + threadIdx.y * blockDim.x; i < kAesTableBytes / 4; i += blockDim.x * blockDim.y) {
-    const uint32_t region = i >> 14, x = (i >> 6) & 255, t1 = (i >> 5) & 1;
-    const uint32_t t = region * 2 + t1;
-    const uint32_t s = c_sbox[x];
-    const uint32_t te0 = (xtime_u8(s) << 24) | (s << 16) | (s << 8) | (xtime_u8(s) ^ s);
-    asm volatile("st.shared.u32 [%0], %1;" ::"r"(kAesTables + 4 * i), "r"(__funnelshift_r(te0, te0, 8 * t)) : "memory");
+  const uint32_t tid = threadIdx.x + threadIdx.y * blockDim.x, piece = tid & 15u;
+  for (uint32_t x = tid >> 4; x < 256; x += (blockDim.x * blockDim.y) >> 4) {
+    const uint32_t s = c_sbox[x], d = xtime_u8(s);
+    const uint32_t te0 = (d << 24) | (s << 16) | (s << 8) | (d ^ s);
+    const uint32_t lo = piece & 8u ? __funnelshift_r(te0, te0, 8) : te0, hi = __funnelshift_r(lo, lo, 16);
+    const uint32_t at = kAesTables + x * 256 + piece * 16;
+    asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(at), "r"(lo) : "memory");
+    asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(at + 65536), "r"(hi) : "memory");
   }
 }
 

@@ -966,9 +966,9 @@ int ctx_setup_gpu_map(Ctx &c, const uint8_t *seed2, const uint8_t *seed3, uint32
   aes_key_expand(seed2, keys.data());
   aes_key_expand(seed3, keys.data() + 60);
   CUFE_CUDA(cudaMemcpyAsync(rk, keys.data(), keys.size() * 4, cudaMemcpyHostToDevice, s));
-  rc = sample_gpu_map(0, rk, 0, l, n, d_msk, c.d_status, s);
+  rc = sample_gpu_map(0, rk, 0, l, n, d_msk, c.d_status, c.num_sms, s);
   if (rc) return rc;
-  rc = sample_gpu_map(0, rk + 60, 0, l, n, e, c.d_status, s);
+  rc = sample_gpu_map(0, rk + 60, 0, l, n, e, c.d_status, c.num_sms, s);
   if (rc) return rc;
   return setup_tail(c, l, d_mpk, d_msk, e, a_sh, s);
 }
@@ -1062,9 +1062,9 @@ int ctx_encrypt_gpu_map(Ctx &c, int batch, const uint32_t *d_x, const uint32_t *
   CUFE_CUDA(cudaMemcpyAsync(rk, keys, sizeof(keys), cudaMemcpyHostToDevice, s));
   // r and f_0 come from the same key and counters (src/rlwe_sife_gpu.cu:135-147), f_i from the
   // same key with polynomial index i (src/sample_gpu.cu:217-289); every instance shares them.
-  rc = sample_gpu_map(1, rk, 0, 1, n, r, c.d_status, s);
+  rc = sample_gpu_map(1, rk, 0, 1, n, r, c.d_status, c.num_sms, s);
   if (rc) return rc;
-  rc = sample_gpu_map(2, rk, 0, l, n, f3, c.d_status, s);
+  rc = sample_gpu_map(2, rk, 0, l, n, f3, c.d_status, c.num_sms, s);
   if (rc) return rc;
   CUFE_CUDA(cudaMemcpyAsync(rhat, r, poly * 4, cudaMemcpyDeviceToDevice, s));
   rc = ntt_fwd_shoup_launch(c.ring.args, rhat, rhat_sh, 3, s);
@@ -1384,7 +1384,7 @@ int ctx_sample_gpu_map(Ctx &c, int sig, const uint8_t *key, int poly0, int npoly
   uint32_t k[60];
   aes_key_expand(key, k);
   CUFE_CUDA(cudaMemcpyAsync(c.ws, k, sizeof(k), cudaMemcpyHostToDevice, s));
-  return sample_gpu_map(sig, reinterpret_cast<uint32_t *>(c.ws), poly0, npolys, c.n, d_out, c.d_status, s);
+  return sample_gpu_map(sig, reinterpret_cast<uint32_t *>(c.ws), poly0, npolys, c.n, d_out, c.d_status, c.num_sms, s);
 }
 
 int ctx_sample_polya(Ctx &c, const uint8_t *seed, uint32_t *d_a, cudaStream_t s) {

@@ -165,19 +165,22 @@ template <int SIG, bool FULL, int VAR>
 __global__ void __launch_bounds__(kCandThreads, 1)
     k_cand_cpu(const uint32_t *__restrict__ rkeys, SegDev sg, double kinv, uint32_t *__restrict__ cand_lo,
                uint8_t *__restrict__ amask, uint16_t *__restrict__ chs, uint32_t *__restrict__ status) {
+  // the host keeps the flattened refill count below 2^32 - 2^24 (no wrap of g)
+  const uint32_t total = (uint32_t)__ldg(sg.roff + sg.nstreams);
+  // A contiguous run of refills per warp (the counter cache's upper part lasts 2,730 refills); warps are
+  // dealt to the CTAs in turn, so that few refills spread over the SMs, where a warp alone is
+  // three times as fast as one of 16.
+  const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+  const uint32_t run = ((total + warps - 1) / warps + 31u) & ~31u;
+  if (blockIdx.x * run >= total) return;
   aes_fill_tables();
   __syncthreads();
   const AesCtx c = aes_ctx();
-  // the host keeps the flattened refill count below 2^32 - 2^24 (no wrap of g)
-  const uint32_t total = (uint32_t)__ldg(sg.roff + sg.nstreams);
   uint32_t rk[60];
   uint32_t st = 0;
   uint32_t lo = 1, hi = 0;  // refill range of stream st (empty: forces the first lookup)
   CtrCache cc;
-  // a contiguous run of refills per warp: the counter cache's upper part lasts 2,730 refills
-  const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-  const uint32_t run = ((total + warps - 1) / warps + 31u) & ~31u;
-  const uint32_t g0 = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * run, g1 = min(total, g0 + run);
+  const uint32_t g0 = ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * run, g1 = min(total, g0 + run);
   for (uint32_t g = g0 + (threadIdx.x & 31u); g < g1; g += 32u) {
     if (g < lo || g >= hi) {
       st = seg_find(sg.roff, sg.nstreams, g);
@@ -651,116 +654,196 @@ __global__ void k_seg_uniform(uint32_t nstreams, uint32_t calls, uint32_t n, uin
 
 // ------------------------------------------------------------------ GPU mapping
 
-// chained AES refill of the GPU mapping (src/AES.cuh:380-435): 18 blocks (bytes 0..287)
-// into buf; blocks 18..23 only when a uniform draw needs them.
-__device__ __forceinline__ void chain_blocks(uint32_t *buf, int from, int to, uint32_t &s0, uint32_t &s1,
-                                             uint32_t &s2, uint32_t &s3, const uint32_t (&rk)[60],
-                                             AesCtx c) {
-  for (int m = from; m < to; ++m) {
+// The GPU mapping's refills are independent of each other: refill rep of thread t (n / 8 threads per
+// polynomial, 8 samples each) starts at its own counter, poly * 5 T 24 + rep * T 24 + t 24 with
+// T = n / 8, and chains its blocks (src/AES.cuh:380-435).  A task is one thread's 8 samples; it needs
+// about 2.1 / 2.3 / 3.1 refills for S1 / S2 / S3.
+struct ChainRefill {
+  uint32_t z[8], y[8];  // low words of |candidate|; the uniform draws
+  uint32_t bits;        // accept mask, bits 32 (<< 8), wide flag (bit 16); k8 << 24
+};
+
+// One refill from its full words, block by block (rare: a uniform draw beyond the first 10 words or a
+// tied top word); the reference's order throughout.
+template <int SIG>
+__device__ __noinline__ void chain_refill_slow(uint32_t ctr, const uint32_t *__restrict__ rkg, AesCtx c, double kinv,
+                                               ChainRefill &r, uint32_t *status) {
+  uint32_t rk[60], buf[96];
+#pragma unroll
+  for (int i = 0; i < 60; ++i) rk[i] = __ldg(rkg + i);
+  uint32_t s0 = rk[0], s1 = rk[1], s2 = rk[2], s3 = ctr ^ rk[3];
+#pragma unroll 1
+  for (int m = 0; m < 24; ++m) {
     aes256_rounds(s0, s1, s2, s3, rk, c);
-    buf[4 * m] = s0;
-    buf[4 * m + 1] = s1;
-    buf[4 * m + 2] = s2;
-    buf[4 * m + 3] = s3;
+    buf[4 * m] = s0, buf[4 * m + 1] = s1, buf[4 * m + 2] = s2, buf[4 * m + 3] = s3;
+  }
+  int w = 50;  // uniform words from byte 200
+  const uint32_t k8 = buf[70] >> 24;  // byte 280
+  r.bits = k8 << 24;
+  for (int i = 0; i < 8; ++i) {
+    uint32_t x = 0;
+    for (;;) {
+      if (w >= 96) {
+        atomicOr(status, kStatusUniformOverrun);
+        x = 0;
+        break;
+      }
+      x = bswap32(buf[w++]);
+      if (uniform_ok<SIG>(x)) break;
+    }
+    r.y[i] = uniform_reduce<SIG>(x);
+  }
+  for (int ln = 0; ln < 8; ++ln) {
+    const int bw = (ln < 4 ? 0 : 25) + 2 * (ln & 3);
+    const uint32_t x = cdt_sample<false>(le64_of(buf[bw + 8], buf[bw + 9]), 0);
+    const uint32_t rexp = (buf[ln < 4 ? 24 : 49] >> (24 - 8 * (ln & 3))) & 0xffu;
+    uint64_t z;
+    const bool b = candidate<SIG, 2>(x, r.y[ln], le64_of(buf[bw + 16], buf[bw + 17]), rexp, kinv, z);
+    r.z[ln] = (uint32_t)z;
+    r.bits |= candidate_bits(ln, b, z, k8);
   }
 }
 
-// 512 threads: the 128 KB of tables allow one CTA per SM, and the chained blocks leave one
-// thread little independent work, so the CTA brings as many warps as the register file holds
+// A warp runs a contiguous range of tasks, `group` lanes (1 or 4) per task: with 1, a lane that has its
+// 8 samples takes the warp's next task at once, so no lane waits for the slowest of 32; with 4 the
+// lanes draw consecutive refills of one task, the shortest way through a call with few tasks.
+// Warps are dealt to the CTAs in turn, so that few warps spread over the SMs.
+//
+// A refill's 18 blocks are a serial chain, so they come in order and what needs a later word waits in
+// registers: CDT samples and top Bernoulli words until the uniform draws (blocks 12..14), the
+// candidates until the sign byte (block 17).  Top words decide as in the CPU mapping (k_cand_cpu).
+// Bound by the table lookups: 4,020 per refill, 16 cycles of a warp's round against 12 of the ALU.
+// One CTA of 512 tasks with its own tables, a buffered keystream and lanes that waited for the slowest
+// of their warp took 901 us for 785 polynomials of S3 and 159 for one of S2 on a B200 (n = 4096); now 525 and 20.
 constexpr int kGpuMapThreads = 512;
 template <int SIG>
 __global__ void __launch_bounds__(kGpuMapThreads, 1)
-    k_gauss_gpu_map(const uint32_t *__restrict__ rkey, uint32_t poly0, uint32_t npolys, uint32_t n, double kinv,
-                    ModArgs m, uint32_t *__restrict__ out, uint32_t *__restrict__ status) {
+    k_gauss_gpu_map(const uint32_t *__restrict__ rkey, uint32_t poly0, uint32_t tasks, uint32_t n, uint32_t run,
+                    uint32_t group, double kinv, ModArgs m, uint32_t *__restrict__ out, uint32_t *__restrict__ status) {
+  const uint32_t T = n / 8, lane = threadIdx.x & 31u;
+  if ((uint64_t)blockIdx.x * run >= tasks) return;  // no task for this CTA's first warp, nor for the others
   aes_fill_tables();
   __syncthreads();
+  const uint32_t wi = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+  const uint64_t first = (uint64_t)wi * run;
+  if (first >= tasks) return;
+  const uint32_t end = (uint32_t)min((uint64_t)tasks, first + run);
+  uint32_t next = (uint32_t)first;
   const AesCtx c = aes_ctx();
   uint32_t rk[60];
 #pragma unroll
   for (int i = 0; i < 60; ++i) rk[i] = __ldg(rkey + i);
-  const uint32_t T = n / 8;
-  const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
-  if (gid >= npolys * T) return;
-  const uint32_t p = gid / T, t = gid - p * T, poly = poly0 + p;
-  uint32_t buf[96];
-  uint32_t y[8], x[8], acc = 0, k8 = 0;
-  uint64_t z[8];
-  uint32_t i = 8, rep = 0;
-  uint32_t *o = out + (size_t)p * 3 * n;
-  bool gave_up = false;
-  for (uint32_t j = 0; j < 8 && !gave_up; ++j) {
-    uint32_t k = 0;
-    for (;;) {
-      if (i == 8) {
-        if (rep >= kMaxRefillsPerThread) {  // never reached by a working sampler; bounded anyway
-          atomicOr(status, kStatusRefillCap);
-          gave_up = true;
-          break;
-        }
-        const uint32_t ctr = poly * 5u * T * 24u + rep * T * 24u + t * 24u;
-        uint32_t s0 = rk[0], s1 = rk[1], s2 = rk[2], s3 = ctr ^ rk[3];
-        aes256_rounds(s0, s1, s2, s3, rk, c);
-        buf[0] = s0; buf[1] = s1; buf[2] = s2; buf[3] = s3;
-        chain_blocks(buf, 1, 18, s0, s1, s2, s3, rk, c);
-        int have = 18;
-        // uniform words from byte 200 (word 50)
-        int w = 0;
-        for (int jj = 0; jj < 8; ++jj) {
-          uint32_t xx;
-          for (;;) {
-            const int wi = 50 + w;
-            if (wi >= 96) {
-              atomicOr(status, kStatusUniformOverrun);
-              xx = 0;
-              break;
-            }
-            if ((wi >> 2) >= have) {
-              chain_blocks(buf, have, have + 1, s0, s1, s2, s3, rk, c);
-              ++have;
-            }
-            xx = bswap32(buf[wi]);
-            ++w;
-            if (uniform_ok<SIG>(xx)) break;
-          }
-          y[jj] = uniform_reduce<SIG>(xx);
-        }
-        for (int h = 0; h < 2; ++h) {
-          const int bw = 25 * h;  // word offset of r + 100*h
-          for (int ln = 0; ln < 4; ++ln) {
-            const uint64_t r2 = ((uint64_t)bswap32(buf[bw + 8 + 2 * ln])) |
-                                ((uint64_t)bswap32(buf[bw + 9 + 2 * ln]) << 32);
-            x[4 * h + ln] = cdt_sample<false>(r2, 0);
-          }
-        }
-        k8 = buf[70] >> 24;  // byte 280
-        acc = 0;
-        for (int h = 0; h < 2; ++h) {
-          const int bw = 25 * h;
-          const uint32_t ew = buf[bw + 24];  // bytes 96..99 (+100 h)
-          for (int ln = 0; ln < 4; ++ln) {
-            const uint64_t rm = ((uint64_t)bswap32(buf[bw + 16 + 2 * ln])) |
-                                ((uint64_t)bswap32(buf[bw + 17 + 2 * ln]) << 32);
-            const uint32_t rexp = (ew >> (24 - 8 * ln)) & 0xffu;
-            uint64_t zz;
-            const bool b = candidate<SIG, 2>(x[4 * h + ln], y[4 * h + ln], rm, rexp, kinv, zz);
-            z[4 * h + ln] = zz;
-            acc |= (uint32_t)b << (4 * h + ln);
-          }
-        }
-        i = 0;
-        ++rep;
-      }
-      k = (k8 >> i) & 1u;
-      ++i;
-      if (accept_final((acc >> (i - 1)) & 1u, z[i - 1], k)) break;
+  const uint32_t leader = lane & ~(group - 1u), rank = lane & (group - 1u);
+  uint32_t task = 0xffffffffu, rep = 0, have = 0;  // the lane's task, the refills and samples it has
+  for (;;) {
+    // lanes without a task take the next ones of the warp's range
+    const uint32_t idle = __ballot_sync(0xffffffffu, task == 0xffffffffu && rank == 0);
+    if (task == 0xffffffffu) {
+      const uint32_t at = next + __popc(idle & ((1u << leader) - 1u));
+      if (at < end) task = at, rep = 0, have = 0;
     }
-    if (gave_up) break;
-    const uint64_t zs = z[i - 1];  // K x + y < 8K < 2^33
-    if (zs >> 33) atomicOr(status, kStatusWideSample);
-    const uint32_t pos = 8 * t + j;
+    next += __popc(idle);
+    const bool live = task != 0xffffffffu;
+    if (!__any_sync(0xffffffffu, live)) break;
+    const uint32_t p = live ? task / T : 0u, t = live ? task - p * T : 0u;
+    const uint32_t ctr = (poly0 + p) * 5u * T * 24u + (rep + rank) * T * 24u + t * 24u;
+    uint32_t s0 = rk[0], s1 = rk[1], s2 = rk[2], s3 = ctr ^ rk[3];
+    uint32_t y[8], rm[8], zl[8];
 #pragma unroll
-    for (int jj = 0; jj < 3; ++jj)
-      o[jj * n + pos] = residue_parts((uint32_t)zs, (uint32_t)(zs >> 32) & 1u, k, m, jj);
+    for (int i = 0; i < 8; ++i) y[i] = 0;
+    uint32_t rej = 0, xp = 0, e0 = 0, e1 = 0, w34 = 0, bits = 0, open = 0, k8 = 0;
+#pragma unroll 1
+    for (int blk = 0; blk < 18; ++blk) {
+      aes256_rounds(s0, s1, s2, s3, rk, c);
+      if (blk == 2 || blk == 3 || blk == 9 || blk == 10) {  // top CDT words of two lanes
+        const uint32_t la = blk == 2 ? 0u : blk == 3 ? 2u : blk == 9 ? 5u : 4u, lb = blk == 10 ? 7u : la + 1u;
+        const uint32_t wa = blk < 4 ? s1 : blk == 9 ? s0 : w34, wb = blk < 4 ? s3 : blk == 9 ? s2 : s0;
+        bool ta, tb;
+        xp |= (cdt_sample_top(bswap32(wa), ta) << (4u * la)) | (cdt_sample_top(bswap32(wb), tb) << (4u * lb));
+        open |= (uint32_t)(ta | tb);
+        if (blk == 10) rm[4] = s2;
+      } else if (blk == 4) {
+        rm[0] = s1, rm[1] = s3;
+      } else if (blk == 5) {
+        rm[2] = s1, rm[3] = s3;
+      } else if (blk == 6) {
+        e0 = s0;
+      } else if (blk == 8) {
+        w34 = s2;
+      } else if (blk == 11) {
+        rm[5] = s0, rm[6] = s2;
+      } else if (blk == 12) {
+        rm[7] = s0, e1 = s1;
+        uniform_step<SIG, 0>(y, rej, s2);
+        uniform_step<SIG, 1>(y, rej, s3);
+      } else if (blk == 13) {
+        uniform_step<SIG, 2>(y, rej, s0);
+        uniform_step<SIG, 3>(y, rej, s1);
+        uniform_step<SIG, 4>(y, rej, s2);
+        uniform_step<SIG, 5>(y, rej, s3);
+      } else if (blk == 14) {
+        uniform_step<SIG, 6>(y, rej, s0);
+        uniform_step<SIG, 7>(y, rej, s1);
+        uniform_step<SIG, 8>(y, rej, s2);
+        uniform_step<SIG, 9>(y, rej, s3);
+      } else if (blk == 17) {
+        k8 = s2 >> 24;  // byte 280
+      }
+    }
+    // the candidates, two at a time through one body
+#pragma unroll 1
+    for (uint32_t ln = 0; ln < 8; ln += 2) {
+      uint64_t za, zb;
+      bool ta, tb;
+      const uint64_t va = candidate_input<SIG>(xp & 15u, y[0], za);
+      const uint64_t vb = candidate_input<SIG>((xp >> 4) & 15u, y[1], zb);
+      const bool ba = bernoulli_accept_top<SIG, 2>(va, bswap32(rm[0]), e0 >> 24, kinv, ta);
+      const bool bb = bernoulli_accept_top<SIG, 2>(vb, bswap32(rm[1]), (e0 >> 16) & 0xffu, kinv, tb);
+      bits |= candidate_bits((int)ln, ba, za, k8) | candidate_bits((int)ln + 1, bb, zb, k8);
+      open |= (uint32_t)(ta | tb);
+#pragma unroll
+      for (int i = 0; i < 6; ++i) y[i] = y[i + 2], rm[i] = rm[i + 2], zl[i] = zl[i + 2];
+      zl[6] = (uint32_t)za;
+      zl[7] = (uint32_t)zb;
+      xp >>= 8;
+      e0 = ln == 2 ? e1 : e0 << 16;
+    }
+    if (live && (open | (uint32_t)(rej > 2))) {
+      ChainRefill r;
+      chain_refill_slow<SIG>(ctr, rkey, c, kinv, r, status);
+      bits = r.bits & 0x00ffffffu;
+      k8 = r.bits >> 24;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) zl[i] = r.z[i];
+    }
+    if (live && (bits & 0x10000u)) atomicOr(status, kStatusWideSample);
+    // positions: the samples of this task's earlier lanes come first
+    uint32_t cnt = live ? __popc(bits & 0xffu) : 0u, pos = have, total = cnt;
+    for (uint32_t d = 1; d < group; d <<= 1) {
+      const uint32_t o = __shfl_up_sync(0xffffffffu, total, d);
+      if (rank >= d) total += o;
+    }
+    pos += total - cnt;
+    have += __shfl_sync(0xffffffffu, total, leader + group - 1u);
+    if (live) {
+      uint32_t *o = out + (size_t)p * 3 * n + 8 * t;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (((bits >> i) & 1u) && pos < 8) {
+#pragma unroll
+          for (int j = 0; j < 3; ++j)
+            o[j * n + pos] = residue_parts(zl[i], (bits >> (8 + i)) & 1u, (k8 >> i) & 1u, m, j);
+          ++pos;
+        }
+      }
+      rep += group;
+      if (have >= 8) {
+        task = 0xffffffffu;
+      } else if (rep >= kMaxRefillsPerThread) {  // never reached by a working sampler; bounded anyway
+        atomicOr(status, kStatusRefillCap);
+        task = 0xffffffffu;
+      }
+    }
   }
 }
 
@@ -1055,7 +1138,7 @@ int sample_cpu_map_seg(int sig, const SegDev &sg, const SegSizes &z, const uint3
   uint32_t *cstart = reinterpret_cast<uint32_t *>(take((z.calls + z.nstreams) * 4));
   const double kinv = kinv_of(sig);
   const uint32_t grid =
-      (uint32_t)std::min<uint64_t>((uint64_t)num_sms, (z.refills + kCandThreads - 1) / kCandThreads);
+      (uint32_t)std::min<uint64_t>((uint64_t)num_sms, (z.refills + 31) / 32);
   if (grid > 0) {
     ProfScope ps(sig == 0 ? "sample_cand_s1" : (sig == 1 ? "sample_cand_s2" : "sample_cand_s3"), s);
     if (sig == 0)
@@ -1128,20 +1211,25 @@ int sample_cpu_map(int sig, uint32_t nstreams, const uint32_t *d_rkeys, uint32_t
 }
 
 int sample_gpu_map(int sig, const uint32_t *d_rkey, uint32_t poly0, uint32_t npolys, uint32_t n, uint32_t *d_out,
-                   uint32_t *d_status, cudaStream_t s) {
-  const uint32_t threads = npolys * (n / 8);
-  const uint32_t grid = (threads + kGpuMapThreads - 1) / kGpuMapThreads;
+                   uint32_t *d_status, int num_sms, cudaStream_t s) {
+  const uint32_t tasks = npolys * (n / 8);
+  const uint32_t warps = (uint32_t)num_sms * (kGpuMapThreads / 32);
+  // 4 lanes per task while that leaves at most half of the warps a task group
+  const uint32_t group = (uint64_t)tasks * 4 <= (uint64_t)warps * 16 ? 4u : 1u;
+  const uint32_t run = std::max((tasks + warps - 1) / warps, 32u / group);
+  const uint32_t grid = std::min<uint32_t>((uint32_t)num_sms, (tasks + run - 1) / run);
   const double kinv = kinv_of(sig);
   ProfScope ps("sample_gpu_map", s);
+  note_launch();
   if (sig == 0)
-    note_launch(), k_gauss_gpu_map<0><<<grid, kGpuMapThreads, kAesSmemBytes, s>>>(d_rkey, poly0, npolys, n, kinv,
-                                                                               mod_args(), d_out, d_status);
+    k_gauss_gpu_map<0><<<grid, kGpuMapThreads, kAesSmemBytes, s>>>(d_rkey, poly0, tasks, n, run, group, kinv, mod_args(),
+                                                                   d_out, d_status);
   else if (sig == 1)
-    note_launch(), k_gauss_gpu_map<1><<<grid, kGpuMapThreads, kAesSmemBytes, s>>>(d_rkey, poly0, npolys, n, kinv,
-                                                                               mod_args(), d_out, d_status);
+    k_gauss_gpu_map<1><<<grid, kGpuMapThreads, kAesSmemBytes, s>>>(d_rkey, poly0, tasks, n, run, group, kinv, mod_args(),
+                                                                   d_out, d_status);
   else
-    note_launch(), k_gauss_gpu_map<2><<<grid, kGpuMapThreads, kAesSmemBytes, s>>>(d_rkey, poly0, npolys, n, kinv,
-                                                                               mod_args(), d_out, d_status);
+    k_gauss_gpu_map<2><<<grid, kGpuMapThreads, kAesSmemBytes, s>>>(d_rkey, poly0, tasks, n, run, group, kinv, mod_args(),
+                                                                   d_out, d_status);
   CUFE_CUDA(cudaGetLastError());
   return CUFE_OK;
 }

@@ -73,7 +73,7 @@ int sample_cpu_map_seg(int sig, const SegDev &sg, const SegSizes &z, const uint3
 // GPU counter mapping: polynomials poly0 .. poly0+npolys-1 of one key, residues to
 // d_out[npolys][3][n].
 int sample_gpu_map(int sig, const uint32_t *d_rkey, uint32_t poly0, uint32_t npolys, uint32_t n,
-                   uint32_t *d_out, uint32_t *d_status, cudaStream_t s);
+                   uint32_t *d_out, uint32_t *d_status, int num_sms, cudaStream_t s);
 
 // uniform a (sample_polya): d_a[3][n]
 int sample_polya(const uint32_t *d_rkey, uint32_t n, uint32_t *d_a, cudaStream_t s);
