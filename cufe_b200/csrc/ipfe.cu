@@ -515,6 +515,48 @@ __global__ void __launch_bounds__(NttPlan<LOGN>::T * ppc<LOGN>(), MINB)
   }
 }
 
+// Encryption where every instance has the same r and f (the GPU mapping: one seed for a call,
+// src/rlwe_sife_gpu.cu:102-188): the instances differ in floor(q/p) x_i only, so INTT(pk_r * r^) + f is
+// computed once per residue and written `batch` times with another constant added; CTAs of
+// blockIdx.y take a share of the instances each.  Bound by the ciphertexts' writes.  8 instances at
+// n = 4096, l = 785 on a B200: 274 us with an inverse transform per instance, now 80.
+template <int LOGN>
+__global__ void __launch_bounds__(NttPlan<LOGN>::T * ppc<LOGN>())
+    k_encrypt_shared(const uint32_t *__restrict__ mpk, const uint32_t *__restrict__ rhat,
+                     const uint32_t *__restrict__ rhat_sh, const uint32_t *__restrict__ f3,
+                     const uint32_t *__restrict__ f0, const uint32_t *__restrict__ x, uint32_t *__restrict__ ct,
+                     int batch, SchemeArgs sa) {
+  using P = NttPlan<LOGN>;
+  extern __shared__ uint32_t smem_u32[];
+  const int th = threadIdx.x, l = sa.l, nres = 3 * (l + 1);
+  const int rr = blockIdx.x * blockDim.y + threadIdx.y;
+  const bool act = rr < nres;
+  const int res = act ? rr : nres - 1, m = res % 3, i = res / 3;
+  const uint32_t q = sa.ra.q[m];
+  uint32_t *sm = smem_u32 + threadIdx.y * P::SMEM_WORDS;
+  uint32_t a[16], w[16], wsh[16];
+  load16(mpk + (size_t)res * P::N + th * 16, a);
+  load16(rhat + (size_t)m * P::N + th * 16, w);
+  load16(rhat_sh + (size_t)m * P::N + th * 16, wsh);
+#pragma unroll
+  for (int e = 0; e < 16; ++e) a[e] = shoup_mul(a[e], w[e], wsh[e], q);
+  ntt_inv_core<LOGN>(a, sm, th, q, sa.ra.ipsi2 + (size_t)m * P::N, sa.ra.ninv[m], sa.ra.ninv_sh[m], sa.ra.w1n[m],
+                     sa.ra.w1n_sh[m]);
+  if (!act) return;
+  const uint32_t *f = (i < l ? f3 + (size_t)i * 3 * P::N : f0) + (size_t)m * P::N;
+#pragma unroll
+  for (int e = 0; e < 16; ++e) a[e] = mod_add(a[e], f[P::template idx<0>(th, e)], q);
+  const int b0 = (int)((long long)batch * blockIdx.y / gridDim.y);
+  const int b1 = (int)((long long)batch * (blockIdx.y + 1) / gridDim.y);
+  uint32_t *c = ct + ((size_t)b0 * nres + res) * P::N + P::template idx_th<0>(th);
+  for (int b = b0; b < b1; ++b, c += (size_t)nres * P::N) {
+    uint32_t msg = 0;
+    if (i < l) msg = shoup_mul(mod_u64(x[(size_t)b * l + i], sa.mu[m], q), sa.delta_mod[m], sa.delta_sh[m], q);
+#pragma unroll
+    for (int e = 0; e < 16; ++e) c[P::template idx_e<0>(e)] = mod_add(a[e], msg, q);
+  }
+}
+
 // Decryption (src/rlwe_sife.c:248-278), d_y = sum_i y_i c_i - INTT(NTT(c_l) NTT(sk_y)): the
 // l-sums come from mac_launch; k_dec_tail subtracts the negacyclic product c_l * sk_y from them,
 // in place.
@@ -567,7 +609,8 @@ __global__ void k_decode(const uint32_t *__restrict__ dy, int count, int ncoeff,
 //   d_y[0] = sum_i y_i c_i[0] - (c_l * sk_y)[0],
 //   (c_l * sk_y)[0] = c_l[0] sk_y[0] - sum_{t=1}^{n-1} c_l[t] sk_y[n-t]   (negacyclic),
 // equal to coefficient 0 of the full decryption (src/rlwe_sife.c:248-286) residue for residue.
-// One CTA per (ciphertext, key); reads l + 2n words per modulus instead of (l+1) n.
+// One CTA per (ciphertext, key); reads l + 2n words per modulus instead of (l+1) n.  Without out the
+// residues go to d0 only (k_decode_triples follows).
 __global__ void __launch_bounds__(256)
     k_dec_coef0(const uint32_t *__restrict__ ct, const uint32_t *__restrict__ y, int y_signed, int nkeys,
                 const uint32_t *__restrict__ sky, uint32_t *__restrict__ d0, uint32_t *__restrict__ out,
@@ -600,7 +643,7 @@ __global__ void __launch_bounds__(256)
       d0[(size_t)blockIdx.x * 3 + 1] = r[1];
       d0[(size_t)blockIdx.x * 3 + 2] = r[2];
     }
-    out[blockIdx.x] = decode_one(r[0], r[1], r[2], dd);
+    if (out) out[blockIdx.x] = decode_one(r[0], r[1], r[2], dd);
   }
 }
 
@@ -616,7 +659,7 @@ __global__ void __launch_bounds__(256)
 // Tile shapes (ciphertexts x keys): 64 x 32, 64 x 64, 32 x 32, 32 x 64; the context's tuner picks per
 // (ciphertexts, keys).  The first gives way to the tensor-core product (coef0.cu) where that can run.
 constexpr int kC0Kc = 32;
-constexpr int kCoef0TiledMinKeys = 32;  // fewer keys never take the integer tiles untuned
+constexpr int kCoef0TiledMinKeys = 32;  // fewer keys take neither the integer tiles nor a separate decode untuned
 constexpr int kCoef0Forms = 5;          // 0 per pair, 1..4 the tile shapes below
 template <int TM, int R>
 __device__ __forceinline__ int c0_swz(int kk, int i) {
@@ -1069,7 +1112,20 @@ int ctx_encrypt_gpu_map(Ctx &c, int batch, const uint32_t *d_x, const uint32_t *
   CUFE_CUDA(cudaMemcpyAsync(rhat, r, poly * 4, cudaMemcpyDeviceToDevice, s));
   rc = ntt_fwd_shoup_launch(c.ring.args, rhat, rhat_sh, 3, s);
   if (rc) return rc;
-  return encrypt_tail(c, batch, d_x, d_mpk, rhat, rhat_sh, 0, f3, 0, r, 0, d_ct, s);
+  const SchemeArgs sa = scheme_args(c);
+  return dispatch_logn(c.ring.logn, [&](auto L) {
+    constexpr int LOGN = decltype(L)::value;
+    constexpr int G = ppc<LOGN>();
+    ProfScope ps("encrypt_intt", s);
+    const unsigned ctas = (unsigned)((3 * (l + 1) + G - 1) / G);
+    // shares of the instances: enough CTAs for four per SM
+    const unsigned shares = std::max(1u, std::min((unsigned)batch, ((unsigned)c.num_sms * 4 + ctas - 1) / ctas));
+    CUFE_CUDA(cudaFuncSetAttribute(k_encrypt_shared<LOGN>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
+    note_launch(), k_encrypt_shared<LOGN><<<dim3(ctas, shares), dim3(NttPlan<LOGN>::T, G), G * NttPlan<LOGN>::SMEM_WORDS * 4, s>>>(
+        d_mpk, rhat, rhat_sh, f3, r, d_x, d_ct, batch, sa);
+    CUFE_CUDA(cudaGetLastError());
+    return (int)CUFE_OK;
+  });
 }
 
 int ctx_keygen(Ctx &c, int nkeys, const uint32_t *d_y, int y_signed, const uint32_t *d_msk, uint32_t *d_sky,
@@ -1357,7 +1413,25 @@ int ctx_decrypt_coef0(Ctx &c, int nct, const uint32_t *d_ct, int nkeys, const ui
   // n = 2048, l = 124: 64 x 8 pairs 18 | 23 | 185, 1,000 x 1 28 | 35 | 213, 64 x 32 43 | 23 | 218, 200 x 64
   // 219 | 26 | 223, 1,000 x 500 8178 | 88 | 1261; n = 4096, l = 784: 64 x 8 33 | 30 | 411
   const long long pairs = (long long)nct * nkeys;
-  int form = !d_d0 && coef0_mma_ok(c) ? (pairs >= 1024 ? 1 : 0) : (nkeys >= kCoef0TiledMinKeys && pairs >= 12800 ? 1 : 0);
+  const bool mma = !d_d0 && coef0_mma_ok(c);
+  if (it == c.coef0_form.end() && nct >= 1 && nkeys >= kCoef0TiledMinKeys && pairs < (mma ? 1024 : 12800)) {
+    // many keys, few pairs: per pair, but the decodes by one kernel instead of one thread per CTA
+    uint32_t *d0 = d_d0;
+    if (!d0) {
+      const int rc = c.ensure_ws((size_t)pairs * 12);
+      if (rc) return rc;
+      d0 = reinterpret_cast<uint32_t *>(c.ws);
+    }
+    ProfScope ps("decrypt_coef0", s);
+    const DecodeArgs dd = decode_args(c);
+    note_launch(), k_dec_coef0<<<(unsigned)pairs, 256, 0, s>>>(d_ct, d_y, y_signed, nkeys, d_sky, d0, nullptr,
+                                                               scheme_args(c), dd);
+    CUFE_CUDA(cudaGetLastError());
+    note_launch(), k_decode_triples<<<(unsigned)((pairs + 255) / 256), 256, 0, s>>>(d0, pairs, d_out, dd);
+    CUFE_CUDA(cudaGetLastError());
+    return CUFE_OK;
+  }
+  int form = mma ? (pairs >= 1024 ? 1 : 0) : (nkeys >= kCoef0TiledMinKeys ? 1 : 0);
   if (it != c.coef0_form.end()) form = it->second;
   return ctx_decrypt_coef0_form(c, form, nct, d_ct, nkeys, d_y, y_signed, d_sky, d_d0, d_out, s);
 }
