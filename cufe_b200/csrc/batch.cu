@@ -856,8 +856,8 @@ struct Server {
   static uint64_t enc_scratch_bytes(uint32_t n, uint32_t l) {
     const uint64_t poly = (uint64_t)3 * n * 4;
     const uint64_t R3 = cpu_map_refills(l, n, 2), R2 = cpu_map_refills(2, n, 1);
-    // sampler scratch: 39 B per refill (candidate low words 32, accept mask 1, bit-32 and sign
-    // bytes 2, prefix 4) plus tiles and call starts; 44 leaves room for the per-tile terms
+    // sampler scratch: 35 B per refill (candidate low words 32, accept mask 1, bit-32 and sign
+    // bytes 2) plus call starts; admission charges 44
     return poly * (2 + 2 + l) + std::max(R3, R2) * 44 + 2 * 60 * 4 + 8192;
   }
 
@@ -1110,9 +1110,6 @@ struct Server {
       uint32_t *rhsh = reinterpret_cast<uint32_t *>(take(w_rh * 4));
       uint32_t *f3 = reinterpret_cast<uint32_t *>(take(w_f3 * 4));
       uint32_t *rk = reinterpret_cast<uint32_t *>(take((size_t)2 * ne * 60 * 4));
-      const size_t before = (size_t)(p - d_scr);
-      if (before + std::max(seg_scratch_bytes(z2), seg_scratch_bytes(z3)) > scr_bytes)
-        z2.doubling = z3.doubling = false;  // no room for the doubling tables: serial walk
       void *samp = take(std::max(seg_scratch_bytes(z2), seg_scratch_bytes(z3)));
       if ((size_t)(p - d_scr) > scr_bytes) {
         set_last_error("server: tick scratch exceeded");

@@ -7,8 +7,8 @@
 //    the accepted candidates in order and drops the rest of its last refill.  The stream is
 //    sequential by construction, so it is computed in three parallel phases: (1) every
 //    refill's 8 candidates and accept mask for a generous refill range (the AES work, one
-//    thread per refill), (2) a per-stream exclusive scan of accept counts and a one-warp
-//    walk that finds where each call starts (each call starts at a fresh refill), (3) a
+//    thread per refill), (2) a walk per stream over the accept counts that finds where each
+//    call starts (each call starts at a fresh refill), (3) a
 //    scatter of the accepted candidates to their coefficient positions as residues.
 //  * GPU mapping (src/sample_gpu.cu, src/AES.cuh): thread t of polynomial p owns coefficients
 //    8t..8t+7 and draws chained-AES refills from counter p*5*T*24 + rep*T*24 + t*24.
@@ -27,6 +27,29 @@ namespace {
 
 __device__ __forceinline__ uint64_t le64_of(uint32_t be_lo, uint32_t be_hi) {
   return (uint64_t)bswap32(be_lo) | ((uint64_t)bswap32(be_hi) << 32);
+}
+
+// ------------------------------------------------------------------ segment tables
+
+// The tables of a run with different streams, or the arithmetic of one with equal streams
+__device__ __forceinline__ uint32_t seg_n(const SegDev &sg, uint32_t st) { return sg.n ? __ldg(sg.n + st) : sg.u_n; }
+__device__ __forceinline__ uint32_t seg_calls(const SegDev &sg, uint32_t st) {
+  return sg.n ? __ldg(sg.calls + st) : sg.u_calls;
+}
+__device__ __forceinline__ uint64_t seg_roff(const SegDev &sg, uint32_t st) {
+  return sg.n ? __ldg(sg.roff + st) : (uint64_t)st * sg.u_refills;
+}
+__device__ __forceinline__ uint64_t seg_coff(const SegDev &sg, uint32_t st) {
+  return sg.n ? __ldg(sg.coff + st) : (uint64_t)st * sg.u_calls;
+}
+__device__ __forceinline__ uint64_t seg_ooff(const SegDev &sg, uint32_t st) {
+  return sg.n ? __ldg(sg.ooff + st) : st * sg.u_ostride;
+}
+__device__ __forceinline__ uint32_t seg_of_refill(const SegDev &sg, uint32_t g) {
+  return sg.n ? seg_find(sg.roff, sg.nstreams, g) : g / sg.u_refills;
+}
+__device__ __forceinline__ uint32_t seg_of_call(const SegDev &sg, uint32_t c) {
+  return sg.n ? seg_find(sg.coff, sg.nstreams, c) : c / sg.u_calls;
 }
 
 // ------------------------------------------------------------------ CPU mapping, phase 1
@@ -166,7 +189,7 @@ __global__ void __launch_bounds__(kCandThreads, 1)
     k_cand_cpu(const uint32_t *__restrict__ rkeys, SegDev sg, double kinv, uint32_t *__restrict__ cand_lo,
                uint8_t *__restrict__ amask, uint16_t *__restrict__ chs, uint32_t *__restrict__ status) {
   // the host keeps the flattened refill count below 2^32 - 2^24 (no wrap of g)
-  const uint32_t total = (uint32_t)__ldg(sg.roff + sg.nstreams);
+  const uint32_t total = (uint32_t)seg_roff(sg, sg.nstreams);
   // A contiguous run of refills per warp (the counter cache's upper part lasts 2,730 refills); warps are
   // dealt to the CTAs in turn, so that few refills spread over the SMs, where a warp alone is
   // three times as fast as one of 16.
@@ -183,9 +206,9 @@ __global__ void __launch_bounds__(kCandThreads, 1)
   const uint32_t g0 = ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * run, g1 = min(total, g0 + run);
   for (uint32_t g = g0 + (threadIdx.x & 31u); g < g1; g += 32u) {
     if (g < lo || g >= hi) {
-      st = seg_find(sg.roff, sg.nstreams, g);
-      lo = (uint32_t)__ldg(sg.roff + st);
-      hi = (uint32_t)__ldg(sg.roff + st + 1);
+      st = seg_of_refill(sg, g);
+      lo = (uint32_t)seg_roff(sg, st);
+      hi = (uint32_t)seg_roff(sg, st + 1);
 #pragma unroll
       for (int i = 0; i < 60; ++i) rk[i] = __ldg(rkeys + (size_t)st * 60 + i);
       ctr_cache_key(cc, rk, c);
@@ -290,265 +313,343 @@ __global__ void __launch_bounds__(kCandThreads, 1)
 
 // ------------------------------------------------------------------ CPU mapping, phase 2
 
-constexpr int kScanTile = 4096;  // refills per scan tile (512 threads x 8)
+// Call c of a stream starts at a fresh refill a_c and ends with the first refill e whose inclusive
+// count of accepted candidates reaches E(a_c) + n; a_{c+1} = e + 1.  call_start of stream st:
+// coff[st] + st .. coff[st+1] + st (calls + 1 entries; the last is the end of the last call).
+//
+// Short runs: k_walk, below, one CTA per stream.  Long runs: by the overshoot.  A call ends up to 7
+// samples beyond its n, and call c ends where the count reaches (c + 1) n + s, s being the overshoot of the
+// calls before it: a number close to c times its mean.  So the refill that ends call c can be
+// written down beforehand for every s in a window around that (k_ends: every refill writes itself
+// to the at most 8 thresholds that it reaches), and what remains serial is one table read per call
+// (k_chain).  The table is W words per call; s outside of the window is searched for directly.
+// 785 calls of n = 4096 from one stream: 3 + 10 + 54 us where scanning the counts and walking over them
+// in memory took 124; of 40 streams: 12 + 108 + 54 against 731, the chain being bound by the latency of
+// one step (a shared-memory read and ten instructions, 69 ns) and k_ends by its instructions.
+struct EndTable {
+  uint32_t *ends;   // [call][W]: refill | overshoot << 28
+  uint32_t *counts; // [stream][max_tiles]: accepted candidates per tile
+  uint32_t W, max_tiles, mean;  // mean overshoot, 16 fractional bits
+};
+constexpr int kCountTile = 4096;
 
-// per-tile exclusive scan of accept counts: elocal[g] (within the tile), tile_sum[tile];
-// one CTA per tile of the flattened tile space
-__global__ void __launch_bounds__(512) k_scan_tiles(const uint8_t *__restrict__ amask, SegDev sg,
-                                                    uint32_t *__restrict__ elocal, uint32_t *__restrict__ tile_sum) {
-  __shared__ uint32_t wsum[16];
-  const uint32_t T = blockIdx.x;
-  const uint32_t st = seg_find(sg.toff, sg.nstreams, T);
-  const uint64_t r0 = __ldg(sg.roff + st), R = __ldg(sg.roff + st + 1) - r0;
-  const uint64_t base = (uint64_t)(T - __ldg(sg.toff + st)) * kScanTile + threadIdx.x * 8;
-  uint32_t cnt[8], tot = 0;
-  // whole runs at 8-byte aligned masks and 16-byte aligned prefixes (every refill range of a
-  // uniform table in the 256-byte aligned scratch): one 8-byte load, two 16-byte stores
-  const bool vec = base + 8 <= R && (reinterpret_cast<uintptr_t>(amask + r0 + base) & 7u) == 0 &&
-                   (reinterpret_cast<uintptr_t>(elocal + r0 + base) & 15u) == 0;
-  if (vec) {
-    const uint2 m8 = __ldg(reinterpret_cast<const uint2 *>(amask + r0 + base));
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      cnt[i] = __popc((m8.x >> (8 * i)) & 0xffu);
-      cnt[4 + i] = __popc((m8.y >> (8 * i)) & 0xffu);
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const uint64_t t = base + i;
-      cnt[i] = t < R ? __popc(amask[r0 + t]) : 0u;
-    }
+// window of call c: s in [first, first + W)
+__device__ __forceinline__ uint32_t window_first(const EndTable &t, uint32_t c) {
+  const uint32_t mid = (uint32_t)(((uint64_t)t.mean * c) >> 16);
+  return mid > t.W / 2 ? mid - t.W / 2 : 0u;
+}
+
+// accept counts of tile blockIdx.x of stream blockIdx.y
+__global__ void __launch_bounds__(256) k_tile_counts(const uint8_t *__restrict__ amask, SegDev sg, EndTable t) {
+  __shared__ uint32_t wsum[8];
+  const uint64_t r0 = seg_roff(sg, blockIdx.y);
+  const uint32_t R = (uint32_t)(seg_roff(sg, blockIdx.y + 1) - r0), at = blockIdx.x * kCountTile + threadIdx.x * 16;
+  if (blockIdx.x * kCountTile >= R) return;
+  uint32_t n = 0;
+  if (at < R) {  // R and r0 are multiples of 32
+    const uint4 m = __ldg(reinterpret_cast<const uint4 *>(amask + r0 + at));
+    n = __popc(m.x) + __popc(m.y) + __popc(m.z) + __popc(m.w);
   }
-#pragma unroll
-  for (int i = 0; i < 8; ++i) tot += cnt[i];
-  // block exclusive scan of per-thread totals
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  uint32_t inc = tot;
+  n = __reduce_add_sync(0xffffffffu, n);
+  if ((threadIdx.x & 31u) == 0) wsum[threadIdx.x >> 5] = n;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    uint32_t v = 0;
+    for (int i = 0; i < 8; ++i) v += wsum[i];
+    t.counts[(size_t)blockIdx.y * t.max_tiles + blockIdx.x] = v;
+  }
+}
+
+// the table entries that the refills of tile blockIdx.x of stream blockIdx.y reach
+__global__ void __launch_bounds__(256) k_ends(const uint8_t *__restrict__ amask, SegDev sg, EndTable t) {
+  __shared__ uint32_t wsum[8], psum[8];
+  const uint32_t st = blockIdx.y, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint64_t r0 = seg_roff(sg, st);
+  const uint32_t R = (uint32_t)(seg_roff(sg, st + 1) - r0), at = blockIdx.x * kCountTile + threadIdx.x * 16;
+  if (blockIdx.x * kCountTile >= R) return;
+  uint32_t past = 0;  // accepted in the tiles before
+  for (uint32_t i = threadIdx.x; i < blockIdx.x; i += 256) past += __ldg(t.counts + (size_t)st * t.max_tiles + i);
+  uint4 m = make_uint4(0, 0, 0, 0);
+  if (at < R) m = __ldg(reinterpret_cast<const uint4 *>(amask + r0 + at));
+  const uint32_t own = __popc(m.x) + __popc(m.y) + __popc(m.z) + __popc(m.w);
+  uint32_t inc = own;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= o) inc += v;
+    if (lane >= (uint32_t)o) inc += v;
   }
-  if (lane == 31) wsum[wid] = inc;
+  past = __reduce_add_sync(0xffffffffu, past);
+  if (lane == 0) psum[warp] = past;
+  if (lane == 31) wsum[warp] = inc;
   __syncthreads();
-  if (wid == 0) {
-    uint32_t s = lane < 16 ? wsum[lane] : 0u, si = s;
+  uint32_t E = inc - own;
 #pragma unroll
-    for (int o = 1; o < 16; o <<= 1) {
-      const uint32_t v = __shfl_up_sync(0xffffffffu, si, o);
-      if (lane >= o) si += v;
-    }
-    if (lane < 16) wsum[lane] = si - s;
-    if (lane == 15) tile_sum[T] = si;
-  }
-  __syncthreads();
-  uint32_t run = wsum[wid] + inc - tot;
-  uint32_t ex[8];
+  for (uint32_t i = 0; i < 8; ++i) E += psum[i] + (i < warp ? wsum[i] : 0u);
+  // thresholds (c + 1) n + s in (E, E + own], c the call whose window they can lie in (end_table_width)
+  const uint32_t n = seg_n(sg, st), calls = seg_calls(sg, st);
+  // c + 1 to the nearest, (c + 1) (n + mean) - mean being the middle of call c's window
+  const double mean = (double)t.mean / 65536.0, inv = 1.0 / ((double)n + mean);
+  const uint32_t c1 = (uint32_t)(((double)(E + own / 2) + mean) * inv + 0.5);
+  if (c1 == 0 || c1 > calls || own == 0) return;
+  const uint32_t c = c1 - 1, lo = c1 * n + window_first(t, c), hi = lo + t.W;
+  if (E + own < lo || E >= hi) return;
+  uint32_t *row = t.ends + (seg_coff(sg, st) + c) * t.W;
+  const uint32_t w[4] = {m.x, m.y, m.z, m.w};
+#pragma unroll 1
+  for (uint32_t i = 0; i < 16; ++i) {
+    const uint32_t to = E + __popc((w[i >> 2] >> (8 * (i & 3u))) & 0xffu);
+    if (to >= lo && E < hi) {
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    ex[i] = run;
-    run += cnt[i];
-  }
-  if (vec) {
-    uint4 *o = reinterpret_cast<uint4 *>(elocal + r0 + base);
-    o[0] = make_uint4(ex[0], ex[1], ex[2], ex[3]);
-    o[1] = make_uint4(ex[4], ex[5], ex[6], ex[7]);
-  } else {
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-      if (base + i < R) elocal[r0 + base + i] = ex[i];
-  }
-}
-
-// exclusive scan of the tile sums of each stream (one block per stream)
-__global__ void __launch_bounds__(1024) k_scan_sums(uint32_t *__restrict__ tile_sum, SegDev sg) {
-  __shared__ uint32_t wsum[32];
-  __shared__ uint32_t carry;
-  const uint32_t st = blockIdx.x;
-  const uint32_t t0 = __ldg(sg.toff + st), tiles = __ldg(sg.toff + st + 1) - t0;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  for (uint32_t b0 = 0; b0 < tiles; b0 += 1024) {
-    const uint32_t i = b0 + threadIdx.x;
-    const uint32_t v = i < tiles ? tile_sum[t0 + i] : 0u;
-    uint32_t inc = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
-      if (lane >= o) inc += u;
-    }
-    if (lane == 31) wsum[wid] = inc;
-    __syncthreads();
-    if (wid == 0) {
-      uint32_t s = wsum[lane], si = s;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t u = __shfl_up_sync(0xffffffffu, si, o);
-        if (lane >= o) si += u;
+      for (uint32_t j = 1; j <= 8; ++j) {
+        const uint32_t x = E + j;
+        if (x <= to && x >= lo && x < hi) row[x - lo] = (at + i) | ((to - x) << 28);
       }
-      wsum[lane] = si - s;
     }
-    __syncthreads();
-    const uint32_t excl = carry + wsum[wid] + inc - v;
-    if (i < tiles) tile_sum[t0 + i] = excl;
-    __syncthreads();
-    if (threadIdx.x == 1023) carry = excl + v;
-    __syncthreads();
+    E = to;
   }
 }
 
-// exclusive prefix E(t) of stream st's accept counts, t in [0, R]
-struct SegView {
-  uint64_t r0;
-  uint32_t R, t0;
-};
-__device__ __forceinline__ SegView seg_view(const SegDev &sg, uint32_t st) {
-  SegView v;
-  v.r0 = __ldg(sg.roff + st);
-  v.R = (uint32_t)(__ldg(sg.roff + st + 1) - v.r0);
-  v.t0 = __ldg(sg.toff + st);
-  return v;
-}
-__device__ __forceinline__ uint32_t prefix_at(const uint32_t *elocal, const uint32_t *tile_off, const uint8_t *amask,
-                                              const SegView &v, uint32_t t) {
-  if (t < v.R) return elocal[v.r0 + t] + tile_off[v.t0 + t / kScanTile];
-  const uint32_t l = v.R - 1;
-  return elocal[v.r0 + l] + tile_off[v.t0 + l / kScanTile] + __popc(amask[v.r0 + l]);
-}
-
-// one warp per stream: call c starts at a fresh refill a_c; it ends at the first refill e
-// whose inclusive prefix reaches E(a_c) + n; a_{c+1} = e + 1.  call_start of stream st:
-// coff[st] + st .. coff[st+1] + st (calls + 1 entries; the last is the end of the last call).
-__global__ void k_walk(const uint32_t *__restrict__ elocal, const uint32_t *__restrict__ tile_off,
-                       const uint8_t *__restrict__ amask, SegDev sg, float mean_accept,
-                       uint32_t *__restrict__ call_start, uint32_t *__restrict__ status) {
-  const uint32_t st = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (st >= sg.nstreams) return;  // whole warps only
-  const SegView v = seg_view(sg, st);
-  const uint32_t n = __ldg(sg.n + st), calls = __ldg(sg.calls + st);
-  const uint32_t guess = (uint32_t)((float)n / mean_accept);
-  uint32_t *cs = call_start + __ldg(sg.coff + st) + st;
-  uint32_t a = 0;
-  bool bad = v.R == 0;
-  uint32_t c = 0;
-  // exclusive prefix at a, the start of the current call; afterwards it is carried over from
-  // the search, where the lane that found a call's last refill e has read prefix_at(e + 1)
-  uint32_t base = bad ? 0u : prefix_at(elocal, tile_off, amask, v, 0);
-  for (; c < calls && !bad; ++c) {
-    const uint32_t target = base + n;
-    // smallest e >= a whose inclusive prefix reaches target (monotone in e), searched in
-    // windows of 32 refills around the expected call length; `known` is a position already
-    // seen to satisfy (its prefix in known_pv).  Upward moves stop at the refill range,
-    // downward moves at a.
-    uint32_t lo = a + (guess > 16 ? guess - 16 : 0);
-    int64_t known = -1;
-    uint32_t known_pv = 0, e = 0, next_base = 0;
-    for (int it = 0;; ++it) {
-      if (it > (1 << 22)) {  // cannot happen for a monotone prefix; bounded regardless
-        bad = true;
-        break;
+// One CTA per stream follows the table.  Warp 0 makes the steps, about ten instructions each, since a warp
+// alone issues one in four or five cycles; the others copy the rows of 16 calls to shared memory three
+// groups of calls ahead, 128 entries each around the s that is expected there.  A group in which s
+// left a copied row is made again with reads of the table, and outside of the window by a search.
+constexpr uint32_t kChainRows = 16, kChainAhead = 4, kChainCols = 128;
+__global__ void __launch_bounds__(128)
+    k_chain(const uint8_t *__restrict__ amask, SegDev sg, EndTable t, uint32_t *__restrict__ call_start,
+            uint32_t *__restrict__ status) {
+  __shared__ __align__(16) uint32_t ring[kChainAhead][kChainRows][kChainCols];
+  __shared__ uint32_t low[kChainAhead][kChainRows];  // the s of a copied row's first entry
+  __shared__ uint32_t now;                           // s at the start of the walker's group
+  const uint32_t st = blockIdx.x, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint32_t n = seg_n(sg, st), calls = seg_calls(sg, st), groups = (calls + kChainRows - 1) / kChainRows;
+  const uint32_t *ends = t.ends + seg_coff(sg, st) * t.W;
+  // the copies of group g, from the overshoot s before call c
+  const auto copy = [&](uint32_t g, uint32_t s, uint32_t c) {
+    for (uint32_t i = warp - 1; i < kChainRows; i += 3) {
+      const uint32_t r = g * kChainRows + i;
+      if (r >= calls) break;
+      const uint32_t expect = s + (uint32_t)(((uint64_t)t.mean * (r - c)) >> 16), first = window_first(t, r);
+      const uint32_t from = min(expect > first + kChainCols / 2 ? (expect - first - kChainCols / 2) & ~3u : 0u, t.W - kChainCols);
+      const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&ring[g % kChainAhead][i][4 * lane]);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(ends + (size_t)r * t.W + from + 4 * lane)
+                   : "memory");
+      if (lane == 0) low[g % kChainAhead][i] = first + from;
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  if (threadIdx.x == 0) now = 0;
+  if (warp) {
+    for (uint32_t g = 0; g + 1 < kChainAhead; ++g) copy(g, 0, 0);
+    asm volatile("cp.async.wait_group %0;" ::"n"(kChainAhead - 2) : "memory");
+    __syncthreads();
+    for (uint32_t g = 0; g < groups; ++g) {
+      copy(g + kChainAhead - 1, now, g * kChainRows);
+      asm volatile("cp.async.wait_group %0;" ::"n"(kChainAhead - 2) : "memory");  // group g + 1 is there
+      __syncthreads();
+      if (__syncthreads_or(0)) break;
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    return;
+  }
+  const uint64_t r0 = seg_roff(sg, st);
+  const uint32_t R = (uint32_t)(seg_roff(sg, st + 1) - r0), tiles = (R + kCountTile - 1) / kCountTile;
+  const uint32_t *counts = t.counts + (size_t)st * t.max_tiles;
+  uint32_t *cs = call_start + seg_coff(sg, st) + st;
+  uint32_t total = 0;
+  for (uint32_t i = lane; i < tiles; i += 32) total += __ldg(counts + i);
+  total = __reduce_add_sync(0xffffffffu, total);
+  uint32_t s = 0, a = 0, c = 0;  // overshoot so far, start refill of call c
+  bool bad = false;
+  __syncthreads();
+  for (uint32_t g = 0; g < groups; ++g) {
+    const uint32_t rows = min(kChainRows, calls - c), s0 = s, a0 = a;
+    const uint32_t(*rg)[kChainCols] = ring[g % kChainAhead];
+    const uint32_t *lw = low[g % kChainAhead];
+    uint32_t worst = 0;
+    // every threshold of a whole group within the stream's count: the short steps
+    bool slow = rows < kChainRows || (uint64_t)(c + kChainRows) * n + s + 8 * kChainRows > total;
+    if (!slow) {
+#pragma unroll
+      for (uint32_t i = 0; i < kChainRows; ++i) {
+        const uint32_t in = s - lw[i];
+        worst = max(worst, in);
+        const uint32_t end = rg[i][min(in, kChainCols - 1)];
+        if (lane == 0) cs[c + i] = a;
+        a = (end & 0x0fffffffu) + 1u;
+        s += end >> 28;
       }
-      const uint32_t j = lo + lane;
-      const uint32_t pv = j < v.R ? prefix_at(elocal, tile_off, amask, v, j + 1) : 0u;
-      const bool ok = (j < v.R) && pv >= target;
-      const uint32_t bal = __ballot_sync(0xffffffffu, ok);
-      if (bal == 0) {
-        if (known >= 0) {
-          e = (uint32_t)known;
-          next_base = known_pv;
-          break;
-        }
-        if (lo + 32 >= v.R) {
+      slow = worst >= kChainCols;
+      if (!slow) c += kChainRows;
+    }
+    if (slow) {
+      s = s0;
+      a = a0;
+      for (uint32_t i = 0; i < rows; ++i) {
+        const uint32_t x = (c + 1) * n + s, col = s - window_first(t, c);
+        if (x > total) {  // the refill range was too short
           bad = true;
           break;
         }
-        lo += 32;
-        continue;
+        uint32_t end;
+        if (col < t.W) {
+          end = __ldg(ends + (size_t)c * t.W + col);
+        } else {  // the tile, then the refill that reaches the threshold
+          uint32_t E = 0, k = 0;
+          while (k + 1 < tiles && E + __ldg(counts + k) < x) E += __ldg(counts + k++);
+          for (uint32_t e = k * kCountTile;; e += 32) {  // total >= x: some refill below R reaches it
+            const uint32_t own = e + lane < R ? __popc((uint32_t)__ldg(amask + r0 + e + lane)) : 0u;
+            uint32_t inc = own;
+            for (int o = 1; o < 32; o <<= 1) {
+              const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
+              if (lane >= (uint32_t)o) inc += v;
+            }
+            const uint32_t hit = __ballot_sync(0xffffffffu, E + inc >= x);
+            if (hit || e >= R) {
+              const uint32_t f = hit ? (uint32_t)__ffs(hit) - 1u : 31u;
+              end = (e + f) | ((E + __shfl_sync(0xffffffffu, inc, f) - x) << 28);
+              break;
+            }
+            E += __shfl_sync(0xffffffffu, inc, 31);
+          }
+        }
+        if (lane == 0) cs[c] = a;
+        a = (end & 0x0fffffffu) + 1u;
+        s += end >> 28;
+        ++c;
       }
-      const int first = __ffs(bal) - 1;
-      const uint32_t first_pv = __shfl_sync(0xffffffffu, pv, first);
-      if (first > 0 || lo == a) {
-        e = lo + first;
-        next_base = first_pv;
-        break;
-      }
-      known = lo;
-      known_pv = first_pv;
-      lo = lo > a + 32 ? lo - 32 : a;
     }
-    if (bad) break;
-    if (lane == 0) cs[c] = a;
-    a = e + 1;
-    base = next_base;
+    __syncthreads();  // the copiers have read `now`
+    if (lane == 0) now = s;
+    if (__syncthreads_or(bad)) break;
   }
   if (lane == 0) {
     if (bad) atomicOr(status, kStatusRefillsExhausted);
-    for (uint32_t r = bad ? c : calls; r <= calls; ++r) cs[r] = bad ? v.R : a;
+    for (uint32_t i = c; i <= calls; ++i) cs[i] = bad ? R : a;
   }
 }
 
-// Pointer doubling for the call starts (the same result as k_walk).  next(t) of stream s is
-// the refill after a call that starts at refill t ends: e + 1 for the first e >= t whose
-// inclusive prefix reaches E(t) + n, or R + 1 (absorbing) when the stream runs out; the start
-// of call c is next applied c times to 0, assembled from the bits of c with the tables
-// J_k = next^(2^k).
-__global__ void k_next_start(const uint32_t *__restrict__ elocal, const uint32_t *__restrict__ tile_off,
-                             const uint8_t *__restrict__ amask, SegDev sg, float mean_accept,
-                             uint32_t *__restrict__ next) {
-  const uint64_t total = __ldg(sg.roff + sg.nstreams);
-  const uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= total) return;
-  const uint32_t st = seg_find(sg.roff, sg.nstreams, g);
-  const SegView v = seg_view(sg, st);
-  const uint32_t t = (uint32_t)(g - v.r0), n = __ldg(sg.n + st);
-  const uint32_t target = prefix_at(elocal, tile_off, amask, v, t) + n;
-  // smallest e in [t, R) with E(e + 1) >= target; try the expected call length first
-  uint32_t lo = t, hi = v.R;
-  const uint32_t guess = t + 2u * (uint32_t)((float)n / mean_accept) + 64u;
-  if (guess < v.R && prefix_at(elocal, tile_off, amask, v, guess + 1) >= target) hi = guess;
-  while (lo < hi) {
-    const uint32_t mid = lo + (hi - lo) / 2;
-    if (prefix_at(elocal, tile_off, amask, v, mid + 1) >= target) hi = mid;
-    else lo = mid + 1;
+// One CTA per stream, for runs of few calls or small n.
+//
+// The stream is serial in its calls, so one warp walks; the other eight stream the accept masks
+// ahead of it, 8,192 refills at a time, and leave in shared memory the count before every 16
+// refills and the counts within them.  A call then costs the walker one round of reads around its
+// expected end, a ballot and a shuffle, whatever n is, and no count goes through memory.  (Walked over
+// prefixes in global memory a call cost 0.85 us of dependent loads.)
+constexpr int kWalkTile = 8192, kWalkGroups = kWalkTile / 16;
+constexpr int kWalkThreads = 32 + 256;  // the walker, and 32 refills per thread
+__global__ void __launch_bounds__(kWalkThreads)
+    k_walk(const uint8_t *__restrict__ amask, SegDev sg, float mean_accept, uint32_t *__restrict__ call_start,
+           uint32_t *__restrict__ status) {
+  __shared__ uint32_t before[2][kWalkGroups + 1];         // E at the groups' starts and the tile's end
+  __shared__ __align__(16) uint8_t within[2][kWalkTile];  // inclusive count within the group (at most 128)
+  __shared__ uint32_t wsum[2][8];
+  const uint32_t st = blockIdx.x, lane = threadIdx.x & 31u;
+  const uint64_t r0 = seg_roff(sg, st);
+  const uint32_t R = (uint32_t)(seg_roff(sg, st + 1) - r0);  // a multiple of 32, as every r0
+  const uint32_t tiles = (R + kWalkTile - 1) / kWalkTile;
+  if (threadIdx.x >= 32) {
+    const uint32_t g = threadIdx.x - 32, warp = g >> 5;
+    const uint4 *src = reinterpret_cast<const uint4 *>(amask + r0) + 2 * g;
+    const auto load = [&](uint32_t tile, uint4 (&m)[2]) {
+      const bool in = tile * kWalkTile + 32 * g < R;
+      m[0] = in ? __ldg(src + (size_t)tile * kWalkGroups) : make_uint4(0, 0, 0, 0);
+      m[1] = in ? __ldg(src + (size_t)tile * kWalkGroups + 1) : make_uint4(0, 0, 0, 0);
+    };
+    // 16 masks to the inclusive counts up to each; returns the sum
+    const auto count = [](uint4 m, uint8_t *to) {
+      uint32_t w[4] = {m.x, m.y, m.z, m.w}, run = 0;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {  // bytes to their bit counts, then to the sums up to each byte
+        uint32_t v = w[i] - ((w[i] >> 1) & 0x55555555u);
+        v = (v & 0x33333333u) + ((v >> 2) & 0x33333333u);
+        v = (v + (v >> 4)) & 0x0f0f0f0fu;
+        w[i] = (v + run) * 0x01010101u;  // at most 128 each
+        run = w[i] >> 24;
+      }
+      *reinterpret_cast<uint4 *>(to) = make_uint4(w[0], w[1], w[2], w[3]);
+      return run;
+    };
+    uint32_t carry = 0;
+    uint4 m[2], m1[2];  // two tiles of loads in flight
+    load(0, m);
+    load(1, m1);
+    for (uint32_t k = 0; k <= tiles; ++k) {
+      if (k < tiles) {
+        const uint32_t buf = k & 1u;
+        const uint32_t c0 = count(m[0], &within[buf][32 * g]), c1 = count(m[1], &within[buf][32 * g + 16]);
+        m[0] = m1[0], m[1] = m1[1];
+        load(k + 2, m1);
+        uint32_t inc = c0 + c1;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
+          if (lane >= (uint32_t)o) inc += v;
+        }
+        if (lane == 31) wsum[buf][warp] = inc;
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        uint32_t base = carry;
+#pragma unroll
+        for (uint32_t i = 0; i < 8; ++i) {
+          const uint32_t v = wsum[buf][i];
+          if (i < warp) base += v;
+          carry += v;
+        }
+        before[buf][2 * g] = base + inc - c0 - c1;
+        before[buf][2 * g + 1] = base + inc - c1;
+        if (g == 255) before[buf][kWalkGroups] = carry;
+      }
+      if (__syncthreads_or(0)) return;  // the walker has every call
+    }
+    return;
   }
-  next[g] = lo < v.R ? lo + 1 : v.R + 1;
-}
-
-__global__ void k_next_square(const uint32_t *__restrict__ jin, uint32_t *__restrict__ jout, SegDev sg) {
-  const uint64_t total = __ldg(sg.roff + sg.nstreams);
-  const uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= total) return;
-  const uint32_t st = seg_find(sg.roff, sg.nstreams, g);
-  const uint64_t r0 = __ldg(sg.roff + st);
-  const uint32_t R = (uint32_t)(__ldg(sg.roff + st + 1) - r0);
-  const uint32_t a = jin[g];
-  jout[g] = a < R ? jin[r0 + a] : R + 1;
-}
-
-// one thread per (stream, c), c = 0 .. calls: call_start[coff[s] + s + c]
-__global__ void k_starts_from_tables(const uint32_t *__restrict__ tables, int levels, uint64_t refills, SegDev sg,
-                                     uint32_t *__restrict__ call_start, uint32_t *__restrict__ status) {
-  const uint64_t total = __ldg(sg.coff + sg.nstreams) + sg.nstreams;
-  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= total) return;
-  uint32_t lo = 0, hi = sg.nstreams;  // stream s owns entries [coff[s] + s, coff[s+1] + s + 1)
-  while (hi - lo > 1) {
-    const uint32_t mid = (lo + hi) >> 1;
-    if (__ldg(sg.coff + mid) + mid <= i) lo = mid;
-    else hi = mid;
+  const uint32_t n = seg_n(sg, st), calls = seg_calls(sg, st);
+  const uint32_t guess = (uint32_t)((float)n / mean_accept);
+  uint32_t *cs = call_start + seg_coff(sg, st) + st;
+  uint32_t a = 0, c = 0, target = n;  // start refill of call c, E(a) + n
+  if (lane == 0 && calls) cs[0] = 0;
+  __syncthreads_or(0);  // tile 0 is there
+  for (uint32_t k = 0; k < tiles; ++k) {
+    const uint32_t *bf = before[k & 1u];
+    const uint32_t *in = reinterpret_cast<const uint32_t *>(within[k & 1u]) + lane;
+    const uint32_t t0 = k * kWalkTile, tile_end = bf[kWalkGroups];
+    // 128 refills around refill a + span, four per lane
+    const auto window = [&](uint32_t span) {
+      const uint32_t at = a + span > t0 + 64 ? a + span - t0 - 64 : 0u;
+      return min(at & ~3u, (uint32_t)kWalkTile - 128);
+    };
+    const auto base = [&](uint32_t w) { return bf[((w >> 2) + lane) >> 2]; };
+    uint32_t w = window(guess), v = in[w >> 2], e = base(w);
+    while (c < calls && tile_end >= target) {
+      // the next call's window is read while this call is decided
+      const uint32_t w1 = window(2 * guess), v1 = in[w1 >> 2], e1 = base(w1);
+      uint32_t first, mine;
+      for (;;) {
+        const int32_t left = (int32_t)(target - e);
+        // refills of these four that do not reach the target, and how far the next one goes beyond it
+        const uint32_t cnt = (uint32_t)((int32_t)(v & 0xffu) < left) + (uint32_t)((int32_t)((v >> 8) & 0xffu) < left) +
+                             (uint32_t)((int32_t)((v >> 16) & 0xffu) < left) + (uint32_t)((int32_t)(v >> 24) < left);
+        const uint32_t hit = __ballot_sync(0xffffffffu, cnt < 4);
+        mine = cnt | ((uint32_t)((int32_t)((v >> (8 * (cnt & 3u))) & 0xffu) - left) << 2);
+        first = (uint32_t)__ffs(hit) - 1u;
+        mine = __shfl_sync(0xffffffffu, mine, first & 31u);
+        if (hit && (first | (mine & 3u) | (uint32_t)(w == 0))) break;
+        // outside of the window; reached in its first refill, the call may have ended before it
+        w = hit ? (w > 124 ? w - 124 : 0u) : min(w + 128, (uint32_t)kWalkTile - 128);
+        v = in[w >> 2];
+        e = base(w);
+      }
+      a = t0 + w + 4 * first + (mine & 3u) + 1u;
+      target += (mine >> 2) + n;
+      ++c;
+      if (lane == 0) cs[c] = a;
+      w = w1, v = v1, e = e1;
+    }
+    if (__syncthreads_or(c >= calls)) return;
   }
-  const uint32_t st = lo;
-  const uint32_t c = (uint32_t)(i - (__ldg(sg.coff + st) + st));
-  const uint64_t r0 = __ldg(sg.roff + st);
-  const uint32_t R = (uint32_t)(__ldg(sg.roff + st + 1) - r0);
-  uint32_t a = 0;
-  for (int k = 0; k < levels; ++k)
-    if ((c >> k) & 1u) a = a < R ? tables[(uint64_t)k * refills + r0 + a] : R + 1;
-  call_start[i] = a <= R ? a : R;
-  if (a > R && c == __ldg(sg.calls + st)) atomicOr(status, kStatusRefillsExhausted);
+  if (c < calls && lane == 0) {  // the refill range was too short
+    atomicOr(status, kStatusRefillsExhausted);
+    for (uint32_t i = c; i <= calls; ++i) cs[i] = R;
+  }
 }
 
 // ------------------------------------------------------------------ CPU mapping, phase 3
@@ -576,42 +677,48 @@ __device__ __forceinline__ uint32_t residue_parts(uint32_t lo, uint32_t hi, uint
 // t + 4k + L / 8 (eight coalesced 128-byte loads in flight per warp).  Per k the warp ballots the accepted lanes and packs
 // them, in refill order and then candidate order (the order the reference consumes them), into
 // a per-warp staging array; then every lane reduces one staged sample and the warp writes
-// consecutive output positions.  Only the first position of each warp's run comes from the
-// prefix tables.
+// consecutive output positions.  The first position of a warp's run is the accept count of the
+// runs before it, which the warps count first.
 constexpr int kScatterThreads = 256;
 __global__ void __launch_bounds__(kScatterThreads)
     k_scatter(const uint32_t *__restrict__ cand_lo, const uint8_t *__restrict__ amask,
-              const uint16_t *__restrict__ chs, const uint32_t *__restrict__ elocal,
-              const uint32_t *__restrict__ tile_off, const uint32_t *__restrict__ call_start, SegDev sg, ModArgs m,
+              const uint16_t *__restrict__ chs, const uint32_t *__restrict__ call_start, SegDev sg, ModArgs m,
               uint32_t *__restrict__ out) {
   __shared__ uint2 stage[kScatterThreads / 32][256];
-  const uint32_t st = seg_find(sg.coff, sg.nstreams, blockIdx.x);
-  const uint64_t cs0 = __ldg(sg.coff + st);
-  const uint32_t c = (uint32_t)(blockIdx.x - cs0);
-  const SegView v = seg_view(sg, st);
-  const uint32_t n = __ldg(sg.n + st);
+  __shared__ uint32_t counts[kScatterThreads / 32];
+  const uint32_t st = seg_of_call(sg, blockIdx.x);
+  const uint64_t cs0 = seg_coff(sg, st), r0 = seg_roff(sg, st);
+  const uint32_t c = (uint32_t)(blockIdx.x - cs0), R = (uint32_t)(seg_roff(sg, st + 1) - r0);
+  const uint32_t n = seg_n(sg, st);
   const uint32_t *cs = call_start + cs0 + st;
-  const uint32_t a = cs[c], b = min(cs[c + 1], v.R);
+  const uint32_t a = cs[c], b = min(cs[c + 1], R);
   if (a >= b) return;
-  const uint32_t lane = threadIdx.x & 31u, nw = blockDim.x >> 5;
+  constexpr uint32_t nw = kScatterThreads / 32;
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint32_t span = ((b - a + nw - 1) / nw + 3u) & ~3u;  // refills per warp
-  const uint32_t t0 = a + (threadIdx.x >> 5) * span;
-  if (t0 >= b) return;  // whole warps leave together; no CTA barrier follows
-  const uint32_t t1 = min(t0 + span, b);
-  uint32_t pos = prefix_at(elocal, tile_off, amask, v, t0) - prefix_at(elocal, tile_off, amask, v, a);
-  uint32_t *o = out + __ldg(sg.ooff + st) + (size_t)c * 3 * n;
-  uint2 *sw = stage[threadIdx.x >> 5];
+  const uint32_t t0 = min(a + warp * span, b), t1 = min(t0 + span, b);
+  uint32_t mine = 0;
+#pragma unroll 4
+  for (uint32_t t = t0 + lane; t < t1; t += 32) mine += __popc((uint32_t)__ldg(amask + r0 + t));
+  mine = __reduce_add_sync(0xffffffffu, mine);
+  if (lane == 0) counts[warp] = mine;
+  __syncthreads();
+  uint32_t pos = 0;
+#pragma unroll
+  for (uint32_t i = 0; i < nw; ++i) pos += i < warp ? counts[i] : 0u;
+  uint32_t *o = out + seg_ooff(sg, st) + (size_t)c * 3 * n;
+  uint2 *sw = stage[warp];
   const uint32_t below = (1u << lane) - 1u, ci = lane & 7u;
   for (uint32_t t = t0; t < t1 && pos < n; t += 32) {
     // refill t + lane: accept bits, bit 32 of each |value| (<< 8), signs (<< 16)
-    const uint32_t mk = t + lane < t1 ? (uint32_t)__ldg(amask + v.r0 + t + lane) |
-                                            ((uint32_t)__ldg(chs + v.r0 + t + lane) << 8)
+    const uint32_t mk = t + lane < t1 ? (uint32_t)__ldg(amask + r0 + t + lane) |
+                                            ((uint32_t)__ldg(chs + r0 + t + lane) << 8)
                                       : 0u;
     uint32_t lv[8];
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
       const uint32_t r = t + 4 * k + (lane >> 3);
-      lv[k] = r < t1 ? __ldg(cand_lo + (v.r0 + r) * 8 + ci) : 0u;
+      lv[k] = r < t1 ? __ldg(cand_lo + (r0 + r) * 8 + ci) : 0u;
     }
     uint32_t cnt = 0;
 #pragma unroll
@@ -631,24 +738,6 @@ __global__ void __launch_bounds__(kScatterThreads)
     }
     __syncwarp();  // the next step overwrites the staging array
     pos += cnt;
-  }
-}
-
-// segment table of nstreams equal streams (calls x n each, refills R each, output stride
-// `ostride` words per stream)
-__global__ void k_seg_uniform(uint32_t nstreams, uint32_t calls, uint32_t n, uint32_t R, uint32_t tiles,
-                              uint64_t ostride, uint32_t *__restrict__ sn, uint32_t *__restrict__ scalls,
-                              uint64_t *__restrict__ roff, uint32_t *__restrict__ toff, uint64_t *__restrict__ coff,
-                              uint64_t *__restrict__ ooff) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i > nstreams) return;
-  roff[i] = (uint64_t)i * R;
-  toff[i] = i * tiles;
-  coff[i] = (uint64_t)i * calls;
-  if (i < nstreams) {
-    sn[i] = n;
-    scalls[i] = calls;
-    ooff[i] = (uint64_t)i * ostride;
   }
 }
 
@@ -996,6 +1085,9 @@ int sampler_init_device() {
 // K).  The means below are those rounded down, the variance bound is 2.0 for all three.
 static double mean_accept(int sig) { return sig == 0 ? 5.443 : (sig == 1 ? 4.393 : 3.094); }
 constexpr double kAcceptVarBound = 2.0;
+// Mean samples by which a call overshoots its n, with 16 fractional bits: (E[X^2] / E[X] - 1) / 2 for
+// the accept count X of a refill with the moments above: 2.38, 1.92 and 1.35.
+static uint32_t mean_overshoot(int sig) { return sig == 0 ? 156100u : (sig == 1 ? 126000u : 88500u); }
 
 // Refills precomputed for `calls` consecutive calls of n samples.  A call consumes r refills,
 // the first whose accepted total reaches n; E[r] = (n + overshoot) / mu < n / mu + 1 (the
@@ -1024,8 +1116,6 @@ SegLayout seg_layout(uint32_t S) {
   o += align256((size_t)S * 4);
   L.calls = o;
   o += align256((size_t)S * 4);
-  L.toff = o;
-  o += align256((size_t)(S + 1) * 4);
   L.roff = o;
   o += align256((size_t)(S + 1) * 8);
   L.coff = o;
@@ -1039,11 +1129,10 @@ SegLayout seg_layout(uint32_t S) {
 SegDev seg_bind(void *base, uint32_t S) {
   const SegLayout L = seg_layout(S);
   uint8_t *b = static_cast<uint8_t *>(base);
-  SegDev d;
+  SegDev d{};
   d.nstreams = S;
   d.n = reinterpret_cast<const uint32_t *>(b + L.n);
   d.calls = reinterpret_cast<const uint32_t *>(b + L.calls);
-  d.toff = reinterpret_cast<const uint32_t *>(b + L.toff);
   d.roff = reinterpret_cast<const uint64_t *>(b + L.roff);
   d.coff = reinterpret_cast<const uint64_t *>(b + L.coff);
   d.ooff = reinterpret_cast<const uint64_t *>(b + L.ooff);
@@ -1055,73 +1144,59 @@ SegSizes seg_fill_host(int sig, uint32_t S, const uint32_t *calls, const uint32_
   const SegLayout L = seg_layout(S);
   uint8_t *b = static_cast<uint8_t *>(host_base);
   uint32_t *hn = reinterpret_cast<uint32_t *>(b + L.n), *hc = reinterpret_cast<uint32_t *>(b + L.calls);
-  uint32_t *ht = reinterpret_cast<uint32_t *>(b + L.toff);
   uint64_t *hr = reinterpret_cast<uint64_t *>(b + L.roff), *hco = reinterpret_cast<uint64_t *>(b + L.coff);
   uint64_t *ho = reinterpret_cast<uint64_t *>(b + L.ooff);
-  SegSizes z{S, 0, 0, 0, 0, false};
+  SegSizes z{S, 0, 0, 0, 0, 0xffffffffu};
   for (uint32_t i = 0; i < S; ++i) {
     const uint32_t R = cpu_map_refills(calls[i], n[i], sig);
     hn[i] = n[i];
     hc[i] = calls[i];
     ho[i] = ooff ? ooff[i] : 0;
     hr[i] = z.refills;
-    ht[i] = z.tiles;
     hco[i] = z.calls;
     z.refills += R;
-    z.tiles += (R + kScanTile - 1) / kScanTile;
-    z.calls += calls[i];
+    z.max_refills = std::max(z.max_refills, R);
     z.max_calls = std::max(z.max_calls, calls[i]);
+    z.min_n = std::min(z.min_n, n[i]);
+    z.calls += calls[i];
   }
   hr[S] = z.refills;
-  ht[S] = z.tiles;
   hco[S] = z.calls;
-  z.doubling = seg_auto_doubling(z.refills, z.max_calls);
   return z;
 }
 
 static SegSizes seg_uniform_sizes(uint32_t S, uint32_t calls, uint32_t n, int sig) {
   const uint32_t R = cpu_map_refills(calls, n, sig);
-  return SegSizes{S, (uint64_t)S * R, S * ((R + kScanTile - 1) / kScanTile), (uint64_t)S * calls, calls,
-                  seg_auto_doubling((uint64_t)S * R, calls)};
+  return SegSizes{S, (uint64_t)S * R, (uint64_t)S * calls, R, calls, n};
 }
 
-static int g_call_search = 0;
-void set_call_search(int mode) { g_call_search = mode; }
-int get_call_search() { return g_call_search; }
-
-constexpr uint64_t kDoublingMaxRefills = (uint64_t)32 << 20;
-
-static int doubling_levels(uint32_t max_calls) {
-  int k = 1;
-  while (k < 31 && (1u << k) <= max_calls) ++k;
-  return k;  // bit_length(max_calls), at least 1
+// Width of the table of call ends, 0: k_walk.  The overshoot of a call has a standard deviation
+// below 2, so that of c calls one below 2 sqrt(c): the window takes 4 of those and 64 to either side.  The
+// windows may be n / 2 - 128 wide, so that a threshold is in one of them, and the nearest call to
+// any of a thread's 128 thresholds is the one whose window it is in (k_ends).  From 128 calls on the
+// three launches are shorter than the walk (sigma_2, n = 4096, one stream / 16, us against the
+// walk's: 64 calls 22 / 25 against 19 / 19, 128 27 / 32 against 31 / 31, 256 35 / 51 against 56 / 57, 785
+// 72 / 114 against 158 / 158).
+static uint32_t end_table_width(const SegSizes &z) {
+  const uint32_t W = ((uint32_t)(16.0 * std::sqrt((double)z.max_calls)) + 128 + 63) & ~63u;
+  return z.max_calls >= 128 && 2 * (W + 128) <= z.min_n && z.max_refills < (1u << 28) && z.nstreams < 65536u ? W : 0u;
 }
-// Doubling costs about 6.4 ps per refill per table level (memory-bound gathers); the walk
-// about 1.0-1.4 us per call of its longest stream (serial dependent loads), both measured on
-// a B200 (sigma_3 at n = 4096, l = 784: doubling 0.48 / 1.12 ms at 8 / 16 encryptions, walk
-// 0.78 ms up to 16 and 1.13 ms from 24).  Doubling is chosen when it is the cheaper of the two
-// and its tables stay below 32 Mi refills.
-bool seg_auto_doubling(uint64_t refills, uint32_t max_calls) {
-  if (g_call_search == 1 || refills > kDoublingMaxRefills) return false;
-  if (g_call_search == 2) return true;
-  return refills * (uint64_t)doubling_levels(max_calls) <= (uint64_t)max_calls * 200000u;
-}
+
+static uint32_t count_tiles(const SegSizes &z) { return (z.max_refills + kCountTile - 1) / kCountTile; }
 
 size_t seg_scratch_bytes(const SegSizes &z) {
-  size_t b = align256(z.refills * 32) + align256(z.refills) + align256(z.refills * 2) + align256(z.refills * 4) +
-             align256((size_t)z.tiles * 4) +
-             align256((z.calls + z.nstreams) * 4);
-  if (z.doubling) b += (size_t)doubling_levels(z.max_calls) * align256(z.refills * 4);
-  return b;
+  return align256(z.refills * 32) + align256(z.refills) + align256(z.refills * 2) +
+         align256((z.calls + z.nstreams) * 4) + align256((size_t)z.calls * end_table_width(z) * 4) +
+         align256((size_t)z.nstreams * count_tiles(z) * 4);
 }
 
 size_t cpu_map_workspace_bytes(uint32_t nstreams, uint32_t calls, uint32_t n, int sig) {
-  return seg_layout(nstreams).bytes + seg_scratch_bytes(seg_uniform_sizes(nstreams, calls, n, sig));
+  return seg_scratch_bytes(seg_uniform_sizes(nstreams, calls, n, sig));
 }
 
 int sample_cpu_map_seg(int sig, const SegDev &sg, const SegSizes &z, const uint32_t *d_rkeys, uint32_t *d_out,
                        void *scratch, uint32_t *d_status, int num_sms, cudaStream_t s) {
-  if (sig < 0 || sig > 2 || z.nstreams == 0 || z.tiles >= (1u << 31) || z.calls >= (1ull << 31) ||
+  if (sig < 0 || sig > 2 || z.nstreams == 0 || z.calls >= (1ull << 31) ||
       z.refills >= (1ull << 32) - (1ull << 24))
     return CUFE_ERR_INVALID;
   uint8_t *p = static_cast<uint8_t *>(scratch);
@@ -1133,8 +1208,6 @@ int sample_cpu_map_seg(int sig, const SegDev &sg, const SegSizes &z, const uint3
   uint32_t *cand = reinterpret_cast<uint32_t *>(take(z.refills * 32));  // low words of |candidate|
   uint8_t *amask = take(z.refills);
   uint16_t *chs = reinterpret_cast<uint16_t *>(take(z.refills * 2));  // bit 32 of each, signs << 8
-  uint32_t *elocal = reinterpret_cast<uint32_t *>(take(z.refills * 4));
-  uint32_t *tsum = reinterpret_cast<uint32_t *>(take((size_t)z.tiles * 4));
   uint32_t *cstart = reinterpret_cast<uint32_t *>(take((z.calls + z.nstreams) * 4));
   const double kinv = kinv_of(sig);
   const uint32_t grid =
@@ -1152,62 +1225,46 @@ int sample_cpu_map_seg(int sig, const SegDev &sg, const SegSizes &z, const uint3
                                                                              d_status);
   }
   CUFE_CUDA(cudaGetLastError());
-  if (z.tiles) {
-    ProfScope ps("sample_scan", s);
-    note_launch(), k_scan_tiles<<<z.tiles, 512, 0, s>>>(amask, sg, elocal, tsum);
-    note_launch(), k_scan_sums<<<z.nstreams, 1024, 0, s>>>(tsum, sg);
-  }
-  if (z.doubling) {
-    const int levels = doubling_levels(z.max_calls);
-    uint32_t *tab = reinterpret_cast<uint32_t *>(take((size_t)levels * align256(z.refills * 4)));
-    const uint64_t stride = align256(z.refills * 4) / 4;
+  {
     ProfScope ps("sample_walk", s);
-    const unsigned rg = (unsigned)((z.refills + 255) / 256);
-    note_launch(), k_next_start<<<rg, 256, 0, s>>>(elocal, tsum, amask, sg, (float)mean_accept(sig), tab);
-    for (int k = 1; k < levels; ++k) note_launch(), k_next_square<<<rg, 256, 0, s>>>(tab + (k - 1) * stride, tab + k * stride, sg);
-    note_launch(), k_starts_from_tables<<<(unsigned)((z.calls + z.nstreams + 255) / 256), 256, 0, s>>>(tab, levels, stride, sg,
-                                                                                        cstart, d_status);
-  } else {
-    ProfScope ps("sample_walk", s);
-    note_launch(), k_walk<<<(z.nstreams + 3) / 4, 128, 0, s>>>(elocal, tsum, amask, sg, (float)mean_accept(sig), cstart, d_status);
+    const uint32_t W = end_table_width(z);
+    if (W) {
+      EndTable t;
+      t.ends = reinterpret_cast<uint32_t *>(take((size_t)z.calls * W * 4));
+      t.max_tiles = count_tiles(z);
+      t.counts = reinterpret_cast<uint32_t *>(take((size_t)z.nstreams * t.max_tiles * 4));
+      t.W = W;
+      t.mean = mean_overshoot(sig);
+      const dim3 grid(t.max_tiles, z.nstreams);
+      note_launch(), k_tile_counts<<<grid, 256, 0, s>>>(amask, sg, t);
+      note_launch(), k_ends<<<grid, 256, 0, s>>>(amask, sg, t);
+      note_launch(), k_chain<<<z.nstreams, 128, 0, s>>>(amask, sg, t, cstart, d_status);
+    } else {
+      note_launch(), k_walk<<<z.nstreams, kWalkThreads, 0, s>>>(amask, sg, (float)mean_accept(sig), cstart, d_status);
+    }
+    CUFE_CUDA(cudaGetLastError());
   }
-  CUFE_CUDA(cudaGetLastError());
   if (d_out && z.calls) {
     ProfScope ps_sc("sample_scatter", s);
-    note_launch(), k_scatter<<<(uint32_t)z.calls, kScatterThreads, 0, s>>>(cand, amask, chs, elocal, tsum, cstart, sg,
-                                                                           mod_args(), d_out);
+    note_launch(), k_scatter<<<(uint32_t)z.calls, kScatterThreads, 0, s>>>(cand, amask, chs, cstart, sg, mod_args(),
+                                                                           d_out);
     CUFE_CUDA(cudaGetLastError());
   }
   return CUFE_OK;
 }
 
-// the uniform case: nstreams equal streams, tables built on the device (capturable)
-static int seg_uniform(uint32_t nstreams, uint32_t calls, uint32_t n, int sig, void *ws, cudaStream_t s, SegDev *sg,
-                       SegSizes *z, void **scratch) {
-  const SegLayout L = seg_layout(nstreams);
-  *z = seg_uniform_sizes(nstreams, calls, n, sig);
-  if (z->refills / nstreams >= (1ull << 32) / 24) return CUFE_ERR_INVALID;  // AES counter range
-  uint8_t *b = static_cast<uint8_t *>(ws);
-  *sg = seg_bind(b, nstreams);
-  const uint32_t R = (uint32_t)(z->refills / nstreams);
-  note_launch(), k_seg_uniform<<<(nstreams + 256) / 256, 256, 0, s>>>(
-      nstreams, calls, n, R, z->tiles / nstreams, (uint64_t)calls * 3 * n, reinterpret_cast<uint32_t *>(b + L.n),
-      reinterpret_cast<uint32_t *>(b + L.calls), reinterpret_cast<uint64_t *>(b + L.roff),
-      reinterpret_cast<uint32_t *>(b + L.toff), reinterpret_cast<uint64_t *>(b + L.coff),
-      reinterpret_cast<uint64_t *>(b + L.ooff));
-  CUFE_CUDA(cudaGetLastError());
-  *scratch = b + L.bytes;
-  return CUFE_OK;
-}
-
+// the uniform case: nstreams equal streams, no tables
 int sample_cpu_map(int sig, uint32_t nstreams, const uint32_t *d_rkeys, uint32_t calls, uint32_t n,
                    uint32_t *d_out, void *ws, uint32_t *d_status, int num_sms, cudaStream_t s) {
-  SegDev sg;
-  SegSizes z;
-  void *scratch;
-  int rc = seg_uniform(nstreams, calls, n, sig, ws, s, &sg, &z, &scratch);
-  if (rc) return rc;
-  return sample_cpu_map_seg(sig, sg, z, d_rkeys, d_out, scratch, d_status, num_sms, s);
+  const SegSizes z = seg_uniform_sizes(nstreams, calls, n, sig);
+  if (z.refills / nstreams >= (1ull << 32) / 24) return CUFE_ERR_INVALID;  // AES counter range
+  SegDev sg{};
+  sg.nstreams = nstreams;
+  sg.u_n = n;
+  sg.u_calls = calls;
+  sg.u_refills = (uint32_t)(z.refills / nstreams);
+  sg.u_ostride = (uint64_t)calls * 3 * n;
+  return sample_cpu_map_seg(sig, sg, z, d_rkeys, d_out, ws, d_status, num_sms, s);
 }
 
 int sample_gpu_map(int sig, const uint32_t *d_rkey, uint32_t poly0, uint32_t npolys, uint32_t n, uint32_t *d_out,

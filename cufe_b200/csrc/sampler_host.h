@@ -29,33 +29,25 @@ int sample_cpu_map(int sig, uint32_t nstreams, const uint32_t *d_rkeys, uint32_t
 
 // Segmented form: S CPU-mapping streams of different lengths.  Stream s runs calls[s]
 // sampler calls of n[s] samples; its refills occupy [roff[s], roff[s+1]) of the flattened
-// refill space, its scan tiles [toff[s], toff[s+1]), its call starts
-// call_start[coff[s] + s .. coff[s+1] + s] (calls + 1 entries), and the scatter writes its
-// residues to out[ooff[s] + c * 3 n[s] ...][3][n[s]].  Round keys rkeys[s][60].
+// refill space (multiples of 32), its call starts call_start[coff[s] + s .. coff[s+1] + s] (calls + 1
+// entries), and the scatter writes its residues to out[ooff[s] + c * 3 n[s] ...][3][n[s]].  Round
+// keys rkeys[s][60].  Without tables (n == nullptr) the streams are equal: u_calls calls of u_n
+// samples, u_refills refills, u_ostride words of output each.
 struct SegDev {
   uint32_t nstreams;
-  const uint32_t *n, *calls, *toff;
+  const uint32_t *n, *calls;
   const uint64_t *roff, *coff, *ooff;
+  uint32_t u_n, u_calls, u_refills;
+  uint64_t u_ostride;
 };
 struct SegSizes {
   uint32_t nstreams;
   uint64_t refills;
-  uint32_t tiles;
   uint64_t calls;
-  uint32_t max_calls;  // the largest calls[s]
-  bool doubling;       // call starts by pointer doubling (its tables are part of the scratch)
+  uint32_t max_refills, max_calls, min_n;  // over the streams
 };
-// How the call starts of the CPU mapping are found.  Pointer doubling is parallel over
-// refills and calls but costs bit_length(max_calls) table passes over all refills (and as
-// many words of scratch per refill); the serial walk (one warp per stream) costs a dependent
-// search per call.  Doubling is chosen when it is estimated cheaper and stays below 32 Mi
-// refills; set_call_search(1) forces the walk.  The choice is fixed in SegSizes when a
-// scratch is sized.
-void set_call_search(int mode);
-int get_call_search();
-bool seg_auto_doubling(uint64_t refills, uint32_t max_calls);
 struct SegLayout {
-  size_t n, calls, toff, roff, coff, ooff, bytes;
+  size_t n, calls, roff, coff, ooff, bytes;
 };
 // the tables of S streams in one buffer (device or host, same layout)
 SegLayout seg_layout(uint32_t S);

@@ -182,12 +182,9 @@ int cufe_sample_gpu_map(cufe_ctx *ctx, int sig, const uint8_t key[32], int poly0
 /* sample_polya (src/sample.c:56-128): d_a[3][n] */
 int cufe_sample_polya(cufe_ctx *ctx, const uint8_t seed[32], uint32_t *d_a, void *stream);
 
-/* How the CPU-mapping samplers find where each gaussian_sampler_S* call starts (process-wide;
- * all give the same samples): 0 (default) the cheaper of pointer doubling (parallel over
- * refills, log2(calls) table levels; runs up to 32 Mi refills) and the serial one-warp walk
- * (dependent loads per call of the longest stream), by a cost model measured on a B200;
- * 1 always the walk; 2 doubling whenever the run is within 32 Mi refills.  Applies to
- * workspaces sized after the call. */
+/* The CPU-mapping samplers find where each gaussian_sampler_S* call starts by a streamed walk, or
+ * by a table of call ends in long runs.  Modes 0, 1 and 2, which chose between a walk and pointer
+ * doubling, are accepted and make no difference; others are refused. */
 int cufe_sampler_call_search(int mode);
 
 /* Serialized keys and ciphertexts: a 32-byte header (magic "CUFE", version 1, kind, n, l,
