@@ -120,8 +120,8 @@ __global__ void __launch_bounds__(512)
   uint32_t *sm = smem_u32 + threadIdx.y * P::SMEM_WORDS;
   uint32_t a[16], w[16], wsh[16];
   load16(keys + I.mpk + (size_t)local * P::N + th * 16, a);
-  load16(rh + I.rh + (size_t)m * P::N + th * 16, w);
-  load16(rh_sh + I.rh + (size_t)m * P::N + th * 16, wsh);
+  load16_own(rh + I.rh + (size_t)m * P::N + th * 16, w);
+  load16_own(rh_sh + I.rh + (size_t)m * P::N + th * 16, wsh);
 #pragma unroll
   for (int e = 0; e < 16; ++e) a[e] = shoup_mul(a[e], w[e], wsh[e], q);
   ntt_inv_core<LOGN>(a, sm, th, q, ra.ipsi2 + (size_t)m * P::N, ra.ninv[m], ra.ninv_sh[m], ra.w1n[m],

@@ -20,7 +20,7 @@ struct Ring {
   int device = 0, n = 0, logn = 0, k = 0;
   std::vector<uint32_t> q, psi_root;       // primes and the primitive 2n-th roots used
   std::vector<uint32_t> h_psi, h_ipsi;     // host copies [k][n] (bit-reversed powers)
-  uint32_t *d_tab = nullptr;               // psi2, ipsi2: 2 x [k][n] (w, w_shoup) pairs
+  uint32_t *d_tab = nullptr;               // psi2, ipsi2, both in plain order: 4 x [k][n] (w, w_shoup) pairs
   RingArgs args{};
   int init(int n, int k, const uint32_t *primes, int device);
   void release();

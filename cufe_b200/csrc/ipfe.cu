@@ -121,7 +121,7 @@ int Ring::init(int n_, int k_, const uint32_t *primes, int dev) {
   q = primes ? std::vector<uint32_t>(primes, primes + k) : ntt_primes(k);
   for (uint32_t qq : q)
     if (qq >= (1u << 31) || (qq - 1) % (2u * n) != 0 || !is_prime32(qq)) return CUFE_ERR_INVALID;
-  std::vector<uint32_t> tab(4 * (size_t)k * n);
+  std::vector<uint32_t> tab(8 * (size_t)k * n);
   h_psi.assign((size_t)k * n, 0);
   h_ipsi.assign((size_t)k * n, 0);
   psi_root.assign(k, 0);
@@ -136,11 +136,20 @@ int Ring::init(int n_, int k_, const uint32_t *primes, int dev) {
       const uint32_t a = (uint32_t)pw[bitrev(i, logn)], b = (uint32_t)ipw[bitrev(i, logn)];
       h_psi[(size_t)m * n + i] = a;
       h_ipsi[(size_t)m * n + i] = b;
-      // interleaved (w, floor(w 2^32 / q)) pairs: psi2[k][n], then ipsi2[k][n]
-      tab[2 * ((size_t)m * n + i)] = a;
-      tab[2 * ((size_t)m * n + i) + 1] = shoup_of(a, (uint32_t)qq);
-      tab[2 * ((size_t)(k + m) * n + i)] = b;
-      tab[2 * ((size_t)(k + m) * n + i) + 1] = shoup_of(b, (uint32_t)qq);
+      // interleaved (w, floor(w 2^32 / q)) pairs: psi2[k][n], then ipsi2[k][n], then both in plain order
+      int at = i;
+      if (i >= n / 2) {
+        const int th = (i - n / 2) >> 3, g = i & 7;
+        at = n / 2 + (((g >> 2) * (n / 16) + th) << 2) + (g & 3);
+      }
+      const uint32_t a_sh = shoup_of(a, (uint32_t)qq), b_sh = shoup_of(b, (uint32_t)qq);
+      for (int flat = 0; flat < 2; ++flat) {
+        uint32_t *f = &tab[2 * (((size_t)2 * flat * k + m) * n + (flat ? i : at))];
+        f[0] = a;
+        f[1] = a_sh;
+        f[2 * (size_t)k * n] = b;
+        f[2 * (size_t)k * n + 1] = b_sh;
+      }
     }
     args.q[m] = (uint32_t)qq;
     args.ninv[m] = (uint32_t)invmod(n, qq);
@@ -159,7 +168,9 @@ int Ring::init(int n_, int k_, const uint32_t *primes, int dev) {
   CUFE_CUDA(cudaMalloc(&d_tab, tab.size() * 4));
   CUFE_CUDA(cudaMemcpy(d_tab, tab.data(), tab.size() * 4, cudaMemcpyHostToDevice));
   args.psi2 = reinterpret_cast<const uint2 *>(d_tab);
-  args.ipsi2 = reinterpret_cast<const uint2 *>(d_tab) + (size_t)k * n;
+  args.ipsi2 = args.psi2 + (size_t)k * n;
+  args.psi2_flat = args.psi2 + (size_t)2 * k * n;
+  args.ipsi2_flat = args.psi2 + (size_t)3 * k * n;
   return CUFE_OK;
 }
 
@@ -218,7 +229,7 @@ __global__ void __launch_bounds__(LBT, MINB)
 #pragma unroll
       for (int e = 0; e < E; ++e) a[p][e] = d[P::template idx<0>(th, e)];
     }
-    ntt_fwd_core<LOGN, PP, LE, SQ>(a, sm, th, q, ra.psi2 + (size_t)m * P::N, ra.qr[m]);
+    ntt_fwd_core<LOGN, PP, LE, SQ>(a, sm, th, q, (LE == 4 ? ra.psi2 : ra.psi2_flat) + (size_t)m * P::N, ra.qr[m]);
 #pragma unroll
     for (int p = 0; p < PP; ++p) {
       if (!live[p]) continue;
@@ -233,7 +244,7 @@ __global__ void __launch_bounds__(LBT, MINB)
   } else {
 #pragma unroll
     for (int p = 0; p < PP; ++p) load_vec(data + res[p] * P::N + th * E, a[p]);
-    ntt_inv_core<LOGN, PP, LE, SQ>(a, sm, th, q, ra.ipsi2 + (size_t)m * P::N, ra.ninv[m], ra.ninv_sh[m],
+    ntt_inv_core<LOGN, PP, LE, SQ>(a, sm, th, q, (LE == 4 ? ra.ipsi2 : ra.ipsi2_flat) + (size_t)m * P::N, ra.ninv[m], ra.ninv_sh[m],
                                    ra.w1n[m], ra.w1n_sh[m]);
 #pragma unroll
     for (int p = 0; p < PP; ++p) {
@@ -445,8 +456,8 @@ __global__ void __launch_bounds__(512) k_setup_mpk(const uint32_t *__restrict__ 
   ntt_fwd_core<LOGN>(a, sm, th, q, ra.psi2 + (size_t)m * P::N);
   uint32_t w[16], wsh[16], ev[16];
   load16(ahat + (size_t)m * P::N + th * 16, w);
-  load16(ahat_sh + (size_t)m * P::N + th * 16, wsh);
-  load16(ehat + rr * P::N + th * 16, ev);
+  load16_own(ahat_sh + (size_t)m * P::N + th * 16, wsh);
+  load16_own(ehat + rr * P::N + th * 16, ev);
 #pragma unroll
   for (int e = 0; e < 16; ++e) a[e] = mod_add(shoup_mul(a[e], w[e], wsh[e], q), ev[e], q);
   if (act) store16(mpk + rr * P::N + th * 16, a);
@@ -484,8 +495,8 @@ __global__ void __launch_bounds__(NttPlan<LOGN>::T * ppc<LOGN>(), MINB)
     for (int p = 0; p < PP; ++p) {
       const int b = min(b0 + p, batch - 1);  // a dead slot repeats the last instance, stores nothing
       uint32_t w[16], wsh[16];
-      load16(rhat + b * rhat_stride + (size_t)m * P::N + th * 16, w);
-      load16(rhat_sh + b * rhat_stride + (size_t)m * P::N + th * 16, wsh);
+      load16_own(rhat + b * rhat_stride + (size_t)m * P::N + th * 16, w);
+      load16_own(rhat_sh + b * rhat_stride + (size_t)m * P::N + th * 16, wsh);
 #pragma unroll
       for (int e = 0; e < 16; ++e) a[p][e] = shoup_mul(pk[e], w[e], wsh[e], q);
     }
@@ -519,9 +530,10 @@ __global__ void __launch_bounds__(NttPlan<LOGN>::T * ppc<LOGN>(), MINB)
 // src/rlwe_sife_gpu.cu:102-188): the instances differ in floor(q/p) x_i only, so INTT(pk_r * r^) + f is
 // computed once per residue and written `batch` times with another constant added; CTAs of
 // blockIdx.y take a share of the instances each.  Bound by the ciphertexts' writes.  8 instances at
-// n = 4096, l = 785 on a B200: 274 us with an inverse transform per instance, now 80.
+// n = 4096, l = 785 on a B200: 274 us with an inverse transform per instance, now 77.  (48 registers:
+// at 63 a fifth of the CTAs is lost and it took 103.)
 template <int LOGN>
-__global__ void __launch_bounds__(NttPlan<LOGN>::T * ppc<LOGN>())
+__global__ void __launch_bounds__(NttPlan<LOGN>::T * ppc<LOGN>(), NttPlan<LOGN>::T > 256 ? 2 : 5)
     k_encrypt_shared(const uint32_t *__restrict__ mpk, const uint32_t *__restrict__ rhat,
                      const uint32_t *__restrict__ rhat_sh, const uint32_t *__restrict__ f3,
                      const uint32_t *__restrict__ f0, const uint32_t *__restrict__ x, uint32_t *__restrict__ ct,
@@ -536,8 +548,8 @@ __global__ void __launch_bounds__(NttPlan<LOGN>::T * ppc<LOGN>())
   uint32_t *sm = smem_u32 + threadIdx.y * P::SMEM_WORDS;
   uint32_t a[16], w[16], wsh[16];
   load16(mpk + (size_t)res * P::N + th * 16, a);
-  load16(rhat + (size_t)m * P::N + th * 16, w);
-  load16(rhat_sh + (size_t)m * P::N + th * 16, wsh);
+  load16_own(rhat + (size_t)m * P::N + th * 16, w);
+  load16_own(rhat_sh + (size_t)m * P::N + th * 16, wsh);
 #pragma unroll
   for (int e = 0; e < 16; ++e) a[e] = shoup_mul(a[e], w[e], wsh[e], q);
   ntt_inv_core<LOGN>(a, sm, th, q, sa.ra.ipsi2 + (size_t)m * P::N, sa.ra.ninv[m], sa.ra.ninv_sh[m], sa.ra.w1n[m],
@@ -577,9 +589,9 @@ __global__ void __launch_bounds__(512)
   const uint32_t q = sa.ra.q[m];
   uint32_t *sm = smem_u32 + threadIdx.y * P::SMEM_WORDS;
   uint32_t a[16], w[16], wsh[16];
-  load16(clhat + ((size_t)c * 3 + m) * P::N + th * 16, a);
-  load16(skhat + ((size_t)key * 3 + m) * P::N + th * 16, w);
-  load16(skhat_sh + ((size_t)key * 3 + m) * P::N + th * 16, wsh);
+  load16_own(clhat + ((size_t)c * 3 + m) * P::N + th * 16, a);
+  load16_own(skhat + ((size_t)key * 3 + m) * P::N + th * 16, w);
+  load16_own(skhat_sh + ((size_t)key * 3 + m) * P::N + th * 16, wsh);
 #pragma unroll
   for (int e = 0; e < 16; ++e) a[e] = shoup_mul(a[e], w[e], wsh[e], q);
   ntt_inv_core<LOGN>(a, sm, th, q, sa.ra.ipsi2 + (size_t)m * P::N, sa.ra.ninv[m],

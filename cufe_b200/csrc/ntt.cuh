@@ -17,6 +17,14 @@
 // warps touch 32 consecutive words.  Twiddles use Shoup's precomputed quotient (1 mul.hi +
 // 2 mul.lo per product) and residues stay canonical in [0, q), q < 2^31, between kernels.
 // The inverse folds n^-1 into its last stage.
+//
+// What bounds it: at n = 4096 neither memory (2.9 TB/s of 6.6) nor the multipliers (a large-modulus
+// butterfly's 3 products take 8 of its 11 cycles per warp and subpartition, about 65 % of the kernel's time) but the
+// two together, at 8 warps per subpartition.  Lanes 64 bytes apart cost the load/store unit a visit per
+// cache line, 76 % of its cycles: with 256-bit accesses and the last stage's twiddles laid out for
+// contiguous reads it is 58 %, and 24,576 transforms of 4096 went from 284 to 271 us forward and from 279
+// to 268 inverse, the encryption kernel of 40 instances (l = 784) from 1,331 to 1,241, of a mixed batch of 96
+// from 992 to 875.
 #pragma once
 #include "cufe_internal.cuh"
 
@@ -101,24 +109,49 @@ struct InvScale {
   uint32_t ninv, ninv_sh, w1n, w1n_sh;
 };
 
-// twiddles (w, w_shoup) tw[ti0 .. ti0+NG-1]: pairs of entries per 16-byte load when NG >= 2
-// (ti0 is then even, so the load is aligned)
-template <int NG>
+// 256-bit accesses (32-byte aligned).  The loads may move: no kernel reads what another of its threads writes.
+__device__ __forceinline__ void ld_256(const void *p, uint32_t *r) {
+  asm("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+      : "l"(p));
+}
+__device__ __forceinline__ void st_256(void *p, const uint32_t *r) {
+  asm volatile("st.global.v8.b32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};"
+               :
+               : "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "l"(p)
+               : "memory");
+}
+__device__ __forceinline__ void ldg_256(const void *p, uint32_t *r) {
+  asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+      : "l"(p));
+}
+
+// twiddles (w, w_shoup) tw[ti0 .. ti0+NG-1]: two entries per 16-byte or four per 32-byte load, which
+// are aligned since ti0 is a multiple of NG.  Groups of four are STEP groups apart.
+template <int NG, int STEP = 1>
 __device__ __forceinline__ void load_twiddles(const uint2 *__restrict__ tw, int ti0, uint32_t (&w)[NG],
                                               uint32_t (&wsh)[NG]) {
   if constexpr (NG == 1) {
     const uint2 t = __ldg(tw + ti0);
     w[0] = t.x;
     wsh[0] = t.y;
+  } else if constexpr (NG == 2) {
+    const uint4 t = __ldg(reinterpret_cast<const uint4 *>(tw + ti0));
+    w[0] = t.x;
+    wsh[0] = t.y;
+    w[1] = t.z;
+    wsh[1] = t.w;
   } else {
-    const uint4 *t4 = reinterpret_cast<const uint4 *>(tw + ti0);
 #pragma unroll
-    for (int g = 0; g < NG / 2; ++g) {
-      const uint4 t = __ldg(t4 + g);
-      w[2 * g] = t.x;
-      wsh[2 * g] = t.y;
-      w[2 * g + 1] = t.z;
-      wsh[2 * g + 1] = t.w;
+    for (int g = 0; g < NG / 4; ++g) {
+      uint32_t t[8];
+      ldg_256(tw + ti0 + 4 * g * STEP, t);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        w[4 * g + j] = t[2 * j];
+        wsh[4 * g + j] = t[2 * j + 1];
+      }
     }
   }
 }
@@ -150,7 +183,12 @@ __device__ __forceinline__ void ntt_stage(uint32_t (&a)[P_][E], int th, uint32_t
       }
     } else {
       uint32_t w[ng], wsh[ng];
-      load_twiddles<ng>(tw, (1 << s) + (H << LS), w, wsh);
+      // the last stage's 8 twiddles of a thread are two groups of 4, T groups apart (Ring::init), so that a
+      // warp's loads are contiguous
+      if constexpr (LE == 4 && LS == 3 && plo == 0)
+        load_twiddles<ng, P::T>(tw, (1 << s) + (H << 2), w, wsh);
+      else
+        load_twiddles<ng>(tw, (1 << s) + (H << LS), w, wsh);
 #pragma unroll
       for (int g = 0; g < ng; ++g) {
 #pragma unroll

@@ -11,42 +11,44 @@ constexpr int ppc() {  // residue polynomials per CTA (>= 256 threads per CTA)
   return NttPlan<LOGN, LE>::T >= 256 ? 1 : 256 / NttPlan<LOGN, LE>::T;
 }
 
-__device__ __forceinline__ void load16(const uint32_t *p, uint32_t (&a)[16]) {
-  const uint4 *v = reinterpret_cast<const uint4 *>(p);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const uint4 t = v[i];
-    a[4 * i] = t.x;
-    a[4 * i + 1] = t.y;
-    a[4 * i + 2] = t.z;
-    a[4 * i + 3] = t.w;
-  }
-}
-__device__ __forceinline__ void store16(uint32_t *p, const uint32_t (&a)[16]) {
-  uint4 *v = reinterpret_cast<uint4 *>(p);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) v[i] = make_uint4(a[4 * i], a[4 * i + 1], a[4 * i + 2], a[4 * i + 3]);
-}
-// E consecutive words (E a multiple of 4, p 16-byte aligned)
+// E consecutive words (E a multiple of 16, p 16-byte aligned).  Threads that each hold 16 consecutive
+// coefficients touch a cache line per two lanes, whatever the width of the access, so the widest one has the
+// fewest line visits: 256 bits where the address allows it (arrays of the callers may start on 16 bytes).
 template <int E>
 __device__ __forceinline__ void load_vec(const uint32_t *p, uint32_t (&a)[E]) {
-  const uint4 *v = reinterpret_cast<const uint4 *>(p);
+  if ((reinterpret_cast<uintptr_t>(p) & 31u) == 0) {
 #pragma unroll
-  for (int i = 0; i < E / 4; ++i) {
-    const uint4 t = v[i];
-    a[4 * i] = t.x;
-    a[4 * i + 1] = t.y;
-    a[4 * i + 2] = t.z;
-    a[4 * i + 3] = t.w;
+    for (int i = 0; i < E / 8; ++i) ld_256(p + 8 * i, &a[8 * i]);
+  } else {
+    const uint4 *v = reinterpret_cast<const uint4 *>(p);
+#pragma unroll
+    for (int i = 0; i < E / 4; ++i) {
+      const uint4 t = v[i];
+      a[4 * i] = t.x;
+      a[4 * i + 1] = t.y;
+      a[4 * i + 2] = t.z;
+      a[4 * i + 3] = t.w;
+    }
   }
 }
 template <int E>
 __device__ __forceinline__ void store_vec(uint32_t *p, const uint32_t (&a)[E]) {
-  uint4 *v = reinterpret_cast<uint4 *>(p);
+  if ((reinterpret_cast<uintptr_t>(p) & 31u) == 0) {
 #pragma unroll
-  for (int i = 0; i < E / 4; ++i) v[i] = make_uint4(a[4 * i], a[4 * i + 1], a[4 * i + 2], a[4 * i + 3]);
+    for (int i = 0; i < E / 8; ++i) st_256(p + 8 * i, &a[8 * i]);
+  } else {
+    uint4 *v = reinterpret_cast<uint4 *>(p);
+#pragma unroll
+    for (int i = 0; i < E / 4; ++i) v[i] = make_uint4(a[4 * i], a[4 * i + 1], a[4 * i + 2], a[4 * i + 3]);
+  }
 }
-
+__device__ __forceinline__ void load16(const uint32_t *p, uint32_t (&a)[16]) { load_vec<16>(p, a); }
+// the library's own arrays: aligned, and with no branch that keeps the loads together
+__device__ __forceinline__ void load16_own(const uint32_t *p, uint32_t (&a)[16]) {
+  ld_256(p, &a[0]);
+  ld_256(p + 8, &a[8]);
+}
+__device__ __forceinline__ void store16(uint32_t *p, const uint32_t (&a)[16]) { store_vec<16>(p, a); }
 
 struct SchemeArgs {
   RingArgs ra;
