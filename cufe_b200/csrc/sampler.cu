@@ -333,10 +333,9 @@ struct EndTable {
 };
 constexpr int kCountTile = 4096;
 
-// window of call c: s in [first, first + W)
+// window of call c: s in [first, first + W), first negative (mod 2^32) in the first calls
 __device__ __forceinline__ uint32_t window_first(const EndTable &t, uint32_t c) {
-  const uint32_t mid = (uint32_t)(((uint64_t)t.mean * c) >> 16);
-  return mid > t.W / 2 ? mid - t.W / 2 : 0u;
+  return (uint32_t)(((uint64_t)t.mean * c) >> 16) - t.W / 2;
 }
 
 // accept counts of tile blockIdx.x of stream blockIdx.y
@@ -429,7 +428,8 @@ __global__ void __launch_bounds__(128)
       const uint32_t r = g * kChainRows + i;
       if (r >= calls) break;
       const uint32_t expect = s + (uint32_t)(((uint64_t)t.mean * (r - c)) >> 16), first = window_first(t, r);
-      const uint32_t from = min(expect > first + kChainCols / 2 ? (expect - first - kChainCols / 2) & ~3u : 0u, t.W - kChainCols);
+      const int off = (int)(expect - first) - (int)(kChainCols / 2);
+      const uint32_t from = min(off > 0 ? (uint32_t)off & ~3u : 0u, t.W - kChainCols);
       const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&ring[g % kChainAhead][i][4 * lane]);
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(ends + (size_t)r * t.W + from + 4 * lane)
                    : "memory");
@@ -1172,14 +1172,14 @@ static SegSizes seg_uniform_sizes(uint32_t S, uint32_t calls, uint32_t n, int si
 
 // Width of the table of call ends, 0: k_walk.  The overshoot of a call has a standard deviation
 // below 2, so that of c calls one below 2 sqrt(c): the window takes 4 of those and 64 to either side.  The
-// windows may be n / 2 - 128 wide, so that a threshold is in one of them, and the nearest call to
+// windows may be n - 192 wide, so that a threshold is in one of them, and the nearest call to
 // any of a thread's 128 thresholds is the one whose window it is in (k_ends).  From 128 calls on the
 // three launches are shorter than the walk (sigma_2, n = 4096, one stream / 16, us against the
 // walk's: 64 calls 22 / 25 against 19 / 19, 128 27 / 32 against 31 / 31, 256 35 / 51 against 56 / 57, 785
 // 72 / 114 against 158 / 158).
 static uint32_t end_table_width(const SegSizes &z) {
   const uint32_t W = ((uint32_t)(16.0 * std::sqrt((double)z.max_calls)) + 128 + 63) & ~63u;
-  return z.max_calls >= 128 && 2 * (W + 128) <= z.min_n && z.max_refills < (1u << 28) && z.nstreams < 65536u ? W : 0u;
+  return z.max_calls >= 128 && W + 192 <= z.min_n && z.max_refills < (1u << 28) && z.nstreams < 65536u ? W : 0u;
 }
 
 static uint32_t count_tiles(const SegSizes &z) { return (z.max_refills + kCountTile - 1) / kCountTile; }

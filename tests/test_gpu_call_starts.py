@@ -16,7 +16,7 @@ import cufe_b200 as cf  # noqa: E402
 
 @pytest.mark.parametrize("sig", [0, 1, 2])
 @pytest.mark.parametrize("n,calls", [(16, 700), (256, 200), (1024, 127), (1024, 128), (1024, 200), (2048, 333), (4096, 129),
-                                     (8192, 144), (4096, 3), (512, 128)])
+                                     (8192, 144), (4096, 3), (512, 128), (512, 144), (512, 145), (1024, 785), (1024, 1024)])
 def test_streams_equal_the_oracle(sig, n, calls, rng, oracle_built):
     c = cf.Context(n, 4)
     keys = seeds(rng, 3)
