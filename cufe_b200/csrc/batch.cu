@@ -593,9 +593,8 @@ int Batch::run(cudaStream_t s) {
     if (rc) return rc;
     for (const BatchGroup &g : ch.groups) {
       const size_t nn = (size_t)1 << g.logn;
-      CUFE_CUDA(cudaMemcpy2DAsync(rh + g.rh, 3 * nn * 4, s2o + g.s2o, 6 * nn * 4, 3 * nn * 4, g.count,
-                                  cudaMemcpyDeviceToDevice, s));
-      rc = ntt_fwd_shoup_launch(ctx[(int)nn]->ring.args, rh + g.rh, rhsh + g.rh, (long long)g.count * 3, s);
+      rc = ntt_fwd_from_launch(ctx[(int)nn]->ring.args, s2o + g.s2o, 6 * nn, rh + g.rh, rhsh + g.rh,
+                               (long long)g.count * 3, s);
       if (rc) return rc;
     }
     rc = sample_cpu_map_seg(2, sg3, ch.z3, rk3 + (size_t)ch.first * 60, f3, samp, status, num_sms, s);
@@ -1122,10 +1121,8 @@ struct Server {
         return rc;
       for (const BatchGroup &g : groups) {
         const size_t nn1 = (size_t)1 << g.logn;
-        CUFE_CUDA(cudaMemcpy2DAsync(rh + g.rh, 3 * nn1 * 4, s2o + g.s2o, 6 * nn1 * 4, 3 * nn1 * 4, g.count,
-                                    cudaMemcpyDeviceToDevice, stream));
-        if ((rc = ntt_fwd_shoup_launch(tenants.ctx[(int)nn1]->ring.args, rh + g.rh, rhsh + g.rh,
-                                       (long long)g.count * 3, stream)))
+        if ((rc = ntt_fwd_from_launch(tenants.ctx[(int)nn1]->ring.args, s2o + g.s2o, 6 * nn1, rh + g.rh, rhsh + g.rh,
+                                      (long long)g.count * 3, stream)))
           return rc;
       }
       if ((rc = sample_cpu_map_seg(2, seg_bind(d_tab + seg3, ne), z3, rk + (size_t)ne * 60, f3, samp, tenants.status,

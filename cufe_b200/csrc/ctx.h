@@ -60,6 +60,9 @@ struct Ctx {
 };
 
 int ntt_launch(const RingArgs &ra, uint32_t *data, long long nres, bool inverse, cudaStream_t s);
+// forward from rows of k residues src_row words apart (data itself, or no overlap); sh: companions, or NULL
+int ntt_fwd_from_launch(const RingArgs &ra, const uint32_t *src, size_t src_row, uint32_t *data, uint32_t *sh,
+                        long long nres, cudaStream_t s);
 int ntt_fwd_shoup_launch(const RingArgs &ra, uint32_t *data, uint32_t *sh, long long nres, cudaStream_t s);
 // times the NTT variants on npoly scratch polynomials, keeps the fastest per direction in
 // r.args; ms[2 * CUFE_NTT_VARIANTS] (optional): {fwd v1.., inv v1..} in ms per launch

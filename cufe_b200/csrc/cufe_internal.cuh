@@ -28,6 +28,7 @@ struct RingArgs {
   uint32_t ninv[kMaxModuli], ninv_sh[kMaxModuli];  // n^-1
   uint32_t w1n[kMaxModuli], w1n_sh[kMaxModuli];    // psi_inv[1] * n^-1 (last inverse stage)
   uint32_t qr[kMaxModuli];                          // floor(2^32 / q)
+  uint64_t mu[kMaxModuli];                          // floor(2^64 / q)
   // [k][n] (w, w_shoup) each.  The last stage's entries (n / 2 .. n - 1) in the order in which 16
   // coefficients per thread use them: of every thread's 8, first all threads' first 4, then their others;
   // psi2_flat, ipsi2_flat in plain order, for the transforms with more coefficients per thread.

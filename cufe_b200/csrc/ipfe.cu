@@ -157,6 +157,7 @@ int Ring::init(int n_, int k_, const uint32_t *primes, int dev) {
     args.w1n[m] = (uint32_t)((uint64_t)h_ipsi[(size_t)m * n + 1] * args.ninv[m] % qq);
     args.w1n_sh[m] = shoup_of(args.w1n[m], (uint32_t)qq);
     args.qr[m] = (uint32_t)((1ull << 32) / qq);
+    args.mu[m] = (uint64_t)(((u128)1 << 64) / qq);
   }
   args.n = n;
   args.logn = logn;
@@ -183,8 +184,17 @@ void Ring::release() {
 
 namespace {
 
+// Shoup companion floor(w 2^32 / q) of w < q, mu = floor(2^64 / q): floor(w mu / 2^32) is that or one
+// less, and the remainder -s q (mod 2^32) tells which.  (1,773 transforms of 2048 with companions took
+// 50 us with a 64-bit division and a copy of the input, now 32 without either.)
+__device__ __forceinline__ uint32_t shoup_companion(uint32_t w, uint64_t mu, uint32_t q) {
+  const uint32_t s = w * (uint32_t)(mu >> 32) + __umulhi(w, (uint32_t)mu);
+  return 0u - s * q >= q ? s + 1 : s;
+}
+
 // MODE 0 forward, 1 forward + Shoup companions into sh, 2 inverse.  data holds `rows`
-// polynomials of k residues ([row][k][n]); a thread group transforms PP residues of one
+// polynomials of k residues ([row][k][n]); the forward modes read src, rows src_row words apart, which
+// may be data itself (a thread group reads its residues before it writes them).  A thread group transforms PP residues of one
 // modulus m, rows PP*t .. PP*t+PP-1, sharing twiddles and shared-memory addresses.
 // LBT, MINB: the launch bounds the registers are allocated for -- LBT threads per CTA (at
 // least the CTA's real size) and MINB CTAs per SM.  Variant 1 uses (512, 1): at most 128
@@ -202,7 +212,8 @@ struct ModSel {
 // the launcher runs one grid over the small moduli and one over the others.
 template <int LOGN, int MODE, int PP, int LBT = 512, int MINB = 1, int LE = 4, bool SQ = false>
 __global__ void __launch_bounds__(LBT, MINB)
-    k_ntt(uint32_t *__restrict__ data, uint32_t *__restrict__ sh, long long rows, RingArgs ra, ModSel sel) {
+    k_ntt(const uint32_t *src, long long src_row, uint32_t *data, uint32_t *__restrict__ sh, long long rows,
+          RingArgs ra, ModSel sel) {
   using P = NttPlan<LOGN, LE>;
   constexpr int E = P::E;
   extern __shared__ uint32_t smem_u32[];
@@ -225,7 +236,7 @@ __global__ void __launch_bounds__(LBT, MINB)
   if (MODE != 2) {
 #pragma unroll
     for (int p = 0; p < PP; ++p) {
-      const uint32_t *d = data + res[p] * P::N;
+      const uint32_t *d = src + (live[p] ? row0 + p : row0) * src_row + m * P::N;
 #pragma unroll
       for (int e = 0; e < E; ++e) a[p][e] = d[P::template idx<0>(th, e)];
     }
@@ -237,7 +248,7 @@ __global__ void __launch_bounds__(LBT, MINB)
       if (MODE == 1) {
         uint32_t b[E];
 #pragma unroll
-        for (int e = 0; e < E; ++e) b[e] = (uint32_t)(((uint64_t)a[p][e] << 32) / q);
+        for (int e = 0; e < E; ++e) b[e] = shoup_companion(a[p][e], ra.mu[m], q);
         store_vec(sh + res[p] * P::N + th * E, b);
       }
     }
@@ -257,8 +268,8 @@ __global__ void __launch_bounds__(LBT, MINB)
 }
 
 template <int LOGN, int MODE, int PP, int LBT, int MINB, int LE, bool SQ>
-int launch_ntt_sel(const RingArgs &ra, const ModSel &sel, uint32_t *data, uint32_t *sh, long long rows,
-                   cudaStream_t s) {
+int launch_ntt_sel(const RingArgs &ra, const ModSel &sel, const uint32_t *src, long long src_row, uint32_t *data,
+                   uint32_t *sh, long long rows, cudaStream_t s) {
   using P = NttPlan<LOGN, LE>;
   constexpr int G = ppc<LOGN, LE>();
   const size_t smem = (size_t)G * PP * P::SMEM_WORDS * 4;
@@ -271,25 +282,42 @@ int launch_ntt_sel(const RingArgs &ra, const ModSel &sel, uint32_t *data, uint32
   const long long groups = (rows + PP - 1) / PP * sel.nm;
   const long long grid = (groups + G - 1) / G;
   if (grid <= 0) return CUFE_OK;
-  note_launch(), k_ntt<LOGN, MODE, PP, LBT, MINB, LE, SQ><<<(unsigned)grid, dim3(P::T, G), smem, s>>>(data, sh, rows, ra, sel);
+  note_launch(), k_ntt<LOGN, MODE, PP, LBT, MINB, LE, SQ><<<(unsigned)grid, dim3(P::T, G), smem, s>>>(src, src_row, data, sh,
+                                                                                                     rows, ra, sel);
   CUFE_CUDA(cudaGetLastError());
   return CUFE_OK;
 }
 
-// one grid over the moduli below kSmallQ (lazy butterflies), one over the rest
+inline int device_sms() {
+  static int sms[64] = {0};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+  if (!sms[dev] && cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    sms[dev] = 148;
+  return sms[dev];
+}
+
+// One grid over the moduli below kSmallQ (lazy butterflies), one over the rest; where all of them are at most
+// a CTA per SM, one grid with the butterflies that serve both, since a launch then takes the latency of
+// one transform whatever is in it (three residues of 1024 with companions: 16.4 us in two launches, now 5).
 template <int LOGN, int MODE, int PP, int LBT = 512, int MINB = 1, int LE = 4>
-int launch_ntt_pp(const RingArgs &ra, uint32_t *data, uint32_t *sh, long long rows, cudaStream_t s) {
-  ModSel small{0, {}}, large{0, {}};
+int launch_ntt_pp(const RingArgs &ra, const uint32_t *src, long long src_row, uint32_t *data, uint32_t *sh,
+                  long long rows, cudaStream_t s) {
+  ModSel small{0, {}}, large{0, {}}, all{ra.k, {}};
   for (int m = 0; m < ra.k; ++m) {
+    all.m[m] = m;
     if (ra.q[m] < kSmallQ)
       small.m[small.nm++] = m;
     else
       large.m[large.nm++] = m;
   }
   ProfScope ps(MODE == 2 ? "ntt_inverse" : "ntt_forward", s);
+  if (small.nm && large.nm && (rows + PP - 1) / PP * ra.k <= (long long)ppc<LOGN, LE>() * device_sms())
+    return launch_ntt_sel<LOGN, MODE, PP, LBT, MINB, LE, false>(ra, all, src, src_row, data, sh, rows, s);
   int rc = CUFE_OK;
-  if (small.nm) rc = launch_ntt_sel<LOGN, MODE, PP, LBT, MINB, LE, true>(ra, small, data, sh, rows, s);
-  if (!rc && large.nm) rc = launch_ntt_sel<LOGN, MODE, PP, LBT, MINB, LE, false>(ra, large, data, sh, rows, s);
+  if (small.nm) rc = launch_ntt_sel<LOGN, MODE, PP, LBT, MINB, LE, true>(ra, small, src, src_row, data, sh, rows, s);
+  if (!rc && large.nm)
+    rc = launch_ntt_sel<LOGN, MODE, PP, LBT, MINB, LE, false>(ra, large, src, src_row, data, sh, rows, s);
   return rc;
 }
 
@@ -298,8 +326,8 @@ int launch_ntt_pp(const RingArgs &ra, uint32_t *data, uint32_t *sh, long long ro
 // CTA keeps a residue's worth of loads in flight while it computes.  One residue per thread
 // group; the trip count is uniform per CTA (the exchanges synchronise the CTA).
 template <int LOGN, int MODE>
-__global__ void __maxnreg__(80) k_ntt_stream(uint32_t *__restrict__ data, uint32_t *__restrict__ sh,
-                                                    long long nres, RingArgs ra) {
+__global__ void __maxnreg__(80) k_ntt_stream(const uint32_t *src, long long src_row, uint32_t *data,
+                                                    uint32_t *__restrict__ sh, long long nres, RingArgs ra) {
   using P = NttPlan<LOGN>;
   extern __shared__ uint32_t smem_u32[];
   const int th = threadIdx.x;
@@ -310,12 +338,13 @@ __global__ void __maxnreg__(80) k_ntt_stream(uint32_t *__restrict__ data, uint32
   const long long r0 = cta0 + threadIdx.y;
   uint32_t nx[16];
   {
-    const uint32_t *d = data + (r0 < nres ? r0 : nres - 1) * P::N;
+    const long long r = r0 < nres ? r0 : nres - 1;
     if (MODE != 2) {
+      const uint32_t *d = src + r / ra.k * src_row + r % ra.k * P::N;
 #pragma unroll
       for (int e = 0; e < 16; ++e) nx[e] = d[P::template idx<0>(th, e)];
     } else {
-      load16(d + th * 16, nx);
+      load16(data + r * P::N + th * 16, nx);
     }
   }
   for (long long it = 0; it < iters; ++it) {
@@ -327,12 +356,13 @@ __global__ void __maxnreg__(80) k_ntt_stream(uint32_t *__restrict__ data, uint32
     for (int e = 0; e < 16; ++e) a[e] = nx[e];
     if (it + 1 < iters) {
       const long long nxt = cur + stride;
-      const uint32_t *d = data + (nxt < nres ? nxt : nres - 1) * P::N;
+      const long long r = nxt < nres ? nxt : nres - 1;
       if (MODE != 2) {
+        const uint32_t *d = src + r / ra.k * src_row + r % ra.k * P::N;
 #pragma unroll
         for (int e = 0; e < 16; ++e) nx[e] = d[P::template idx<0>(th, e)];
       } else {
-        load16(d + th * 16, nx);
+        load16(data + r * P::N + th * 16, nx);
       }
     }
     const int m = (int)(cc % ra.k);
@@ -345,7 +375,7 @@ __global__ void __maxnreg__(80) k_ntt_stream(uint32_t *__restrict__ data, uint32
         if (MODE == 1) {
           uint32_t b[16];
 #pragma unroll
-          for (int e = 0; e < 16; ++e) b[e] = (uint32_t)(((uint64_t)a[e] << 32) / q);
+          for (int e = 0; e < 16; ++e) b[e] = shoup_companion(a[e], ra.mu[m], q);
           store16(sh + cc * P::N + th * 16, b);
         }
       }
@@ -361,17 +391,9 @@ __global__ void __maxnreg__(80) k_ntt_stream(uint32_t *__restrict__ data, uint32
   }
 }
 
-inline int device_sms() {
-  static int sms[64] = {0};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-  if (!sms[dev] && cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-    sms[dev] = 148;
-  return sms[dev];
-}
-
 template <int LOGN, int MODE>
-int launch_ntt_stream(const RingArgs &ra, uint32_t *data, uint32_t *sh, long long nres, cudaStream_t s) {
+int launch_ntt_stream(const RingArgs &ra, const uint32_t *src, long long src_row, uint32_t *data, uint32_t *sh, long long nres,
+    cudaStream_t s) {
   using P = NttPlan<LOGN>;
   constexpr int G = ppc<LOGN>();
   const size_t smem = (size_t)G * P::SMEM_WORDS * 4;
@@ -385,49 +407,51 @@ int launch_ntt_stream(const RingArgs &ra, uint32_t *data, uint32_t *sh, long lon
   const long long grid = std::min(need, (long long)device_sms() * occ);
   if (grid <= 0) return CUFE_OK;
   ProfScope ps(MODE == 2 ? "ntt_inverse" : "ntt_forward", s);
-  note_launch(), k_ntt_stream<LOGN, MODE><<<(unsigned)grid, dim3(P::T, G), smem, s>>>(data, sh, nres, ra);
+  note_launch(), k_ntt_stream<LOGN, MODE><<<(unsigned)grid, dim3(P::T, G), smem, s>>>(src, src_row, data, sh, nres, ra);
   CUFE_CUDA(cudaGetLastError());
   return CUFE_OK;
 }
 
 // residues per thread group: the ring's tuned choice for this direction, else 1
 template <int LOGN, int MODE>
-int launch_ntt_t(const RingArgs &ra, uint32_t *data, uint32_t *sh, long long nres, cudaStream_t s) {
+int launch_ntt_t(const RingArgs &ra, const uint32_t *src, long long src_row, uint32_t *data, uint32_t *sh, long long nres,
+    cudaStream_t s) {
   if (nres % ra.k) return CUFE_ERR_INVALID;
   const long long rows = nres / ra.k;
   const int pp = MODE == 2 ? ra.pp_inv : ra.pp_fwd;
-  if (pp == 3) return launch_ntt_stream<LOGN, MODE>(ra, data, sh, nres, s);
+  if (pp == 3) return launch_ntt_stream<LOGN, MODE>(ra, src, src_row, data, sh, nres, s);
   constexpr int nt = NttPlan<LOGN>::T * ppc<LOGN>();  // threads per CTA
-  if (pp == 2 && rows >= 2) return launch_ntt_pp<LOGN, MODE, 2, nt, 1>(ra, data, sh, rows, s);
-  if (pp == 4) return launch_ntt_pp<LOGN, MODE, 1, nt, nt <= 256 ? 5 : 2>(ra, data, sh, rows, s);
-  if (pp == 5 && rows >= 2) return launch_ntt_pp<LOGN, MODE, 2, nt, nt <= 256 ? 3 : 1>(ra, data, sh, rows, s);
-  if (pp == 6 && rows >= 2) return launch_ntt_pp<LOGN, MODE, 2, nt, nt <= 256 ? 4 : 2>(ra, data, sh, rows, s);
+  if (pp == 2 && rows >= 2) return launch_ntt_pp<LOGN, MODE, 2, nt, 1>(ra, src, src_row, data, sh, rows, s);
+  if (pp == 4) return launch_ntt_pp<LOGN, MODE, 1, nt, nt <= 256 ? 5 : 2>(ra, src, src_row, data, sh, rows, s);
+  if (pp == 5 && rows >= 2) return launch_ntt_pp<LOGN, MODE, 2, nt, nt <= 256 ? 3 : 1>(ra, src, src_row, data, sh, rows, s);
+  if (pp == 6 && rows >= 2) return launch_ntt_pp<LOGN, MODE, 2, nt, nt <= 256 ? 4 : 2>(ra, src, src_row, data, sh, rows, s);
   // radix 32 and 64: 32 or 64 coefficients per thread, fewer passes and exchanges
   if constexpr (LOGN >= 10) {
     constexpr int nt5 = NttPlan<LOGN, 5>::T * ppc<LOGN, 5>();
-    if (pp == 7) return launch_ntt_pp<LOGN, MODE, 1, nt5, 2, 5>(ra, data, sh, rows, s);
-    if (pp == 8) return launch_ntt_pp<LOGN, MODE, 1, nt5, 3, 5>(ra, data, sh, rows, s);
+    if (pp == 7) return launch_ntt_pp<LOGN, MODE, 1, nt5, 2, 5>(ra, src, src_row, data, sh, rows, s);
+    if (pp == 8) return launch_ntt_pp<LOGN, MODE, 1, nt5, 3, 5>(ra, src, src_row, data, sh, rows, s);
   }
   if constexpr (LOGN >= 11) {
     constexpr int nt6 = NttPlan<LOGN, 6>::T * ppc<LOGN, 6>();
-    if (pp == 9) return launch_ntt_pp<LOGN, MODE, 1, nt6, 2, 6>(ra, data, sh, rows, s);
+    if (pp == 9) return launch_ntt_pp<LOGN, MODE, 1, nt6, 2, 6>(ra, src, src_row, data, sh, rows, s);
   }
-  return launch_ntt_pp<LOGN, MODE, 1>(ra, data, sh, rows, s);
+  return launch_ntt_pp<LOGN, MODE, 1>(ra, src, src_row, data, sh, rows, s);
 }
 
 template <int MODE>
-int launch_ntt(const RingArgs &ra, uint32_t *data, uint32_t *sh, long long nres, cudaStream_t s) {
+int launch_ntt(const RingArgs &ra, const uint32_t *src, long long src_row, uint32_t *data, uint32_t *sh, long long nres,
+    cudaStream_t s) {
   switch (ra.logn) {
-    case 4: return launch_ntt_t<4, MODE>(ra, data, sh, nres, s);
-    case 5: return launch_ntt_t<5, MODE>(ra, data, sh, nres, s);
-    case 6: return launch_ntt_t<6, MODE>(ra, data, sh, nres, s);
-    case 7: return launch_ntt_t<7, MODE>(ra, data, sh, nres, s);
-    case 8: return launch_ntt_t<8, MODE>(ra, data, sh, nres, s);
-    case 9: return launch_ntt_t<9, MODE>(ra, data, sh, nres, s);
-    case 10: return launch_ntt_t<10, MODE>(ra, data, sh, nres, s);
-    case 11: return launch_ntt_t<11, MODE>(ra, data, sh, nres, s);
-    case 12: return launch_ntt_t<12, MODE>(ra, data, sh, nres, s);
-    case 13: return launch_ntt_t<13, MODE>(ra, data, sh, nres, s);
+    case 4: return launch_ntt_t<4, MODE>(ra, src, src_row, data, sh, nres, s);
+    case 5: return launch_ntt_t<5, MODE>(ra, src, src_row, data, sh, nres, s);
+    case 6: return launch_ntt_t<6, MODE>(ra, src, src_row, data, sh, nres, s);
+    case 7: return launch_ntt_t<7, MODE>(ra, src, src_row, data, sh, nres, s);
+    case 8: return launch_ntt_t<8, MODE>(ra, src, src_row, data, sh, nres, s);
+    case 9: return launch_ntt_t<9, MODE>(ra, src, src_row, data, sh, nres, s);
+    case 10: return launch_ntt_t<10, MODE>(ra, src, src_row, data, sh, nres, s);
+    case 11: return launch_ntt_t<11, MODE>(ra, src, src_row, data, sh, nres, s);
+    case 12: return launch_ntt_t<12, MODE>(ra, src, src_row, data, sh, nres, s);
+    case 13: return launch_ntt_t<13, MODE>(ra, src, src_row, data, sh, nres, s);
   }
   return CUFE_ERR_INVALID;
 }
@@ -778,10 +802,16 @@ __global__ void k_decode_triples(const uint32_t *__restrict__ d0, long long npai
 }  // namespace
 
 int ntt_launch(const RingArgs &ra, uint32_t *data, long long nres, bool inverse, cudaStream_t s) {
-  return inverse ? launch_ntt<2>(ra, data, nullptr, nres, s) : launch_ntt<0>(ra, data, nullptr, nres, s);
+  const long long row = (long long)ra.k * ra.n;
+  return inverse ? launch_ntt<2>(ra, data, row, data, nullptr, nres, s) : launch_ntt<0>(ra, data, row, data, nullptr, nres, s);
+}
+int ntt_fwd_from_launch(const RingArgs &ra, const uint32_t *src, size_t src_row, uint32_t *data, uint32_t *sh,
+                        long long nres, cudaStream_t s) {
+  return sh ? launch_ntt<1>(ra, src, (long long)src_row, data, sh, nres, s)
+            : launch_ntt<0>(ra, src, (long long)src_row, data, nullptr, nres, s);
 }
 int ntt_fwd_shoup_launch(const RingArgs &ra, uint32_t *data, uint32_t *sh, long long nres, cudaStream_t s) {
-  return launch_ntt<1>(ra, data, sh, nres, s);
+  return ntt_fwd_from_launch(ra, data, (size_t)ra.k * ra.n, data, sh, nres, s);
 }
 
 int ring_tune(Ring &r, long long npoly, float *ms, cudaStream_t s) {
@@ -987,11 +1017,11 @@ int ctx_setup_cpu_map_l(Ctx &c, int l, const uint8_t *seed_a, const uint8_t *see
   const int n = c.n;
   const size_t poly = (size_t)3 * n;
   const size_t samp_ws = cpu_map_workspace_bytes(2, l, n, 0);
-  int rc = c.ensure_ws(samp_ws + (2 * l + 2) * poly * 4 + 4096 + 4 * 60 * 4);
+  int rc = c.ensure_ws(samp_ws + (l + 2) * poly * 4 + 4096 + 4 * 60 * 4);
   if (rc) return rc;
   Arena ar(c.ws);
   uint32_t *rk = ar.take<uint32_t>(3 * 60);
-  uint32_t *se = ar.take<uint32_t>(2 * (size_t)l * poly);  // [2][l][3][n]: s, e
+  uint32_t *e = ar.take<uint32_t>((size_t)l * poly);
   uint32_t *a_sh = ar.take<uint32_t>(poly);
   void *sws = ar.take<uint8_t>(samp_ws);
   std::vector<uint32_t> keys(3 * 60, 0u);
@@ -1001,10 +1031,9 @@ int ctx_setup_cpu_map_l(Ctx &c, int l, const uint8_t *seed_a, const uint8_t *see
   CUFE_CUDA(cudaMemcpyAsync(rk, keys.data(), keys.size() * 4, cudaMemcpyHostToDevice, s));
   rc = sample_polya(rk, n, d_mpk + (size_t)l * poly, s);
   if (rc) return rc;
-  rc = sample_cpu_map(0, 2, rk + 60, l, n, se, sws, c.d_status, c.num_sms, s);
+  rc = sample_cpu_map(0, 2, rk + 60, l, n, d_msk, sws, c.d_status, c.num_sms, s, e);
   if (rc) return rc;
-  CUFE_CUDA(cudaMemcpyAsync(d_msk, se, (size_t)l * poly * 4, cudaMemcpyDeviceToDevice, s));
-  return setup_tail(c, l, d_mpk, d_msk, se + (size_t)l * poly, a_sh, s);
+  return setup_tail(c, l, d_mpk, d_msk, e, a_sh, s);
 }
 
 int ctx_setup_gpu_map(Ctx &c, const uint8_t *seed2, const uint8_t *seed3, uint32_t *d_mpk, uint32_t *d_msk,
@@ -1092,8 +1121,7 @@ int ctx_encrypt_cpu_map(Ctx &c, int batch, const uint32_t *d_x, const uint32_t *
   if (rc) return rc;
   rc = sample_cpu_map(2, batch, rk + (size_t)batch * 60, l, n, f3, sws3, c.d_status, c.num_sms, s);
   if (rc) return rc;
-  CUFE_CUDA(cudaMemcpy2DAsync(rhat, poly * 4, s2o, 2 * poly * 4, poly * 4, batch, cudaMemcpyDeviceToDevice, s));
-  rc = ntt_fwd_shoup_launch(c.ring.args, rhat, rhat_sh, (long long)batch * 3, s);
+  rc = ntt_fwd_from_launch(c.ring.args, s2o, 2 * poly, rhat, rhat_sh, (long long)batch * 3, s);
   if (rc) return rc;
   return encrypt_tail(c, batch, d_x, d_mpk, rhat, rhat_sh, (long long)poly, f3, (long long)l * poly, s2o + poly,
                       (long long)2 * poly, d_ct, s);
@@ -1121,8 +1149,7 @@ int ctx_encrypt_gpu_map(Ctx &c, int batch, const uint32_t *d_x, const uint32_t *
   if (rc) return rc;
   rc = sample_gpu_map(2, rk, 0, l, n, f3, c.d_status, c.num_sms, s);
   if (rc) return rc;
-  CUFE_CUDA(cudaMemcpyAsync(rhat, r, poly * 4, cudaMemcpyDeviceToDevice, s));
-  rc = ntt_fwd_shoup_launch(c.ring.args, rhat, rhat_sh, 3, s);
+  rc = ntt_fwd_from_launch(c.ring.args, r, poly, rhat, rhat_sh, 3, s);
   if (rc) return rc;
   const SchemeArgs sa = scheme_args(c);
   return dispatch_logn(c.ring.logn, [&](auto L) {
@@ -1164,12 +1191,9 @@ static int decrypt_with(Ctx &c, int nct, const uint32_t *d_ct, int nkeys, const 
   const size_t poly = (size_t)3 * c.n, ct_words = (size_t)(c.l + 1) * poly;
   const long long nwork = (long long)nct * nkeys * 3;
   const SchemeArgs sa = scheme_args(c);
-  CUFE_CUDA(cudaMemcpy2DAsync(clhat, poly * 4, d_ct + (size_t)c.l * poly, ct_words * 4, poly * 4, nct,
-                              cudaMemcpyDeviceToDevice, s));
-  int rc = ntt_launch(c.ring.args, clhat, (long long)nct * 3, false, s);
+  int rc = ntt_fwd_from_launch(c.ring.args, d_ct + (size_t)c.l * poly, ct_words, clhat, nullptr, (long long)nct * 3, s);
   if (rc) return rc;
-  CUFE_CUDA(cudaMemcpyAsync(skhat, d_sky, (size_t)nkeys * poly * 4, cudaMemcpyDeviceToDevice, s));
-  rc = ntt_fwd_shoup_launch(c.ring.args, skhat, skhat_sh, (long long)nkeys * 3, s);
+  rc = ntt_fwd_from_launch(c.ring.args, d_sky, poly, skhat, skhat_sh, (long long)nkeys * 3, s);
   if (rc) return rc;
   {
     ProfScope ps("decrypt_mac", s);

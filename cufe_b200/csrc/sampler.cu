@@ -1255,15 +1255,18 @@ int sample_cpu_map_seg(int sig, const SegDev &sg, const SegSizes &z, const uint3
 
 // the uniform case: nstreams equal streams, no tables
 int sample_cpu_map(int sig, uint32_t nstreams, const uint32_t *d_rkeys, uint32_t calls, uint32_t n,
-                   uint32_t *d_out, void *ws, uint32_t *d_status, int num_sms, cudaStream_t s) {
+                   uint32_t *d_out, void *ws, uint32_t *d_status, int num_sms, cudaStream_t s, uint32_t *d_out1) {
   const SegSizes z = seg_uniform_sizes(nstreams, calls, n, sig);
   if (z.refills / nstreams >= (1ull << 32) / 24) return CUFE_ERR_INVALID;  // AES counter range
+  if (d_out1 && nstreams != 2) return CUFE_ERR_INVALID;
   SegDev sg{};
   sg.nstreams = nstreams;
   sg.u_n = n;
   sg.u_calls = calls;
   sg.u_refills = (uint32_t)(z.refills / nstreams);
   sg.u_ostride = (uint64_t)calls * 3 * n;
+  if (d_out1)  // two streams: the distance between their outputs, wherever they lie
+    sg.u_ostride = (uint64_t)((reinterpret_cast<intptr_t>(d_out1) - reinterpret_cast<intptr_t>(d_out)) / 4);
   return sample_cpu_map_seg(sig, sg, z, d_rkeys, d_out, ws, d_status, num_sms, s);
 }
 

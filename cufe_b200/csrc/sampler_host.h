@@ -21,18 +21,19 @@ int expand_keys_device(const uint8_t *d_seeds, const uint32_t *d_perm, uint32_t 
 
 // CPU stream mapping: nstreams independent AES-CTR streams (round keys d_rkeys[nstreams][60],
 // nonce 0, counter 0), each running `calls` consecutive sampler calls of n samples with
-// sigma index sig; residues written to d_out[nstreams][calls][3][n].
+// sigma index sig; residues written to d_out[nstreams][calls][3][n], those of the second of two to d_out1 where given.
 uint32_t cpu_map_refills(uint32_t calls, uint32_t n, int sig);
 size_t cpu_map_workspace_bytes(uint32_t nstreams, uint32_t calls, uint32_t n, int sig);
 int sample_cpu_map(int sig, uint32_t nstreams, const uint32_t *d_rkeys, uint32_t calls, uint32_t n,
-                   uint32_t *d_out, void *ws, uint32_t *d_status, int num_sms, cudaStream_t s);
+                   uint32_t *d_out, void *ws, uint32_t *d_status, int num_sms, cudaStream_t s,
+                   uint32_t *d_out1 = nullptr);
 
 // Segmented form: S CPU-mapping streams of different lengths.  Stream s runs calls[s]
 // sampler calls of n[s] samples; its refills occupy [roff[s], roff[s+1]) of the flattened
 // refill space (multiples of 32), its call starts call_start[coff[s] + s .. coff[s+1] + s] (calls + 1
 // entries), and the scatter writes its residues to out[ooff[s] + c * 3 n[s] ...][3][n[s]].  Round
 // keys rkeys[s][60].  Without tables (n == nullptr) the streams are equal: u_calls calls of u_n
-// samples, u_refills refills, u_ostride words of output each.
+// samples, u_refills refills, output u_ostride words apart (mod 2^64: backwards too).
 struct SegDev {
   uint32_t nstreams;
   const uint32_t *n, *calls;

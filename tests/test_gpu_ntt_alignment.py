@@ -1,6 +1,7 @@
 """Transforms and key material on buffers that start on a 16-byte but not a 32-byte boundary: the
 kernels that hold 16 consecutive coefficients per thread read and write 256 bits at a time where the
-address allows it and 128 where it does not.  Both must give the same residues."""
+address allows it and 128 where it does not.  Both must give the same residues, and so must the launches
+for few and for many transforms."""
 import numpy as np
 import pytest
 
@@ -30,6 +31,19 @@ def test_transforms(n, variant, rng):
     f, g = ring.forward(a.clone()), ring.forward(b)
     assert torch.equal(f, g)
     assert torch.equal(ring.inverse(g), a) and torch.equal(ring.inverse(f), a)
+    ring.close()
+
+
+@pytest.mark.parametrize("n,rows", [(1024, 394), (1024, 395), (4096, 98), (4096, 99), (8192, 1), (8192, 100)])
+def test_one_launch_or_two(n, rows, rng):
+    """few transforms go in one launch for all moduli, more in one per class of modulus: the same residues"""
+    ring = cf.Ring(n, 3)
+    a = cf.to_dev(np.stack([rng.integers(0, q, (rows, n), dtype=np.uint32) for q in ring.primes], axis=1))
+    f = ring.forward(a.clone())
+    for i in range(0, rows, 40):
+        assert torch.equal(ring.forward(a[i:i + 40].clone()), f[i:i + 40])
+        assert torch.equal(ring.inverse(f[i:i + 40].clone()), a[i:i + 40])
+    assert torch.equal(ring.inverse(f), a)
     ring.close()
 
 
