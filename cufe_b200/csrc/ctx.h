@@ -43,6 +43,12 @@ struct Ctx {
   uint8_t *ws = nullptr;
   size_t ws_bytes = 0;
   uint32_t *d_status = nullptr;  // sampler status word (device)
+  // a second stream for the part of a call that does not depend on the rest: fork() makes it wait for
+  // what is queued on s, join() makes s wait for it
+  cudaStream_t side = nullptr;
+  cudaEvent_t forked = nullptr, joined = nullptr;
+  int fork(cudaStream_t s);
+  int join(cudaStream_t s);
   std::mutex mu;                 // serialises host calls on this context
   Prof prof;                     // per-kernel timing (cufe_profile_*)
   // shapes chosen by the tuners (cufe_tune_*): encryption instances per thread group by batch

@@ -873,6 +873,9 @@ int Ctx::init(int n_, int l_, int dev) {
   CUFE_CUDA(cudaSetDevice(device));
   CUFE_CUDA(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, device));
   CUFE_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+  CUFE_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+  CUFE_CUDA(cudaEventCreateWithFlags(&forked, cudaEventDisableTiming));
+  CUFE_CUDA(cudaEventCreateWithFlags(&joined, cudaEventDisableTiming));
   CUFE_CUDA(cudaMalloc(&d_status, 256));
   CUFE_CUDA(cudaMemset(d_status, 0, 256));
   rc = sampler_init_device();
@@ -896,10 +899,27 @@ void Ctx::release() {
   if (ws) cudaFree(ws);
   if (d_status) cudaFree(d_status);
   if (stream) cudaStreamDestroy(stream);
+  if (side) cudaStreamDestroy(side);
+  if (forked) cudaEventDestroy(forked);
+  if (joined) cudaEventDestroy(joined);
+  side = nullptr;
+  forked = joined = nullptr;
   ring.release();
   ws = nullptr;
   d_status = nullptr;
   stream = nullptr;
+}
+
+int Ctx::fork(cudaStream_t s) {
+  CUFE_CUDA(cudaEventRecord(forked, s));
+  CUFE_CUDA(cudaStreamWaitEvent(side, forked, 0));
+  return CUFE_OK;
+}
+
+int Ctx::join(cudaStream_t s) {
+  CUFE_CUDA(cudaEventRecord(joined, side));
+  CUFE_CUDA(cudaStreamWaitEvent(s, joined, 0));
+  return CUFE_OK;
 }
 
 int Ctx::ensure_ws(size_t bytes) {
@@ -984,15 +1004,17 @@ static int dispatch_logn(int logn, F &&f) {
   return CUFE_ERR_INVALID;
 }
 
-// shared tail of both setups: a^ = NTT(a) in place, e^ = NTT(e), mpk_i = a^ NTT(s_i) + e^_i
-static int setup_tail(Ctx &c, int l, uint32_t *d_mpk, const uint32_t *d_msk, uint32_t *e, uint32_t *a_sh,
+// shared tail of both setups: a^ = NTT(a) in place (already on the side stream if forked), e^ = NTT(e),
+// mpk_i = a^ NTT(s_i) + e^_i
+static int setup_tail(Ctx &c, int l, uint32_t *d_mpk, const uint32_t *d_msk, uint32_t *e, uint32_t *a_sh, bool forked,
                       cudaStream_t s) {
   const int n = c.n;
   uint32_t *ahat = d_mpk + (size_t)l * 3 * n;
-  int rc = ntt_fwd_shoup_launch(c.ring.args, ahat, a_sh, 3, s);
-  if (rc) return rc;
-  rc = ntt_launch(c.ring.args, e, (long long)l * 3, false, s);
-  if (rc) return rc;
+  int rc = CUFE_OK;
+  if (!forked) rc = ntt_fwd_shoup_launch(c.ring.args, ahat, a_sh, 3, s);
+  if (!rc) rc = ntt_launch(c.ring.args, e, (long long)l * 3, false, s);
+  const int rj = forked ? c.join(s) : (int)CUFE_OK;
+  if (rc || rj) return rc ? rc : rj;
   const long long nres = (long long)l * 3;
   return dispatch_logn(c.ring.logn, [&](auto L) {
     constexpr int LOGN = decltype(L)::value;
@@ -1029,11 +1051,19 @@ int ctx_setup_cpu_map_l(Ctx &c, int l, const uint8_t *seed_a, const uint8_t *see
   if (seed_s) aes_key_expand(seed_s, keys.data() + 60);
   aes_key_expand(seed_e, keys.data() + 120);
   CUFE_CUDA(cudaMemcpyAsync(rk, keys.data(), keys.size() * 4, cudaMemcpyHostToDevice, s));
-  rc = sample_polya(rk, n, d_mpk + (size_t)l * poly, s);
+  // a and its transform on the side stream, behind the candidates and beside the rest (l = 785: 573 and 564 us)
+  rc = c.fork(s);
   if (rc) return rc;
-  rc = sample_cpu_map(0, 2, rk + 60, l, n, d_msk, sws, c.d_status, c.num_sms, s, e);
-  if (rc) return rc;
-  return setup_tail(c, l, d_mpk, d_msk, e, a_sh, s);
+  uint32_t *a = d_mpk + (size_t)l * poly;
+  rc = sample_cpu_map(0, 2, rk + 60, l, n, d_msk, sws, c.d_status, c.num_sms, s, e, kSampleCandidates);
+  if (!rc) rc = sample_polya(rk, n, a, c.side);
+  if (!rc) rc = ntt_fwd_shoup_launch(c.ring.args, a, a_sh, 3, c.side);
+  if (!rc) rc = sample_cpu_map(0, 2, rk + 60, l, n, d_msk, sws, c.d_status, c.num_sms, s, e, kSampleRest);
+  if (rc) {
+    c.join(s);
+    return rc;
+  }
+  return setup_tail(c, l, d_mpk, d_msk, e, a_sh, true, s);
 }
 
 int ctx_setup_gpu_map(Ctx &c, const uint8_t *seed2, const uint8_t *seed3, uint32_t *d_mpk, uint32_t *d_msk,
@@ -1054,7 +1084,7 @@ int ctx_setup_gpu_map(Ctx &c, const uint8_t *seed2, const uint8_t *seed3, uint32
   if (rc) return rc;
   rc = sample_gpu_map(0, rk + 60, 0, l, n, e, c.d_status, c.num_sms, s);
   if (rc) return rc;
-  return setup_tail(c, l, d_mpk, d_msk, e, a_sh, s);
+  return setup_tail(c, l, d_mpk, d_msk, e, a_sh, false, s);
 }
 
 static int encrypt_tail(Ctx &c, int batch, const uint32_t *d_x, const uint32_t *d_mpk, const uint32_t *rhat,
@@ -1117,12 +1147,25 @@ int ctx_encrypt_cpu_map(Ctx &c, int batch, const uint32_t *d_x, const uint32_t *
   std::vector<uint32_t> k2 = expand_keys(batch, seeds2), k3 = expand_keys(batch, seeds3);
   k2.insert(k2.end(), k3.begin(), k3.end());
   CUFE_CUDA(cudaMemcpyAsync(rk, k2.data(), k2.size() * 4, cudaMemcpyHostToDevice, s));
-  rc = sample_cpu_map(1, batch, rk, 2, n, s2o, sws2, c.d_status, c.num_sms, s);
+  // r, f_0 and r's transform (four launches of few CTAs, 31 us at n = 1024 and more above) depend on
+  // nothing that the f_i do: on the side stream.  The f_i's candidates go first, so that r's CTAs take the SMs
+  // that they leave and, in large calls, the time in which one CTA finds the starts of the f_i; in
+  // calls that a pass over fewer SMs serves as fast, the candidates leave r its SMs.  n = 1024, l = 57: 73 us in
+// one stream, 43 in two; n = 4096, l = 784: 514 and 476.
+  const long long ctas2 = ((long long)batch * cpu_map_refills(2, n, 1) + 31) / 32;
+  int sms3 = c.num_sms;
+  if (2 * ctas2 <= sms3 &&
+      (long long)batch * cpu_map_refills(l, n, 2) <= (sms3 - ctas2) * (long long)kCandThreads)
+    sms3 -= (int)ctas2;
+  rc = c.fork(s);
   if (rc) return rc;
-  rc = sample_cpu_map(2, batch, rk + (size_t)batch * 60, l, n, f3, sws3, c.d_status, c.num_sms, s);
-  if (rc) return rc;
-  rc = ntt_fwd_from_launch(c.ring.args, s2o, 2 * poly, rhat, rhat_sh, (long long)batch * 3, s);
-  if (rc) return rc;
+  const uint32_t *rk3 = rk + (size_t)batch * 60;
+  rc = sample_cpu_map(2, batch, rk3, l, n, f3, sws3, c.d_status, sms3, s, nullptr, kSampleCandidates);
+  if (!rc) rc = sample_cpu_map(1, batch, rk, 2, n, s2o, sws2, c.d_status, c.num_sms, c.side);
+  if (!rc) rc = ntt_fwd_from_launch(c.ring.args, s2o, 2 * poly, rhat, rhat_sh, (long long)batch * 3, c.side);
+  if (!rc) rc = sample_cpu_map(2, batch, rk3, l, n, f3, sws3, c.d_status, sms3, s, nullptr, kSampleRest);
+  const int rj = c.join(s);  // also after an error: what was launched uses the workspace
+  if (rc || rj) return rc ? rc : rj;
   return encrypt_tail(c, batch, d_x, d_mpk, rhat, rhat_sh, (long long)poly, f3, (long long)l * poly, s2o + poly,
                       (long long)2 * poly, d_ct, s);
 }

@@ -165,7 +165,7 @@ __constant__ uint8_t c_refill_order[kRefillBlocks] = {17, 12, 13, 14, 8, 9, 10, 
 constexpr uint32_t kEvenWords = 0x01ffu;  // blocks 17, 12, 13, 14, 8..11 and 6
 constexpr uint32_t kOddWords = 0x1e0eu;   // blocks 12, 13, 14 and 2..5
 
-constexpr int kCandThreads = 512;  // 1 CTA (128 KiB of tables) per SM; 128 registers per thread
+// kCandThreads = 512: 1 CTA (192 KiB of tables) per SM; 128 registers per thread
 
 // Word W (0..9) of the branch-free uniform scan (src/gauss.c:578-703): the first 8 accepted
 // words from byte 200 become y[0..7], kept in registers (the same 8 words in a shared-memory
@@ -1195,7 +1195,7 @@ size_t cpu_map_workspace_bytes(uint32_t nstreams, uint32_t calls, uint32_t n, in
 }
 
 int sample_cpu_map_seg(int sig, const SegDev &sg, const SegSizes &z, const uint32_t *d_rkeys, uint32_t *d_out,
-                       void *scratch, uint32_t *d_status, int num_sms, cudaStream_t s) {
+                       void *scratch, uint32_t *d_status, int num_sms, cudaStream_t s, int parts) {
   if (sig < 0 || sig > 2 || z.nstreams == 0 || z.calls >= (1ull << 31) ||
       z.refills >= (1ull << 32) - (1ull << 24))
     return CUFE_ERR_INVALID;
@@ -1212,7 +1212,7 @@ int sample_cpu_map_seg(int sig, const SegDev &sg, const SegSizes &z, const uint3
   const double kinv = kinv_of(sig);
   const uint32_t grid =
       (uint32_t)std::min<uint64_t>((uint64_t)num_sms, (z.refills + 31) / 32);
-  if (grid > 0) {
+  if (grid > 0 && (parts & kSampleCandidates)) {
     ProfScope ps(sig == 0 ? "sample_cand_s1" : (sig == 1 ? "sample_cand_s2" : "sample_cand_s3"), s);
     if (sig == 0)
       note_launch(), k_cand_cpu<0, false, 0><<<grid, kCandThreads, kAesSmemBytes, s>>>(d_rkeys, sg, kinv, cand, amask, chs,
@@ -1225,6 +1225,7 @@ int sample_cpu_map_seg(int sig, const SegDev &sg, const SegSizes &z, const uint3
                                                                              d_status);
   }
   CUFE_CUDA(cudaGetLastError());
+  if (!(parts & kSampleRest)) return CUFE_OK;
   {
     ProfScope ps("sample_walk", s);
     const uint32_t W = end_table_width(z);
@@ -1255,7 +1256,8 @@ int sample_cpu_map_seg(int sig, const SegDev &sg, const SegSizes &z, const uint3
 
 // the uniform case: nstreams equal streams, no tables
 int sample_cpu_map(int sig, uint32_t nstreams, const uint32_t *d_rkeys, uint32_t calls, uint32_t n,
-                   uint32_t *d_out, void *ws, uint32_t *d_status, int num_sms, cudaStream_t s, uint32_t *d_out1) {
+                   uint32_t *d_out, void *ws, uint32_t *d_status, int num_sms, cudaStream_t s, uint32_t *d_out1,
+                   int parts) {
   const SegSizes z = seg_uniform_sizes(nstreams, calls, n, sig);
   if (z.refills / nstreams >= (1ull << 32) / 24) return CUFE_ERR_INVALID;  // AES counter range
   if (d_out1 && nstreams != 2) return CUFE_ERR_INVALID;
@@ -1267,7 +1269,7 @@ int sample_cpu_map(int sig, uint32_t nstreams, const uint32_t *d_rkeys, uint32_t
   sg.u_ostride = (uint64_t)calls * 3 * n;
   if (d_out1)  // two streams: the distance between their outputs, wherever they lie
     sg.u_ostride = (uint64_t)((reinterpret_cast<intptr_t>(d_out1) - reinterpret_cast<intptr_t>(d_out)) / 4);
-  return sample_cpu_map_seg(sig, sg, z, d_rkeys, d_out, ws, d_status, num_sms, s);
+  return sample_cpu_map_seg(sig, sg, z, d_rkeys, d_out, ws, d_status, num_sms, s, parts);
 }
 
 int sample_gpu_map(int sig, const uint32_t *d_rkey, uint32_t poly0, uint32_t npolys, uint32_t n, uint32_t *d_out,

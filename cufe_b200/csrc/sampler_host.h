@@ -19,6 +19,11 @@ int sampler_init_device();
 int expand_keys_device(const uint8_t *d_seeds, const uint32_t *d_perm, uint32_t count, uint32_t *d_rk,
                        cudaStream_t s);
 
+// the parts of a CPU-mapping run, which may be launched by two calls: the candidates (num_sms CTAs
+// at most), and the rest
+enum { kSampleCandidates = 1, kSampleRest = 2, kSampleAll = 3 };
+constexpr int kCandThreads = 512;  // threads of a candidate CTA, one CTA per SM
+
 // CPU stream mapping: nstreams independent AES-CTR streams (round keys d_rkeys[nstreams][60],
 // nonce 0, counter 0), each running `calls` consecutive sampler calls of n samples with
 // sigma index sig; residues written to d_out[nstreams][calls][3][n], those of the second of two to d_out1 where given.
@@ -26,7 +31,7 @@ uint32_t cpu_map_refills(uint32_t calls, uint32_t n, int sig);
 size_t cpu_map_workspace_bytes(uint32_t nstreams, uint32_t calls, uint32_t n, int sig);
 int sample_cpu_map(int sig, uint32_t nstreams, const uint32_t *d_rkeys, uint32_t calls, uint32_t n,
                    uint32_t *d_out, void *ws, uint32_t *d_status, int num_sms, cudaStream_t s,
-                   uint32_t *d_out1 = nullptr);
+                   uint32_t *d_out1 = nullptr, int parts = kSampleAll);
 
 // Segmented form: S CPU-mapping streams of different lengths.  Stream s runs calls[s]
 // sampler calls of n[s] samples; its refills occupy [roff[s], roff[s+1]) of the flattened
@@ -61,7 +66,7 @@ size_t seg_scratch_bytes(const SegSizes &z);
 
 // segmented run: candidates, scan, call starts and the scatter of the residues to d_out
 int sample_cpu_map_seg(int sig, const SegDev &sg, const SegSizes &z, const uint32_t *d_rkeys, uint32_t *d_out,
-                       void *scratch, uint32_t *d_status, int num_sms, cudaStream_t s);
+                       void *scratch, uint32_t *d_status, int num_sms, cudaStream_t s, int parts = kSampleAll);
 
 // GPU counter mapping: polynomials poly0 .. poly0+npolys-1 of one key, residues to
 // d_out[npolys][3][n].
