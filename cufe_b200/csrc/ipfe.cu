@@ -1150,7 +1150,7 @@ int ctx_encrypt_cpu_map(Ctx &c, int batch, const uint32_t *d_x, const uint32_t *
   // r, f_0 and r's transform (four launches of few CTAs, 31 us at n = 1024 and more above) depend on
   // nothing that the f_i do: on the side stream.  The f_i's candidates go first, so that r's CTAs take the SMs
   // that they leave and, in large calls, the time in which one CTA finds the starts of the f_i; in
-  // calls that a pass over fewer SMs serves as fast, the candidates leave r its SMs.  n = 1024, l = 57: 73 us in
+  // calls that a pass over fewer SMs serves as fast, the candidates leave r its SMs.  n = 1024, l = 32: 73 us in
 // one stream, 43 in two; n = 4096, l = 784: 514 and 476.
   const long long ctas2 = ((long long)batch * cpu_map_refills(2, n, 1) + 31) / 32;
   int sms3 = c.num_sms;
