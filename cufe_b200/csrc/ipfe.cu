@@ -297,9 +297,11 @@ inline int device_sms() {
   return sms[dev];
 }
 
-// One grid over the moduli below kSmallQ (lazy butterflies), one over the rest; where all of them are at most
-// a CTA per SM, one grid with the butterflies that serve both, since a launch then takes the latency of
-// one transform whatever is in it (three residues of 1024 with companions: 16.4 us in two launches, now 5).
+// One grid over the moduli below kSmallQ (lazy butterflies), one over the rest; where all CTAs are resident at
+// once (MINB per SM), one grid with the butterflies that serve both, since launches of less than a wave
+// take the latency of their transforms whatever their number.  Three residues of 1024 with companions: 16.4 us in
+// two launches, 5 in one; n = 4096, k = 3, forward, 2 / 3 / 4 CTAs per SM: 17.4 / 22.6 / 22.9 us in two,
+// 10.3 / 12.7 / 16.5 in one, above that 22.8 either way.
 template <int LOGN, int MODE, int PP, int LBT = 512, int MINB = 1, int LE = 4>
 int launch_ntt_pp(const RingArgs &ra, const uint32_t *src, long long src_row, uint32_t *data, uint32_t *sh,
                   long long rows, cudaStream_t s) {
@@ -312,7 +314,7 @@ int launch_ntt_pp(const RingArgs &ra, const uint32_t *src, long long src_row, ui
       large.m[large.nm++] = m;
   }
   ProfScope ps(MODE == 2 ? "ntt_inverse" : "ntt_forward", s);
-  if (small.nm && large.nm && (rows + PP - 1) / PP * ra.k <= (long long)ppc<LOGN, LE>() * device_sms())
+  if (small.nm && large.nm && (rows + PP - 1) / PP * ra.k <= (long long)ppc<LOGN, LE>() * MINB * device_sms())
     return launch_ntt_sel<LOGN, MODE, PP, LBT, MINB, LE, false>(ra, all, src, src_row, data, sh, rows, s);
   int rc = CUFE_OK;
   if (small.nm) rc = launch_ntt_sel<LOGN, MODE, PP, LBT, MINB, LE, true>(ra, small, src, src_row, data, sh, rows, s);

@@ -34,7 +34,8 @@ def test_transforms(n, variant, rng):
     ring.close()
 
 
-@pytest.mark.parametrize("n,rows", [(1024, 394), (1024, 395), (4096, 98), (4096, 99), (8192, 1), (8192, 100)])
+@pytest.mark.parametrize("n,rows", [(1024, 394), (1024, 395), (4096, 98), (4096, 99), (8192, 1), (8192, 100),
+                                    (1024, 1578), (1024, 1579), (4096, 394), (4096, 395), (8192, 196), (8192, 199)])
 def test_one_launch_or_two(n, rows, rng):
     """few transforms go in one launch for all moduli, more in one per class of modulus: the same residues"""
     ring = cf.Ring(n, 3)
