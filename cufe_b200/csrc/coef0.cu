@@ -282,6 +282,12 @@ size_t coef0_mma_bytes(const Ctx &c, int nct, int nkeys) {
   return p.pa + p.pb + p.part;
 }
 
+int coef0_mma_slice(const Ctx &c, int nct, int nkeys, size_t bytes) {
+  int m = nct;
+  while (m > kC0Cts && coef0_mma_bytes(c, m, nkeys) > bytes) m = (m / 2 + kC0Cts - 1) / kC0Cts * kC0Cts;
+  return m;
+}
+
 int coef0_mma_launch(Ctx &c, const SchemeArgs &sa, const DecodeArgs &dd, int nct, const uint32_t *d_ct, int nkeys,
                      const uint32_t *d_y, int y_signed, const uint32_t *d_sky, void *ws, uint32_t *d_out, cudaStream_t s) {
   const Coef0Plan p = plan(c, nct, nkeys);

@@ -43,6 +43,14 @@ struct Ctx {
   uint8_t *ws = nullptr;
   size_t ws_bytes = 0;
   uint32_t *d_status = nullptr;  // sampler status word (device)
+  // scratch of the coefficient-0 decryptions that leave the workspace alone: they may overlap any other call
+  // of the context on another stream, so each waits for the event of the one before
+  uint8_t *own = nullptr;
+  size_t own_bytes = 0;
+  cudaEvent_t own_used = nullptr;
+  // own with `bytes` for work on s, or nullptr (s is being captured, or no memory); own_release after the work
+  uint8_t *own_acquire(size_t bytes, cudaStream_t s);
+  int own_release(cudaStream_t s);
   // a second stream for the part of a call that does not depend on the rest: fork() makes it wait for
   // what is queued on s, join() makes s wait for it
   cudaStream_t side = nullptr;
@@ -114,6 +122,8 @@ void svm_delete(SvmModel *m);
 struct DecodeArgs;
 bool coef0_mma_ok(const Ctx &c);
 size_t coef0_mma_bytes(const Ctx &c, int nct, int nkeys);
+// ciphertexts per launch with at most `bytes` of workspace (whole tiles, one at least)
+int coef0_mma_slice(const Ctx &c, int nct, int nkeys, size_t bytes);
 int coef0_mma_launch(Ctx &c, const SchemeArgs &sa, const DecodeArgs &dd, int nct, const uint32_t *d_ct, int nkeys,
                      const uint32_t *d_y, int y_signed, const uint32_t *d_sky, void *ws, uint32_t *d_out, cudaStream_t s);
 int ctx_decrypt_coef0(Ctx &c, int nct, const uint32_t *d_ct, int nkeys, const uint32_t *d_y, int y_signed,

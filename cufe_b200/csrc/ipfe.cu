@@ -899,6 +899,11 @@ int Ctx::init(int n_, int l_, int dev) {
 
 void Ctx::release() {
   if (ws) cudaFree(ws);
+  if (own) cudaFree(own);
+  if (own_used) cudaEventDestroy(own_used);
+  own = nullptr;
+  own_bytes = 0;
+  own_used = nullptr;
   if (d_status) cudaFree(d_status);
   if (stream) cudaStreamDestroy(stream);
   if (side) cudaStreamDestroy(side);
@@ -937,6 +942,36 @@ int Ctx::ensure_ws(size_t bytes) {
     return CUFE_ERR_NOMEM;
   }
   ws_bytes = want;
+  return CUFE_OK;
+}
+
+uint8_t *Ctx::own_acquire(size_t bytes, cudaStream_t s) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  // an allocation here is of no concern to a capture that is open on another stream
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  bool ok = cudaThreadExchangeStreamCaptureMode(&mode) == cudaSuccess;
+  if (ok && !own_used) ok = cudaEventCreateWithFlags(&own_used, cudaEventDisableTiming) == cudaSuccess;
+  if (ok && bytes > own_bytes) {
+    ok = cudaEventSynchronize(own_used) == cudaSuccess;
+    if (own) cudaFree(own);
+    own = nullptr;
+    own_bytes = 0;
+    const size_t want = bytes + (bytes >> 3);
+    ok = ok && cudaMalloc(&own, want) == cudaSuccess;
+    if (ok) own_bytes = want;
+  }
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (ok) ok = cudaStreamWaitEvent(s, own_used, 0) == cudaSuccess;
+  if (!ok) cudaGetLastError();
+  return ok ? own : nullptr;
+}
+
+int Ctx::own_release(cudaStream_t s) {
+  CUFE_CUDA(cudaEventRecord(own_used, s));
   return CUFE_OK;
 }
 
@@ -1512,9 +1547,30 @@ int ctx_decrypt_coef0(Ctx &c, int nct, const uint32_t *d_ct, int nkeys, const ui
     CUFE_CUDA(cudaGetLastError());
     return CUFE_OK;
   }
-  int form = mma ? (pairs >= 1024 ? 1 : 0) : (nkeys >= kCoef0TiledMinKeys ? 1 : 0);
-  if (it != c.coef0_form.end()) form = it->second;
-  return ctx_decrypt_coef0_form(c, form, nct, d_ct, nkeys, d_y, y_signed, d_sky, d_d0, d_out, s);
+  if (it == c.coef0_form.end() && nct >= 1 && nkeys >= 1 && nkeys < kCoef0TiledMinKeys) {
+    // few keys use no workspace, so that they may overlap the context's other calls and be captured whatever
+    // its size: the tensor-core product has a scratch of its own, at most 256 MiB by slices of the
+    // ciphertexts, and where that cannot be had it is form 0
+    constexpr size_t kOwnBytes = (size_t)256 << 20;
+    const int step = mma && pairs >= 1024 ? coef0_mma_slice(c, nct, nkeys, kOwnBytes) : 0;
+    uint8_t *w = nullptr;
+    if (step && pairs <= 0x7fffffffLL) {
+      size_t bytes = coef0_mma_bytes(c, step, nkeys);
+      if (nct % step) bytes = std::max(bytes, coef0_mma_bytes(c, nct % step, nkeys));  // may have more splits
+      w = c.own_acquire(bytes, s);
+    }
+    if (!w) return ctx_decrypt_coef0_form(c, 0, nct, d_ct, nkeys, d_y, y_signed, d_sky, d_d0, d_out, s);
+    ProfScope ps("decrypt_coef0", s);
+    int rc = CUFE_OK;
+    for (int at = 0; at < nct && rc == CUFE_OK; at += step)
+      rc = coef0_mma_launch(c, scheme_args(c), decode_args(c), std::min(step, nct - at),
+                            d_ct + (size_t)at * (c.l + 1) * 3 * c.n, nkeys, d_y, y_signed, d_sky, w,
+                            d_out + (size_t)at * nkeys, s);
+    const int rr = c.own_release(s);  // also after an error: what was launched uses the scratch
+    return rc ? rc : rr;
+  }
+  return ctx_decrypt_coef0_form(c, it == c.coef0_form.end() ? 1 : it->second, nct, d_ct, nkeys, d_y, y_signed, d_sky, d_d0,
+                                d_out, s);
 }
 
 int ctx_sample_cpu_map(Ctx &c, int sig, int nstreams, const uint8_t *keys, int calls, uint32_t *d_out,

@@ -145,7 +145,10 @@ int cufe_decode(cufe_ctx *ctx, int count, const uint32_t *d_dy, int ncoeff, uint
  * d_out[nct][nkeys] = decode of d_y[0], where d_y[0] = sum_i y_i c_i[0] - (c_l * sk_y)[0] with
  * the negacyclic constant term (c_l * sk_y)[0] = c_l[0] sk_y[0] - sum_{t>=1} c_l[t] sk_y[n-t].
  * Equal to cufe_decode(cufe_decrypt(...), ncoeff = 1).  d_d0 (optional, may be NULL) receives
- * the residues d_d0[nct][nkeys][3]. */
+ * the residues d_d0[nct][nkeys][3].  With d_d0, or (untuned) with fewer than 32 keys, the call leaves the
+ * context's workspace alone: it may overlap the context's other calls on other streams and be captured
+ * whatever was called before.  Many pairs of few keys then take a scratch of their own, at most 288 MiB,
+ * which the context keeps. */
 int cufe_decrypt_coef0(cufe_ctx *ctx, int nct, const uint32_t *d_ct, int nkeys, const uint32_t *d_y, int y_signed,
                        const uint32_t *d_sky, uint32_t *d_d0, uint32_t *d_out, void *stream);
 
