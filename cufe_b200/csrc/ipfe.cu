@@ -596,12 +596,12 @@ __global__ void __launch_bounds__(NttPlan<LOGN>::T * ppc<LOGN>(), NttPlan<LOGN>:
 }
 
 // Decryption (src/rlwe_sife.c:248-278), d_y = sum_i y_i c_i - INTT(NTT(c_l) NTT(sk_y)): the
-// l-sums come from mac_launch; k_dec_tail subtracts the negacyclic product c_l * sk_y from them,
-// in place.
+// l-sums come from mac_launch; k_dec_tail subtracts the negacyclic product c_l * sk_y from them
+// (sums may be dy).
 template <int LOGN>
 __global__ void __launch_bounds__(512)
     k_dec_tail(const uint32_t *__restrict__ clhat, const uint32_t *__restrict__ skhat,
-               const uint32_t *__restrict__ skhat_sh, int nkeys, uint32_t *__restrict__ dy, long long nwork,
+               const uint32_t *__restrict__ skhat_sh, int nkeys, const uint32_t *sums, uint32_t *dy, long long nwork,
                SchemeArgs sa) {
   using P = NttPlan<LOGN>;
   extern __shared__ uint32_t smem_u32[];
@@ -623,12 +623,15 @@ __global__ void __launch_bounds__(512)
   ntt_inv_core<LOGN>(a, sm, th, q, sa.ra.ipsi2 + (size_t)m * P::N, sa.ra.ninv[m],
                      sa.ra.ninv_sh[m], sa.ra.w1n[m], sa.ra.w1n_sh[m]);
   if (act) {
+    const uint32_t *t = sums + ww * P::N;
     uint32_t *o = dy + ww * P::N;
 #pragma unroll
     for (int e = 0; e < 16; ++e) {
       const int j = P::template idx<0>(th, e);
-      o[j] = mod_sub(o[j], a[e], q);
+      a[e] = mod_sub(t[j], a[e], q);
     }
+#pragma unroll
+    for (int e = 0; e < 16; ++e) o[P::template idx<0>(th, e)] = a[e];
   }
 }
 
@@ -1263,11 +1266,20 @@ static bool decrypt_length_ok(const Ctx &c, long long nwork, int max_split) {
   return (c.l + nsplit - 1) / nsplit + 1 <= 25600;
 }
 
+// Whether the l-sums may not go straight to d_dy: they are written while d_ct and d_y are read, which
+// callers may let d_dy overlap (only the ciphertexts' and keys' transforms are taken before)
+static bool decrypt_overlaps(const Ctx &c, int nct, const uint32_t *d_ct, int nkeys, const uint32_t *d_y,
+                             const uint32_t *d_dy) {
+  const size_t poly = (size_t)3 * c.n;
+  const uint32_t *end = d_dy + (size_t)nct * nkeys * poly;
+  return (d_dy < d_ct + (size_t)nct * (c.l + 1) * poly && d_ct < end) || (d_dy < d_y + (size_t)nkeys * c.l && d_y < end);
+}
+
 // the decryption of nct ciphertexts under nkeys keys with its scratch: clhat [nct][3][n], skhat
-// and skhat_sh [nkeys][3][n]
+// and skhat_sh [nkeys][3][n], sums [nct][nkeys][3][n] (d_dy, or apart from it)
 static int decrypt_with(Ctx &c, int nct, const uint32_t *d_ct, int nkeys, const uint32_t *d_y, int y_signed,
                         const uint32_t *d_sky, uint32_t *d_dy, uint32_t *clhat, uint32_t *skhat, uint32_t *skhat_sh,
-                        cudaStream_t s) {
+                        uint32_t *sums, cudaStream_t s) {
   const size_t poly = (size_t)3 * c.n, ct_words = (size_t)(c.l + 1) * poly;
   const long long nwork = (long long)nct * nkeys * 3;
   const SchemeArgs sa = scheme_args(c);
@@ -1277,7 +1289,7 @@ static int decrypt_with(Ctx &c, int nct, const uint32_t *d_ct, int nkeys, const 
   if (rc) return rc;
   {
     ProfScope ps("decrypt_mac", s);
-    rc = mac_launch(c, sa, d_ct, ct_words, nct, d_y, y_signed, nkeys, d_dy, s);
+    rc = mac_launch(c, sa, d_ct, ct_words, nct, d_y, y_signed, nkeys, sums, s);
     if (rc) return rc;
   }
   return dispatch_logn(c.ring.logn, [&](auto L) {
@@ -1287,7 +1299,7 @@ static int decrypt_with(Ctx &c, int nct, const uint32_t *d_ct, int nkeys, const 
     CUFE_CUDA(cudaFuncSetAttribute(k_dec_tail<LOGN>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
     ProfScope ps("decrypt_tail", s);
     note_launch(), k_dec_tail<LOGN><<<(unsigned)((nwork + G - 1) / G), dim3(NttPlan<LOGN>::T, G), smem, s>>>(
-        clhat, skhat, skhat_sh, nkeys, d_dy, nwork, sa);
+        clhat, skhat, skhat_sh, nkeys, sums, d_dy, nwork, sa);
     CUFE_CUDA(cudaGetLastError());
     return (int)CUFE_OK;
   });
@@ -1298,13 +1310,15 @@ int ctx_decrypt(Ctx &c, int nct, const uint32_t *d_ct, int nkeys, const uint32_t
   if (nct < 1 || nkeys < 1) return CUFE_ERR_INVALID;
   if (!decrypt_length_ok(c, (long long)nct * nkeys * 3, 32)) return CUFE_ERR_INVALID;
   const size_t poly = (size_t)3 * c.n;
-  int rc = c.ensure_ws(((size_t)nct * poly + 2 * (size_t)nkeys * poly) * 4 + 8 * 256);
+  const size_t sums_words = decrypt_overlaps(c, nct, d_ct, nkeys, d_y, d_dy) ? (size_t)nct * nkeys * poly : 0;
+  int rc = c.ensure_ws(((size_t)nct * poly + 2 * (size_t)nkeys * poly + sums_words) * 4 + 8 * 256);
   if (rc) return rc;
   Arena ar(c.ws);
   uint32_t *clhat = ar.take<uint32_t>((size_t)nct * poly);
   uint32_t *skhat = ar.take<uint32_t>((size_t)nkeys * poly);
   uint32_t *skhat_sh = ar.take<uint32_t>((size_t)nkeys * poly);
-  return decrypt_with(c, nct, d_ct, nkeys, d_y, y_signed, d_sky, d_dy, clhat, skhat, skhat_sh, s);
+  uint32_t *sums = sums_words ? ar.take<uint32_t>(sums_words) : d_dy;
+  return decrypt_with(c, nct, d_ct, nkeys, d_y, y_signed, d_sky, d_dy, clhat, skhat, skhat_sh, sums, s);
 }
 
 // ------------------------------------------------------------------ decryption without allocation
@@ -1315,12 +1329,13 @@ int ctx_decrypt(Ctx &c, int nct, const uint32_t *d_ct, int nkeys, const uint32_t
 // ctx_decrypt_noalloc runs the same decryption kernels as ctx_decrypt with every scratch
 // buffer carved from the file-scope array below instead of the context workspace.  The
 // array is a fixed part of the library image: every GPU that loads the library holds its
-// 432 KiB until the process exits.
+// 625 KiB until the process exits.
 constexpr int kNoAllocMaxN = 4096;    // ring degree
 constexpr int kNoAllocMaxKeys = 4;    // keys per call (one ciphertext per call)
 constexpr int kNoAllocMaxSplit = 8;   // chunks of the l-sum that bound its length
 constexpr size_t kNoAllocWords = (size_t)3 * kNoAllocMaxN                       // NTT(c_l)
                                  + (size_t)2 * kNoAllocMaxKeys * 3 * kNoAllocMaxN  // NTT(sk_y), Shoup
+                                 + (size_t)kNoAllocMaxKeys * 3 * kNoAllocMaxN      // l-sums, where d_dy cannot take them
                                  + 4 * 64;                                          // region padding
 static __device__ __align__(256) uint32_t g_noalloc_scratch[kNoAllocWords];
 
@@ -1365,8 +1380,9 @@ int ctx_decrypt_noalloc(Ctx &c, const uint32_t *d_ct, int nkeys, const uint32_t 
   uint32_t *clhat = base;
   uint32_t *skhat = clhat + round64(poly);
   uint32_t *skhat_sh = skhat + round64((size_t)nkeys * poly);
+  uint32_t *sums = decrypt_overlaps(c, 1, d_ct, nkeys, d_y, d_dy) ? skhat_sh + round64((size_t)nkeys * poly) : d_dy;
   // every scratch word read is written first by this call (no zeroing needed)
-  return decrypt_with(c, 1, d_ct, nkeys, d_y, y_signed, d_sky, d_dy, clhat, skhat, skhat_sh, s);
+  return decrypt_with(c, 1, d_ct, nkeys, d_y, y_signed, d_sky, d_dy, clhat, skhat, skhat_sh, sums, s);
 }
 
 static DecodeArgs decode_args(const Ctx &c) {

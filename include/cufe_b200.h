@@ -122,7 +122,8 @@ int cufe_encrypt_gpu_map(cufe_ctx *ctx, int batch, const uint32_t *d_x, const ui
 int cufe_keygen(cufe_ctx *ctx, int nkeys, const uint32_t *d_y, int y_signed, const uint32_t *d_msk,
                 uint32_t *d_sky, void *stream);
 /* d_y = sum_i y_i c_i - c_l * sk_y (rlwe_sife_decrypt_gmp before the CRT,
- * src/rlwe_sife.c:248-278) for every (ciphertext, key) pair: d_dy[nct][nkeys][3][n] */
+ * src/rlwe_sife.c:248-278) for every (ciphertext, key) pair: d_dy[nct][nkeys][3][n], which may overlap
+ * the inputs (the l-sums then take scratch of its size) */
 int cufe_decrypt(cufe_ctx *ctx, int nct, const uint32_t *d_ct, int nkeys, const uint32_t *d_y, int y_signed,
                  const uint32_t *d_sky, uint32_t *d_dy, void *stream);
 /* Decryption that allocates no device memory, for callers that cannot call cudaMalloc
@@ -130,7 +131,7 @@ int cufe_decrypt(cufe_ctx *ctx, int nct, const uint32_t *d_ct, int nkeys, const 
  * that must not take cudaMalloc's implicit device synchronisation).  No counterpart in the
  * reference.  Same result as cufe_decrypt for one ciphertext d_ct[l+1][3][n] and nkeys
  * keys: d_dy[nkeys][3][n].  Limits: n <= 4096 and 1 <= nkeys <= 4, else CUFE_ERR_INVALID.
- * Its scratch is a fixed array of 432 KiB inside the library image, held on every GPU
+ * Its scratch is a fixed array of 625 KiB inside the library image, held on every GPU
  * that loads the library until the process exits.  The first call on a device looks up the
  * array's device address (make that first call before any stream capture).  All calls share
  * the array: calls that overlap on the GPU (different streams, threads or contexts without
