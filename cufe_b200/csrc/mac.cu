@@ -512,7 +512,9 @@ int mac_launch(Ctx &c, const SchemeArgs &sa, const uint32_t *d_v, size_t vstride
     const long long tiles = (long long)nz * (3 * n / kMmaCols);
     const long long per_key_tile = std::max(1LL, std::min(tiles, (long long)c.num_sms / a.key_tiles));
     const uint32_t smem = mma_smem(l);
-    CUFE_CUDA(cudaFuncSetAttribute(k_mac_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // the limit of the longest l whatever this one: the attribute is the kernel's, and another context's thread may
+    // set it between here and the launch
+    CUFE_CUDA(cudaFuncSetAttribute(k_mac_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mma_smem(kMmaMaxL)));
     note_launch(), k_mac_mma<<<(unsigned)(per_key_tile * a.key_tiles), kMmaThreads, smem, s>>>(a, sa, c.d_status);
     CUFE_CUDA(cudaGetLastError());
     return CUFE_OK;
