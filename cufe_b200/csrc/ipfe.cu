@@ -1240,8 +1240,11 @@ int ctx_encrypt_gpu_map(Ctx &c, int batch, const uint32_t *d_x, const uint32_t *
     constexpr int G = ppc<LOGN>();
     ProfScope ps("encrypt_intt", s);
     const unsigned ctas = (unsigned)((3 * (l + 1) + G - 1) / G);
-    // shares of the instances: enough CTAs for four per SM
-    const unsigned shares = std::max(1u, std::min((unsigned)batch, ((unsigned)c.num_sms * 4 + ctas - 1) / ctas));
+    // shares of the instances: enough CTAs for four per SM; one where ciphertexts lie over the public key,
+    // whose residue a share would read when another has written it
+    const size_t key_words = (size_t)(l + 1) * poly;
+    const bool over = d_ct < d_mpk + key_words && d_mpk < d_ct + (size_t)batch * key_words;
+    const unsigned shares = over ? 1u : std::max(1u, std::min((unsigned)batch, ((unsigned)c.num_sms * 4 + ctas - 1) / ctas));
     CUFE_CUDA(cudaFuncSetAttribute(k_encrypt_shared<LOGN>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
     note_launch(), k_encrypt_shared<LOGN><<<dim3(ctas, shares), dim3(NttPlan<LOGN>::T, G), G * NttPlan<LOGN>::SMEM_WORDS * 4, s>>>(
         d_mpk, rhat, rhat_sh, f3, r, d_x, d_ct, batch, sa);
