@@ -52,11 +52,12 @@ struct Ctx {
   uint8_t *own_acquire(size_t bytes, cudaStream_t s);
   int own_release(cudaStream_t s);
   // a second stream for the part of a call that does not depend on the rest: fork() makes it wait for
-  // what is queued on s, join() makes s wait for it
+  // what is queued on s and gives it, join() makes s wait for it.  While it belongs to a capture that s does
+  // not (an encryption or setup captured on another stream, the capture still open) fork() gives s itself.
   cudaStream_t side = nullptr;
   cudaEvent_t forked = nullptr, joined = nullptr;
-  int fork(cudaStream_t s);
-  int join(cudaStream_t s);
+  int fork(cudaStream_t s, cudaStream_t *second);
+  int join(cudaStream_t s, cudaStream_t second);
   std::mutex mu;                 // serialises host calls on this context
   Prof prof;                     // per-kernel timing (cufe_profile_*)
   // shapes chosen by the tuners (cufe_tune_*): encryption instances per thread group by batch

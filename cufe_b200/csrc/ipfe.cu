@@ -920,14 +920,25 @@ void Ctx::release() {
   stream = nullptr;
 }
 
-int Ctx::fork(cudaStream_t s) {
+int Ctx::fork(cudaStream_t s, cudaStream_t *second) {
+  *second = s;
+  cudaStreamCaptureStatus mine = cudaStreamCaptureStatusNone, theirs = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0, id_s = 0;
+  CUFE_CUDA(cudaStreamGetCaptureInfo(side, &mine, &id));
+  if (mine != cudaStreamCaptureStatusNone &&
+      (cudaStreamGetCaptureInfo(s, &theirs, &id_s) != cudaSuccess || theirs == cudaStreamCaptureStatusNone || id != id_s)) {
+    cudaGetLastError();
+    return CUFE_OK;
+  }
   CUFE_CUDA(cudaEventRecord(forked, s));
   CUFE_CUDA(cudaStreamWaitEvent(side, forked, 0));
+  *second = side;
   return CUFE_OK;
 }
 
-int Ctx::join(cudaStream_t s) {
-  CUFE_CUDA(cudaEventRecord(joined, side));
+int Ctx::join(cudaStream_t s, cudaStream_t second) {
+  if (second == s) return CUFE_OK;
+  CUFE_CUDA(cudaEventRecord(joined, second));
   CUFE_CUDA(cudaStreamWaitEvent(s, joined, 0));
   return CUFE_OK;
 }
@@ -1044,16 +1055,16 @@ static int dispatch_logn(int logn, F &&f) {
   return CUFE_ERR_INVALID;
 }
 
-// shared tail of both setups: a^ = NTT(a) in place (already on the side stream if forked), e^ = NTT(e),
+// shared tail of both setups: a^ = NTT(a) in place (unless a_done, on `second`), e^ = NTT(e),
 // mpk_i = a^ NTT(s_i) + e^_i
-static int setup_tail(Ctx &c, int l, uint32_t *d_mpk, const uint32_t *d_msk, uint32_t *e, uint32_t *a_sh, bool forked,
-                      cudaStream_t s) {
+static int setup_tail(Ctx &c, int l, uint32_t *d_mpk, const uint32_t *d_msk, uint32_t *e, uint32_t *a_sh, bool a_done,
+                      cudaStream_t second, cudaStream_t s) {
   const int n = c.n;
   uint32_t *ahat = d_mpk + (size_t)l * 3 * n;
   int rc = CUFE_OK;
-  if (!forked) rc = ntt_fwd_shoup_launch(c.ring.args, ahat, a_sh, 3, s);
+  if (!a_done) rc = ntt_fwd_shoup_launch(c.ring.args, ahat, a_sh, 3, s);
   if (!rc) rc = ntt_launch(c.ring.args, e, (long long)l * 3, false, s);
-  const int rj = forked ? c.join(s) : (int)CUFE_OK;
+  const int rj = c.join(s, second);
   if (rc || rj) return rc ? rc : rj;
   const long long nres = (long long)l * 3;
   return dispatch_logn(c.ring.logn, [&](auto L) {
@@ -1092,18 +1103,19 @@ int ctx_setup_cpu_map_l(Ctx &c, int l, const uint8_t *seed_a, const uint8_t *see
   aes_key_expand(seed_e, keys.data() + 120);
   CUFE_CUDA(cudaMemcpyAsync(rk, keys.data(), keys.size() * 4, cudaMemcpyHostToDevice, s));
   // a and its transform on the side stream, behind the candidates and beside the rest (l = 785: 573 and 564 us)
-  rc = c.fork(s);
+  cudaStream_t second;
+  rc = c.fork(s, &second);
   if (rc) return rc;
   uint32_t *a = d_mpk + (size_t)l * poly;
   rc = sample_cpu_map(0, 2, rk + 60, l, n, d_msk, sws, c.d_status, c.num_sms, s, e, kSampleCandidates);
-  if (!rc) rc = sample_polya(rk, n, a, c.side);
-  if (!rc) rc = ntt_fwd_shoup_launch(c.ring.args, a, a_sh, 3, c.side);
+  if (!rc) rc = sample_polya(rk, n, a, second);
+  if (!rc) rc = ntt_fwd_shoup_launch(c.ring.args, a, a_sh, 3, second);
   if (!rc) rc = sample_cpu_map(0, 2, rk + 60, l, n, d_msk, sws, c.d_status, c.num_sms, s, e, kSampleRest);
   if (rc) {
-    c.join(s);
+    c.join(s, second);
     return rc;
   }
-  return setup_tail(c, l, d_mpk, d_msk, e, a_sh, true, s);
+  return setup_tail(c, l, d_mpk, d_msk, e, a_sh, true, second, s);
 }
 
 int ctx_setup_gpu_map(Ctx &c, const uint8_t *seed2, const uint8_t *seed3, uint32_t *d_mpk, uint32_t *d_msk,
@@ -1124,7 +1136,7 @@ int ctx_setup_gpu_map(Ctx &c, const uint8_t *seed2, const uint8_t *seed3, uint32
   if (rc) return rc;
   rc = sample_gpu_map(0, rk + 60, 0, l, n, e, c.d_status, c.num_sms, s);
   if (rc) return rc;
-  return setup_tail(c, l, d_mpk, d_msk, e, a_sh, false, s);
+  return setup_tail(c, l, d_mpk, d_msk, e, a_sh, false, s, s);
 }
 
 static int encrypt_tail(Ctx &c, int batch, const uint32_t *d_x, const uint32_t *d_mpk, const uint32_t *rhat,
@@ -1197,14 +1209,15 @@ int ctx_encrypt_cpu_map(Ctx &c, int batch, const uint32_t *d_x, const uint32_t *
   if (2 * ctas2 <= sms3 &&
       (long long)batch * cpu_map_refills(l, n, 2) <= (sms3 - ctas2) * (long long)kCandThreads)
     sms3 -= (int)ctas2;
-  rc = c.fork(s);
+  cudaStream_t second;
+  rc = c.fork(s, &second);
   if (rc) return rc;
   const uint32_t *rk3 = rk + (size_t)batch * 60;
   rc = sample_cpu_map(2, batch, rk3, l, n, f3, sws3, c.d_status, sms3, s, nullptr, kSampleCandidates);
-  if (!rc) rc = sample_cpu_map(1, batch, rk, 2, n, s2o, sws2, c.d_status, c.num_sms, c.side);
-  if (!rc) rc = ntt_fwd_from_launch(c.ring.args, s2o, 2 * poly, rhat, rhat_sh, (long long)batch * 3, c.side);
+  if (!rc) rc = sample_cpu_map(1, batch, rk, 2, n, s2o, sws2, c.d_status, c.num_sms, second);
+  if (!rc) rc = ntt_fwd_from_launch(c.ring.args, s2o, 2 * poly, rhat, rhat_sh, (long long)batch * 3, second);
   if (!rc) rc = sample_cpu_map(2, batch, rk3, l, n, f3, sws3, c.d_status, sms3, s, nullptr, kSampleRest);
-  const int rj = c.join(s);  // also after an error: what was launched uses the workspace
+  const int rj = c.join(s, second);  // also after an error: what was launched uses the workspace
   if (rc || rj) return rc ? rc : rj;
   return encrypt_tail(c, batch, d_x, d_mpk, rhat, rhat_sh, (long long)poly, f3, (long long)l * poly, s2o + poly,
                       (long long)2 * poly, d_ct, s);
