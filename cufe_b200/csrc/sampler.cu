@@ -1139,6 +1139,18 @@ SegDev seg_bind(void *base, uint32_t S) {
   return d;
 }
 
+// Width of the table of call ends, 0: k_walk.  The overshoot of a call has a standard deviation
+// below 2, so that of c calls one below 2 sqrt(c): the window takes 4 of those and 64 to either side.  The
+// windows may be n - 192 wide, so that a threshold is in one of them, and the nearest call to
+// any of a thread's 128 thresholds is the one whose window it is in (k_ends).  From 128 calls on the
+// three launches are shorter than the walk (sigma_2, n = 4096, one stream / 16, us against the
+// walk's: 64 calls 22 / 25 against 19 / 19, 128 27 / 32 against 31 / 31, 256 35 / 51 against 56 / 57, 785
+// 72 / 114 against 158 / 158).
+static uint32_t end_table_width(const SegSizes &z) {
+  const uint32_t W = ((uint32_t)(16.0 * std::sqrt((double)z.max_calls)) + 128 + 63) & ~63u;
+  return z.max_calls >= 128 && W + 192 <= z.min_n && z.max_refills < (1u << 28) && z.nstreams < 65536u ? W : 0u;
+}
+
 SegSizes seg_fill_host(int sig, uint32_t S, const uint32_t *calls, const uint32_t *n, const uint64_t *ooff,
                        void *host_base) {
   const SegLayout L = seg_layout(S);
@@ -1146,7 +1158,7 @@ SegSizes seg_fill_host(int sig, uint32_t S, const uint32_t *calls, const uint32_
   uint32_t *hn = reinterpret_cast<uint32_t *>(b + L.n), *hc = reinterpret_cast<uint32_t *>(b + L.calls);
   uint64_t *hr = reinterpret_cast<uint64_t *>(b + L.roff), *hco = reinterpret_cast<uint64_t *>(b + L.coff);
   uint64_t *ho = reinterpret_cast<uint64_t *>(b + L.ooff);
-  SegSizes z{S, 0, 0, 0, 0, 0xffffffffu};
+  SegSizes z{S, 0, 0, 0, 0, 0xffffffffu, 0};
   for (uint32_t i = 0; i < S; ++i) {
     const uint32_t R = cpu_map_refills(calls[i], n[i], sig);
     hn[i] = n[i];
@@ -1162,32 +1174,23 @@ SegSizes seg_fill_host(int sig, uint32_t S, const uint32_t *calls, const uint32_
   }
   hr[S] = z.refills;
   hco[S] = z.calls;
+  z.end_w = end_table_width(z);
   return z;
 }
 
 static SegSizes seg_uniform_sizes(uint32_t S, uint32_t calls, uint32_t n, int sig) {
   const uint32_t R = cpu_map_refills(calls, n, sig);
-  return SegSizes{S, (uint64_t)S * R, (uint64_t)S * calls, R, calls, n};
-}
-
-// Width of the table of call ends, 0: k_walk.  The overshoot of a call has a standard deviation
-// below 2, so that of c calls one below 2 sqrt(c): the window takes 4 of those and 64 to either side.  The
-// windows may be n - 192 wide, so that a threshold is in one of them, and the nearest call to
-// any of a thread's 128 thresholds is the one whose window it is in (k_ends).  From 128 calls on the
-// three launches are shorter than the walk (sigma_2, n = 4096, one stream / 16, us against the
-// walk's: 64 calls 22 / 25 against 19 / 19, 128 27 / 32 against 31 / 31, 256 35 / 51 against 56 / 57, 785
-// 72 / 114 against 158 / 158).
-static uint32_t end_table_width(const SegSizes &z) {
-  const uint32_t W = ((uint32_t)(16.0 * std::sqrt((double)z.max_calls)) + 128 + 63) & ~63u;
-  return z.max_calls >= 128 && W + 192 <= z.min_n && z.max_refills < (1u << 28) && z.nstreams < 65536u ? W : 0u;
+  SegSizes z{S, (uint64_t)S * R, (uint64_t)S * calls, R, calls, n, 0};
+  z.end_w = end_table_width(z);
+  return z;
 }
 
 static uint32_t count_tiles(const SegSizes &z) { return (z.max_refills + kCountTile - 1) / kCountTile; }
 
 size_t seg_scratch_bytes(const SegSizes &z) {
   return align256(z.refills * 32) + align256(z.refills) + align256(z.refills * 2) +
-         align256((z.calls + z.nstreams) * 4) + align256((size_t)z.calls * end_table_width(z) * 4) +
-         align256((size_t)z.nstreams * count_tiles(z) * 4);
+         align256((z.calls + z.nstreams) * 4) +
+         (z.end_w ? align256((size_t)z.calls * z.end_w * 4) + align256((size_t)z.nstreams * count_tiles(z) * 4) : 0);
 }
 
 size_t cpu_map_workspace_bytes(uint32_t nstreams, uint32_t calls, uint32_t n, int sig) {
@@ -1228,13 +1231,12 @@ int sample_cpu_map_seg(int sig, const SegDev &sg, const SegSizes &z, const uint3
   if (!(parts & kSampleRest)) return CUFE_OK;
   {
     ProfScope ps("sample_walk", s);
-    const uint32_t W = end_table_width(z);
-    if (W) {
+    if (z.end_w) {
       EndTable t;
-      t.ends = reinterpret_cast<uint32_t *>(take((size_t)z.calls * W * 4));
+      t.ends = reinterpret_cast<uint32_t *>(take((size_t)z.calls * z.end_w * 4));
       t.max_tiles = count_tiles(z);
       t.counts = reinterpret_cast<uint32_t *>(take((size_t)z.nstreams * t.max_tiles * 4));
-      t.W = W;
+      t.W = z.end_w;
       t.mean = mean_overshoot(sig);
       const dim3 grid(t.max_tiles, z.nstreams);
       note_launch(), k_tile_counts<<<grid, 256, 0, s>>>(amask, sg, t);

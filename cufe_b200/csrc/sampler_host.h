@@ -51,6 +51,7 @@ struct SegSizes {
   uint64_t refills;
   uint64_t calls;
   uint32_t max_refills, max_calls, min_n;  // over the streams
+  uint32_t end_w;  // words per call of the table of call ends; 0 (also set by callers without room): the walk
 };
 struct SegLayout {
   size_t n, calls, roff, coff, ooff, bytes;
