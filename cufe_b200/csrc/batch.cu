@@ -856,8 +856,8 @@ struct Server {
     const uint64_t poly = (uint64_t)3 * n * 4;
     const uint64_t R3 = cpu_map_refills(l, n, 2), R2 = cpu_map_refills(2, n, 1);
     // sampler scratch: 35 B per refill (candidate low words 32, accept mask 1, bit-32 and sign
-    // bytes 2) plus call starts; admission charges 44, and a tick whose table of call ends does not fit into
-    // what is left walks (launch)
+    // bytes 2) plus call starts; admission charges 44, and a tick whose tables for the call starts do not fit
+    // into what is left walks (launch)
     return poly * (2 + 2 + l) + std::max(R3, R2) * 44 + 2 * 60 * 4 + 8192;
   }
 
@@ -1111,7 +1111,7 @@ struct Server {
       uint32_t *f3 = reinterpret_cast<uint32_t *>(take(w_f3 * 4));
       uint32_t *rk = reinterpret_cast<uint32_t *>(take((size_t)2 * ne * 60 * 4));
       if ((size_t)(p - d_scr) + std::max(seg_scratch_bytes(z2), seg_scratch_bytes(z3)) > scr_bytes)
-        z2.end_w = z3.end_w = 0;
+        seg_search(z2, kSearchWalk), seg_search(z3, kSearchWalk);
       void *samp = take(std::max(seg_scratch_bytes(z2), seg_scratch_bytes(z3)));
       if ((size_t)(p - d_scr) > scr_bytes) {
         set_last_error("server: tick scratch exceeded");

@@ -344,7 +344,9 @@ int cufe_deserialize(cufe_ctx *h, int kind, int count, const uint8_t *d_src, siz
 }
 
 int cufe_sampler_call_search(int mode) {
-  return mode < 0 || mode > 2 ? CUFE_ERR_INVALID : CUFE_OK;  // no choice left to make
+  if (mode < 0 || mode > 2) return CUFE_ERR_INVALID;
+  cufe::set_call_search(mode);
+  return CUFE_OK;
 }
 
 // ------------------------------------------------------------------ encrypted SVM prediction

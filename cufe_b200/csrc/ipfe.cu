@@ -1089,7 +1089,8 @@ int ctx_setup_cpu_map_l(Ctx &c, int l, const uint8_t *seed_a, const uint8_t *see
   if (l < 1 || !seed_a || !seed_e) return CUFE_ERR_INVALID;
   const int n = c.n;
   const size_t poly = (size_t)3 * n;
-  const size_t samp_ws = cpu_map_workspace_bytes(2, l, n, 0);
+  const SegSizes z = cpu_map_sizes(2, l, n, 0);
+  const size_t samp_ws = seg_scratch_bytes(z);
   int rc = c.ensure_ws(samp_ws + (l + 2) * poly * 4 + 4096 + 4 * 60 * 4);
   if (rc) return rc;
   Arena ar(c.ws);
@@ -1107,10 +1108,10 @@ int ctx_setup_cpu_map_l(Ctx &c, int l, const uint8_t *seed_a, const uint8_t *see
   rc = c.fork(s, &second);
   if (rc) return rc;
   uint32_t *a = d_mpk + (size_t)l * poly;
-  rc = sample_cpu_map(0, 2, rk + 60, l, n, d_msk, sws, c.d_status, c.num_sms, s, e, kSampleCandidates);
+  rc = sample_cpu_map(0, z, rk + 60, d_msk, sws, c.d_status, c.num_sms, s, e, kSampleCandidates);
   if (!rc) rc = sample_polya(rk, n, a, second);
   if (!rc) rc = ntt_fwd_shoup_launch(c.ring.args, a, a_sh, 3, second);
-  if (!rc) rc = sample_cpu_map(0, 2, rk + 60, l, n, d_msk, sws, c.d_status, c.num_sms, s, e, kSampleRest);
+  if (!rc) rc = sample_cpu_map(0, z, rk + 60, d_msk, sws, c.d_status, c.num_sms, s, e, kSampleRest);
   if (rc) {
     c.join(s, second);
     return rc;
@@ -1174,19 +1175,15 @@ static int encrypt_tail(Ctx &c, int batch, const uint32_t *d_x, const uint32_t *
   });
 }
 
-size_t encrypt_workspace_bytes(int n, int l, int batch) {
-  const size_t poly = (size_t)3 * n;
-  return cpu_map_workspace_bytes(batch, l, n, 2) + cpu_map_workspace_bytes(batch, 2, n, 1) +
-         (size_t)batch * ((size_t)l * poly + 2 * poly + 2 * poly) * 4 + (size_t)batch * 2 * 60 * 4 + 16 * 256;
-}
-
 int ctx_encrypt_cpu_map(Ctx &c, int batch, const uint32_t *d_x, const uint32_t *d_mpk, const uint8_t *seeds2,
                         const uint8_t *seeds3, uint32_t *d_ct, cudaStream_t s) {
   if (batch < 1 || !seeds2) return CUFE_ERR_INVALID;
   const int n = c.n, l = c.l;
   const size_t poly = (size_t)3 * n;
-  const size_t ws3 = cpu_map_workspace_bytes(batch, l, n, 2), ws2 = cpu_map_workspace_bytes(batch, 2, n, 1);
-  int rc = c.ensure_ws(encrypt_workspace_bytes(n, l, batch));
+  const SegSizes z3 = cpu_map_sizes(batch, l, n, 2), z2 = cpu_map_sizes(batch, 2, n, 1);
+  const size_t ws3 = seg_scratch_bytes(z3), ws2 = seg_scratch_bytes(z2);
+  int rc = c.ensure_ws(ws3 + ws2 + (size_t)batch * ((size_t)l * poly + 2 * poly + 2 * poly) * 4 +
+                       (size_t)batch * 2 * 60 * 4 + 16 * 256);
   if (rc) return rc;
   Arena ar(c.ws);
   uint32_t *rk = ar.take<uint32_t>((size_t)batch * 2 * 60);
@@ -1213,10 +1210,10 @@ int ctx_encrypt_cpu_map(Ctx &c, int batch, const uint32_t *d_x, const uint32_t *
   rc = c.fork(s, &second);
   if (rc) return rc;
   const uint32_t *rk3 = rk + (size_t)batch * 60;
-  rc = sample_cpu_map(2, batch, rk3, l, n, f3, sws3, c.d_status, sms3, s, nullptr, kSampleCandidates);
-  if (!rc) rc = sample_cpu_map(1, batch, rk, 2, n, s2o, sws2, c.d_status, c.num_sms, second);
+  rc = sample_cpu_map(2, z3, rk3, f3, sws3, c.d_status, sms3, s, nullptr, kSampleCandidates);
+  if (!rc) rc = sample_cpu_map(1, z2, rk, s2o, sws2, c.d_status, c.num_sms, second);
   if (!rc) rc = ntt_fwd_from_launch(c.ring.args, s2o, 2 * poly, rhat, rhat_sh, (long long)batch * 3, second);
-  if (!rc) rc = sample_cpu_map(2, batch, rk3, l, n, f3, sws3, c.d_status, sms3, s, nullptr, kSampleRest);
+  if (!rc) rc = sample_cpu_map(2, z3, rk3, f3, sws3, c.d_status, sms3, s, nullptr, kSampleRest);
   const int rj = c.join(s, second);  // also after an error: what was launched uses the workspace
   if (rc || rj) return rc ? rc : rj;
   return encrypt_tail(c, batch, d_x, d_mpk, rhat, rhat_sh, (long long)poly, f3, (long long)l * poly, s2o + poly,
@@ -1608,7 +1605,8 @@ int ctx_decrypt_coef0(Ctx &c, int nct, const uint32_t *d_ct, int nkeys, const ui
 int ctx_sample_cpu_map(Ctx &c, int sig, int nstreams, const uint8_t *keys, int calls, uint32_t *d_out,
                        cudaStream_t s) {
   if (sig < 0 || sig > 2 || nstreams < 1 || calls < 1) return CUFE_ERR_INVALID;
-  const size_t sws = cpu_map_workspace_bytes(nstreams, calls, c.n, sig);
+  const SegSizes z = cpu_map_sizes(nstreams, calls, c.n, sig);
+  const size_t sws = seg_scratch_bytes(z);
   int rc = c.ensure_ws(sws + (size_t)nstreams * 60 * 4 + 512);
   if (rc) return rc;
   Arena ar(c.ws);
@@ -1616,7 +1614,7 @@ int ctx_sample_cpu_map(Ctx &c, int sig, int nstreams, const uint8_t *keys, int c
   void *w = ar.take<uint8_t>(sws);
   std::vector<uint32_t> k = expand_keys(nstreams, keys);
   CUFE_CUDA(cudaMemcpyAsync(rk, k.data(), k.size() * 4, cudaMemcpyHostToDevice, s));
-  return sample_cpu_map(sig, nstreams, rk, calls, c.n, d_out, w, c.d_status, c.num_sms, s);
+  return sample_cpu_map(sig, z, rk, d_out, w, c.d_status, c.num_sms, s);
 }
 
 int ctx_sample_gpu_map(Ctx &c, int sig, const uint8_t *key, int poly0, int npolys, uint32_t *d_out,

@@ -19,6 +19,7 @@
 #include "prof.h"
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 
 namespace cufe {
@@ -317,7 +318,8 @@ __global__ void __launch_bounds__(kCandThreads, 1)
 // count of accepted candidates reaches E(a_c) + n; a_{c+1} = e + 1.  call_start of stream st:
 // coff[st] + st .. coff[st+1] + st (calls + 1 entries; the last is the end of the last call).
 //
-// Short runs: k_walk, below, one CTA per stream.  Long runs: by the overshoot.  A call ends up to 7
+// Short runs: k_walk, below, one CTA per stream.  Many calls of few refills: pointer doubling (k_next and
+// those after it).  Long runs: by the overshoot.  A call ends up to 7
 // samples beyond its n, and call c ends where the count reaches (c + 1) n + s, s being the overshoot of the
 // calls before it: a number close to c times its mean.  So the refill that ends call c can be
 // written down beforehand for every s in a window around that (k_ends: every refill writes itself
@@ -339,7 +341,8 @@ __device__ __forceinline__ uint32_t window_first(const EndTable &t, uint32_t c) 
 }
 
 // accept counts of tile blockIdx.x of stream blockIdx.y
-__global__ void __launch_bounds__(256) k_tile_counts(const uint8_t *__restrict__ amask, SegDev sg, EndTable t) {
+__global__ void __launch_bounds__(256)
+    k_tile_counts(const uint8_t *__restrict__ amask, SegDev sg, uint32_t *__restrict__ counts, uint32_t max_tiles) {
   __shared__ uint32_t wsum[8];
   const uint64_t r0 = seg_roff(sg, blockIdx.y);
   const uint32_t R = (uint32_t)(seg_roff(sg, blockIdx.y + 1) - r0), at = blockIdx.x * kCountTile + threadIdx.x * 16;
@@ -355,22 +358,21 @@ __global__ void __launch_bounds__(256) k_tile_counts(const uint8_t *__restrict__
   if (threadIdx.x == 0) {
     uint32_t v = 0;
     for (int i = 0; i < 8; ++i) v += wsum[i];
-    t.counts[(size_t)blockIdx.y * t.max_tiles + blockIdx.x] = v;
+    counts[(size_t)blockIdx.y * max_tiles + blockIdx.x] = v;
   }
 }
 
-// the table entries that the refills of tile blockIdx.x of stream blockIdx.y reach
-__global__ void __launch_bounds__(256) k_ends(const uint8_t *__restrict__ amask, SegDev sg, EndTable t) {
+// What a stream has accepted before this thread's 16 refills of tile blockIdx.x, and their masks m and count
+// (256 threads; past: the counts of the stream's tiles; refills at .. at + 15 of R)
+__device__ __forceinline__ uint32_t accepted_before(const uint8_t *amask, uint64_t r0, uint32_t R, uint32_t at,
+                                                    const uint32_t *counts, uint4 &m, uint32_t &own) {
   __shared__ uint32_t wsum[8], psum[8];
-  const uint32_t st = blockIdx.y, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  const uint64_t r0 = seg_roff(sg, st);
-  const uint32_t R = (uint32_t)(seg_roff(sg, st + 1) - r0), at = blockIdx.x * kCountTile + threadIdx.x * 16;
-  if (blockIdx.x * kCountTile >= R) return;
-  uint32_t past = 0;  // accepted in the tiles before
-  for (uint32_t i = threadIdx.x; i < blockIdx.x; i += 256) past += __ldg(t.counts + (size_t)st * t.max_tiles + i);
-  uint4 m = make_uint4(0, 0, 0, 0);
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  uint32_t past = 0;
+  for (uint32_t i = threadIdx.x; i < blockIdx.x; i += 256) past += __ldg(counts + i);
+  m = make_uint4(0, 0, 0, 0);
   if (at < R) m = __ldg(reinterpret_cast<const uint4 *>(amask + r0 + at));
-  const uint32_t own = __popc(m.x) + __popc(m.y) + __popc(m.z) + __popc(m.w);
+  own = __popc(m.x) + __popc(m.y) + __popc(m.z) + __popc(m.w);
   uint32_t inc = own;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -384,6 +386,18 @@ __global__ void __launch_bounds__(256) k_ends(const uint8_t *__restrict__ amask,
   uint32_t E = inc - own;
 #pragma unroll
   for (uint32_t i = 0; i < 8; ++i) E += psum[i] + (i < warp ? wsum[i] : 0u);
+  return E;
+}
+
+// the table entries that the refills of tile blockIdx.x of stream blockIdx.y reach
+__global__ void __launch_bounds__(256) k_ends(const uint8_t *__restrict__ amask, SegDev sg, EndTable t) {
+  const uint32_t st = blockIdx.y;
+  const uint64_t r0 = seg_roff(sg, st);
+  const uint32_t R = (uint32_t)(seg_roff(sg, st + 1) - r0), at = blockIdx.x * kCountTile + threadIdx.x * 16;
+  if (blockIdx.x * kCountTile >= R) return;
+  uint4 m;
+  uint32_t own;
+  uint32_t E = accepted_before(amask, r0, R, at, t.counts + (size_t)st * t.max_tiles, m, own);
   // thresholds (c + 1) n + s in (E, E + own], c the call whose window they can lie in (end_table_width)
   const uint32_t n = seg_n(sg, st), calls = seg_calls(sg, st);
   // c + 1 to the nearest, (c + 1) (n + mean) - mean being the middle of call c's window
@@ -650,6 +664,87 @@ __global__ void __launch_bounds__(kWalkThreads)
     atomicOr(status, kStatusRefillsExhausted);
     for (uint32_t i = c; i <= calls; ++i) cs[i] = R;
   }
+}
+
+// Pointer doubling, for runs whose calls are many and their refills few: the walk and the table take a
+// step per call of the longest stream, this one log2(calls) launches over all refills.  next(t) is the refill
+// after a call that starts at refill t, R + 1 where the stream runs out; call c starts where next applied c
+// times to 0 leads, from the bits of c with the tables next^(2^k).
+//
+// counts of accepted candidates up to and with each refill of tile blockIdx.x of stream blockIdx.y
+__global__ void __launch_bounds__(256)
+    k_prefix(const uint8_t *__restrict__ amask, SegDev sg, const uint32_t *__restrict__ counts, uint32_t max_tiles,
+             uint32_t *__restrict__ upto) {
+  const uint64_t r0 = seg_roff(sg, blockIdx.y);
+  const uint32_t R = (uint32_t)(seg_roff(sg, blockIdx.y + 1) - r0), at = blockIdx.x * kCountTile + threadIdx.x * 16;
+  if (blockIdx.x * kCountTile >= R) return;
+  uint4 m;
+  uint32_t own;
+  uint32_t E = accepted_before(amask, r0, R, at, counts + (size_t)blockIdx.y * max_tiles, m, own);
+  if (at >= R) return;
+  const uint32_t w[4] = {m.x, m.y, m.z, m.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    uint4 v;
+    v.x = E += __popc(w[i] & 0xffu);
+    v.y = E += __popc(w[i] & 0xff00u);
+    v.z = E += __popc(w[i] & 0xff0000u);
+    v.w = E += __popc(w[i] & 0xff000000u);
+    reinterpret_cast<uint4 *>(upto + r0 + at)[i] = v;
+  }
+}
+
+__global__ void __launch_bounds__(256) k_next(const uint32_t *__restrict__ upto, SegDev sg, float mean_accept,
+                                              uint32_t *__restrict__ next) {
+  const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= (uint32_t)seg_roff(sg, sg.nstreams)) return;
+  const uint32_t st = seg_of_refill(sg, g), n = seg_n(sg, st);
+  const uint64_t r0 = seg_roff(sg, st);
+  const uint32_t R = (uint32_t)(seg_roff(sg, st + 1) - r0), t = g - (uint32_t)r0;
+  const uint32_t *up = upto + r0;
+  const uint32_t target = (t ? up[t - 1] : 0u) + n;
+  // the first e >= t with up[e] >= target; twice the expected length first
+  uint32_t lo = t, hi = R;
+  const uint32_t guess = t + 2u * (uint32_t)((float)n / mean_accept) + 64u;
+  if (guess < R && up[guess] >= target) hi = guess;
+  while (lo < hi) {
+    const uint32_t mid = lo + (hi - lo) / 2;
+    if (up[mid] >= target) hi = mid;
+    else lo = mid + 1;
+  }
+  next[g] = lo < R ? lo + 1 : R + 1;
+}
+
+__global__ void __launch_bounds__(256)
+    k_next_square(const uint32_t *__restrict__ in, uint32_t *__restrict__ out, SegDev sg) {
+  const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= (uint32_t)seg_roff(sg, sg.nstreams)) return;
+  const uint32_t st = seg_of_refill(sg, g);
+  const uint64_t r0 = seg_roff(sg, st);
+  const uint32_t R = (uint32_t)(seg_roff(sg, st + 1) - r0), a = in[g];
+  out[g] = a < R ? in[r0 + a] : R + 1;
+}
+
+// one thread per entry of call_start, c = 0 .. calls of every stream
+__global__ void __launch_bounds__(256)
+    k_doubled_starts(const uint32_t *__restrict__ tables, uint32_t levels, uint64_t stride, SegDev sg,
+                     uint32_t *__restrict__ call_start, uint32_t *__restrict__ status) {
+  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= seg_coff(sg, sg.nstreams) + sg.nstreams) return;
+  uint32_t lo = 0, hi = sg.nstreams;  // stream s has the entries from coff[s] + s on
+  while (hi - lo > 1) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (seg_coff(sg, mid) + mid <= i) lo = mid;
+    else hi = mid;
+  }
+  const uint32_t c = (uint32_t)(i - (seg_coff(sg, lo) + lo));
+  const uint64_t r0 = seg_roff(sg, lo);
+  const uint32_t R = (uint32_t)(seg_roff(sg, lo + 1) - r0);
+  uint32_t a = 0;
+  for (uint32_t k = 0; k < levels; ++k)
+    if ((c >> k) & 1u) a = a < R ? tables[k * stride + r0 + a] : R + 1;
+  call_start[i] = min(a, R);
+  if (a > R && c == seg_calls(sg, lo)) atomicOr(status, kStatusRefillsExhausted);
 }
 
 // ------------------------------------------------------------------ CPU mapping, phase 3
@@ -1139,16 +1234,49 @@ SegDev seg_bind(void *base, uint32_t S) {
   return d;
 }
 
-// Width of the table of call ends, 0: k_walk.  The overshoot of a call has a standard deviation
+// Width of the table of call ends, 0: not possible.  The overshoot of a call has a standard deviation
 // below 2, so that of c calls one below 2 sqrt(c): the window takes 4 of those and 64 to either side.  The
 // windows may be n - 192 wide, so that a threshold is in one of them, and the nearest call to
-// any of a thread's 128 thresholds is the one whose window it is in (k_ends).  From 128 calls on the
-// three launches are shorter than the walk (sigma_2, n = 4096, one stream / 16, us against the
-// walk's: 64 calls 22 / 25 against 19 / 19, 128 27 / 32 against 31 / 31, 256 35 / 51 against 56 / 57, 785
-// 72 / 114 against 158 / 158).
+// any of a thread's 128 thresholds is the one whose window it is in (k_ends).
 static uint32_t end_table_width(const SegSizes &z) {
   const uint32_t W = ((uint32_t)(16.0 * std::sqrt((double)z.max_calls)) + 128 + 63) & ~63u;
-  return z.max_calls >= 128 && W + 192 <= z.min_n && z.max_refills < (1u << 28) && z.nstreams < 65536u ? W : 0u;
+  return W + 192 <= z.min_n && z.max_refills < (1u << 28) && z.nstreams < 65536u ? W : 0u;
+}
+
+static uint32_t doubling_levels(const SegSizes &z) {
+  uint32_t k = 1;
+  while (k < 31 && (1u << k) <= z.max_calls) ++k;
+  return k;  // bit length of max_calls
+}
+static bool doubling_ok(const SegSizes &z) { return z.refills <= ((uint64_t)32 << 20) && z.nstreams < 65536u; }
+
+bool seg_search(SegSizes &z, CallSearch how) {
+  const uint32_t w = how == kSearchTable ? end_table_width(z) : 0u;
+  if ((how == kSearchTable && !w) || (how == kSearchDoubling && !doubling_ok(z))) return false;
+  z.search = how;
+  z.end_w = w;
+  return true;
+}
+
+static std::atomic<int> g_call_search{0};
+void set_call_search(int mode) { g_call_search = mode; }
+
+// The search of a run: the one that cufe_sampler_call_search asked for, or by time.  From 128 calls on the
+// table's three launches are shorter than the walk.  Doubling takes over where it is at most 3/4 of the other by
+// these estimates, us on a B200, within 25% of what they were fitted to (n 16..8192, 1..40 streams, 16..16,000
+// calls); by less it is not worth its tables, 4 bytes per refill and level.  Measured, walk | table |
+// doubling, sigma_3 of one stream: n = 4096, 64 calls 19 | 22 | 46, 128 31 | 27 | 50, 784 158 | 72 | 87; n = 512,
+// 256 calls 46 | - | 52, 512 84 | - | 58, 784 125 | - | 57, 4,000 617 | - | 89; n = 1024, 1,024 calls 168 | 89 | 64,
+// 4,000 639 | - | 117; n = 2048, 4,000 calls 684 | 312 | 162; n = 512, 8 streams of 784 calls 126 | - | 84, 40 of
+// them 128 | - | 232.
+static void choose_search(SegSizes &z) {
+  const int mode = g_call_search;
+  seg_search(z, kSearchWalk);
+  if (mode == 1) return;
+  const double calls = z.max_calls, refills = (double)z.refills;
+  double best = 6.0 + 0.146 * calls + 37e-6 * z.max_refills;
+  if (mode == 0 && z.max_calls >= 128 && seg_search(z, kSearchTable)) best = 17.0 + 0.078 * calls + 1.4e-6 * refills;
+  if (mode == 2 || 18.0 + doubling_levels(z) * (3.4 + 3.6e-6 * refills) < 0.75 * best) seg_search(z, kSearchDoubling);
 }
 
 SegSizes seg_fill_host(int sig, uint32_t S, const uint32_t *calls, const uint32_t *n, const uint64_t *ooff,
@@ -1158,7 +1286,7 @@ SegSizes seg_fill_host(int sig, uint32_t S, const uint32_t *calls, const uint32_
   uint32_t *hn = reinterpret_cast<uint32_t *>(b + L.n), *hc = reinterpret_cast<uint32_t *>(b + L.calls);
   uint64_t *hr = reinterpret_cast<uint64_t *>(b + L.roff), *hco = reinterpret_cast<uint64_t *>(b + L.coff);
   uint64_t *ho = reinterpret_cast<uint64_t *>(b + L.ooff);
-  SegSizes z{S, 0, 0, 0, 0, 0xffffffffu, 0};
+  SegSizes z{S, 0, 0, 0, 0, 0xffffffffu, kSearchWalk, 0};
   for (uint32_t i = 0; i < S; ++i) {
     const uint32_t R = cpu_map_refills(calls[i], n[i], sig);
     hn[i] = n[i];
@@ -1174,27 +1302,26 @@ SegSizes seg_fill_host(int sig, uint32_t S, const uint32_t *calls, const uint32_
   }
   hr[S] = z.refills;
   hco[S] = z.calls;
-  z.end_w = end_table_width(z);
+  choose_search(z);
   return z;
 }
 
-static SegSizes seg_uniform_sizes(uint32_t S, uint32_t calls, uint32_t n, int sig) {
+SegSizes cpu_map_sizes(uint32_t S, uint32_t calls, uint32_t n, int sig) {
   const uint32_t R = cpu_map_refills(calls, n, sig);
-  SegSizes z{S, (uint64_t)S * R, (uint64_t)S * calls, R, calls, n, 0};
-  z.end_w = end_table_width(z);
+  SegSizes z{S, (uint64_t)S * R, (uint64_t)S * calls, R, calls, n, kSearchWalk, 0};
+  choose_search(z);
   return z;
 }
 
 static uint32_t count_tiles(const SegSizes &z) { return (z.max_refills + kCountTile - 1) / kCountTile; }
 
 size_t seg_scratch_bytes(const SegSizes &z) {
-  return align256(z.refills * 32) + align256(z.refills) + align256(z.refills * 2) +
-         align256((z.calls + z.nstreams) * 4) +
-         (z.end_w ? align256((size_t)z.calls * z.end_w * 4) + align256((size_t)z.nstreams * count_tiles(z) * 4) : 0);
-}
-
-size_t cpu_map_workspace_bytes(uint32_t nstreams, uint32_t calls, uint32_t n, int sig) {
-  return seg_scratch_bytes(seg_uniform_sizes(nstreams, calls, n, sig));
+  size_t b = align256(z.refills * 32) + align256(z.refills) + align256(z.refills * 2) +
+             align256((z.calls + z.nstreams) * 4);
+  if (z.search != kSearchWalk) b += align256((size_t)z.nstreams * count_tiles(z) * 4);
+  if (z.search == kSearchTable) b += align256((size_t)z.calls * z.end_w * 4);
+  if (z.search == kSearchDoubling) b += (1 + (size_t)doubling_levels(z)) * align256(z.refills * 4);
+  return b;
 }
 
 int sample_cpu_map_seg(int sig, const SegDev &sg, const SegSizes &z, const uint32_t *d_rkeys, uint32_t *d_out,
@@ -1231,17 +1358,30 @@ int sample_cpu_map_seg(int sig, const SegDev &sg, const SegSizes &z, const uint3
   if (!(parts & kSampleRest)) return CUFE_OK;
   {
     ProfScope ps("sample_walk", s);
-    if (z.end_w) {
+    const dim3 tiles(count_tiles(z), z.nstreams);
+    if (z.search == kSearchTable) {
       EndTable t;
       t.ends = reinterpret_cast<uint32_t *>(take((size_t)z.calls * z.end_w * 4));
-      t.max_tiles = count_tiles(z);
-      t.counts = reinterpret_cast<uint32_t *>(take((size_t)z.nstreams * t.max_tiles * 4));
+      t.max_tiles = tiles.x;
+      t.counts = reinterpret_cast<uint32_t *>(take((size_t)z.nstreams * tiles.x * 4));
       t.W = z.end_w;
       t.mean = mean_overshoot(sig);
-      const dim3 grid(t.max_tiles, z.nstreams);
-      note_launch(), k_tile_counts<<<grid, 256, 0, s>>>(amask, sg, t);
-      note_launch(), k_ends<<<grid, 256, 0, s>>>(amask, sg, t);
+      note_launch(), k_tile_counts<<<tiles, 256, 0, s>>>(amask, sg, t.counts, tiles.x);
+      note_launch(), k_ends<<<tiles, 256, 0, s>>>(amask, sg, t);
       note_launch(), k_chain<<<z.nstreams, 128, 0, s>>>(amask, sg, t, cstart, d_status);
+    } else if (z.search == kSearchDoubling) {
+      uint32_t *counts = reinterpret_cast<uint32_t *>(take((size_t)z.nstreams * tiles.x * 4));
+      uint32_t *upto = reinterpret_cast<uint32_t *>(take(z.refills * 4));
+      const uint32_t levels = doubling_levels(z), grid = (uint32_t)((z.refills + 255) / 256);
+      const uint64_t stride = align256(z.refills * 4) / 4;
+      uint32_t *tab = reinterpret_cast<uint32_t *>(take(levels * stride * 4));
+      note_launch(), k_tile_counts<<<tiles, 256, 0, s>>>(amask, sg, counts, tiles.x);
+      note_launch(), k_prefix<<<tiles, 256, 0, s>>>(amask, sg, counts, tiles.x, upto);
+      note_launch(), k_next<<<grid, 256, 0, s>>>(upto, sg, (float)mean_accept(sig), tab);
+      for (uint32_t k = 1; k < levels; ++k)
+        note_launch(), k_next_square<<<grid, 256, 0, s>>>(tab + (k - 1) * stride, tab + k * stride, sg);
+      note_launch(), k_doubled_starts<<<(uint32_t)((z.calls + z.nstreams + 255) / 256), 256, 0, s>>>(tab, levels, stride, sg,
+                                                                                                 cstart, d_status);
     } else {
       note_launch(), k_walk<<<z.nstreams, kWalkThreads, 0, s>>>(amask, sg, (float)mean_accept(sig), cstart, d_status);
     }
@@ -1256,19 +1396,17 @@ int sample_cpu_map_seg(int sig, const SegDev &sg, const SegSizes &z, const uint3
   return CUFE_OK;
 }
 
-// the uniform case: nstreams equal streams, no tables
-int sample_cpu_map(int sig, uint32_t nstreams, const uint32_t *d_rkeys, uint32_t calls, uint32_t n,
-                   uint32_t *d_out, void *ws, uint32_t *d_status, int num_sms, cudaStream_t s, uint32_t *d_out1,
-                   int parts) {
-  const SegSizes z = seg_uniform_sizes(nstreams, calls, n, sig);
-  if (z.refills / nstreams >= (1ull << 32) / 24) return CUFE_ERR_INVALID;  // AES counter range
-  if (d_out1 && nstreams != 2) return CUFE_ERR_INVALID;
+// the uniform case: equal streams, no tables
+int sample_cpu_map(int sig, const SegSizes &z, const uint32_t *d_rkeys, uint32_t *d_out, void *ws, uint32_t *d_status,
+                   int num_sms, cudaStream_t s, uint32_t *d_out1, int parts) {
+  if (z.max_refills >= (1ull << 32) / 24) return CUFE_ERR_INVALID;  // AES counter range
+  if (d_out1 && z.nstreams != 2) return CUFE_ERR_INVALID;
   SegDev sg{};
-  sg.nstreams = nstreams;
-  sg.u_n = n;
-  sg.u_calls = calls;
-  sg.u_refills = (uint32_t)(z.refills / nstreams);
-  sg.u_ostride = (uint64_t)calls * 3 * n;
+  sg.nstreams = z.nstreams;
+  sg.u_n = z.min_n;
+  sg.u_calls = z.max_calls;
+  sg.u_refills = z.max_refills;
+  sg.u_ostride = (uint64_t)z.max_calls * 3 * z.min_n;
   if (d_out1)  // two streams: the distance between their outputs, wherever they lie
     sg.u_ostride = (uint64_t)((reinterpret_cast<intptr_t>(d_out1) - reinterpret_cast<intptr_t>(d_out)) / 4);
   return sample_cpu_map_seg(sig, sg, z, d_rkeys, d_out, ws, d_status, num_sms, s, parts);

@@ -24,14 +24,7 @@ int expand_keys_device(const uint8_t *d_seeds, const uint32_t *d_perm, uint32_t 
 enum { kSampleCandidates = 1, kSampleRest = 2, kSampleAll = 3 };
 constexpr int kCandThreads = 512;  // threads of a candidate CTA, one CTA per SM
 
-// CPU stream mapping: nstreams independent AES-CTR streams (round keys d_rkeys[nstreams][60],
-// nonce 0, counter 0), each running `calls` consecutive sampler calls of n samples with
-// sigma index sig; residues written to d_out[nstreams][calls][3][n], those of the second of two to d_out1 where given.
 uint32_t cpu_map_refills(uint32_t calls, uint32_t n, int sig);
-size_t cpu_map_workspace_bytes(uint32_t nstreams, uint32_t calls, uint32_t n, int sig);
-int sample_cpu_map(int sig, uint32_t nstreams, const uint32_t *d_rkeys, uint32_t calls, uint32_t n,
-                   uint32_t *d_out, void *ws, uint32_t *d_status, int num_sms, cudaStream_t s,
-                   uint32_t *d_out1 = nullptr, int parts = kSampleAll);
 
 // Segmented form: S CPU-mapping streams of different lengths.  Stream s runs calls[s]
 // sampler calls of n[s] samples; its refills occupy [roff[s], roff[s+1]) of the flattened
@@ -46,13 +39,22 @@ struct SegDev {
   uint32_t u_n, u_calls, u_refills;
   uint64_t u_ostride;
 };
+// How a run finds where its calls start (sampler.cu)
+enum CallSearch : uint32_t { kSearchWalk, kSearchDoubling, kSearchTable };
 struct SegSizes {
   uint32_t nstreams;
   uint64_t refills;
   uint64_t calls;
   uint32_t max_refills, max_calls, min_n;  // over the streams
-  uint32_t end_w;  // words per call of the table of call ends; 0 (also set by callers without room): the walk
+  CallSearch search;
+  uint32_t end_w;  // words per call of the table of call ends (kSearchTable)
 };
+// another search for a run, before its scratch is laid out; false, and no change, where its sizes do not allow
+// it (the walk they always do)
+bool seg_search(SegSizes &z, CallSearch how);
+// cufe_sampler_call_search: 0 the quickest, 1 the walk, 2 doubling where it is possible, for the sizes computed
+// from now on
+void set_call_search(int mode);
 struct SegLayout {
   size_t n, calls, roff, coff, ooff, bytes;
 };
@@ -68,6 +70,14 @@ size_t seg_scratch_bytes(const SegSizes &z);
 // segmented run: candidates, scan, call starts and the scatter of the residues to d_out
 int sample_cpu_map_seg(int sig, const SegDev &sg, const SegSizes &z, const uint32_t *d_rkeys, uint32_t *d_out,
                        void *scratch, uint32_t *d_status, int num_sms, cudaStream_t s, int parts = kSampleAll);
+
+// CPU stream mapping: equal independent AES-CTR streams (round keys d_rkeys[nstreams][60], nonce 0, counter
+// 0), each running `calls` consecutive sampler calls of n samples with sigma index sig; z from cpu_map_sizes,
+// scratch of seg_scratch_bytes(z); residues written to d_out[nstreams][calls][3][n], those of the second of two
+// streams to d_out1 where given.
+SegSizes cpu_map_sizes(uint32_t nstreams, uint32_t calls, uint32_t n, int sig);
+int sample_cpu_map(int sig, const SegSizes &z, const uint32_t *d_rkeys, uint32_t *d_out, void *ws, uint32_t *d_status,
+                   int num_sms, cudaStream_t s, uint32_t *d_out1 = nullptr, int parts = kSampleAll);
 
 // GPU counter mapping: polynomials poly0 .. poly0+npolys-1 of one key, residues to
 // d_out[npolys][3][n].

@@ -186,9 +186,12 @@ int cufe_sample_gpu_map(cufe_ctx *ctx, int sig, const uint8_t key[32], int poly0
 /* sample_polya (src/sample.c:56-128): d_a[3][n] */
 int cufe_sample_polya(cufe_ctx *ctx, const uint8_t seed[32], uint32_t *d_a, void *stream);
 
-/* The CPU-mapping samplers find where each gaussian_sampler_S* call starts by a streamed walk, or
- * by a table of call ends in long runs.  Modes 0, 1 and 2, which chose between a walk and pointer
- * doubling, are accepted and make no difference; others are refused. */
+/* How the CPU-mapping samplers find where each gaussian_sampler_S* call starts (process-wide; all give
+ * the same samples): 0 (default) the quickest by estimated time of a streamed walk (one step per call of the
+ * longest stream), a table of call ends (one shorter step per call; rings wide enough for its windows)
+ * and pointer doubling (parallel over refills, log2(calls) table levels; runs up to 32 Mi refills); 1
+ * always the walk; 2 doubling whenever the run is within 32 Mi refills.  Applies to workspaces sized
+ * after the call. */
 int cufe_sampler_call_search(int mode);
 
 /* Serialized keys and ciphertexts: a 32-byte header (magic "CUFE", version 1, kind, n, l,
