@@ -131,7 +131,18 @@ int Ring::init(int n_, int k_, const uint32_t *primes, int dev) {
     const uint64_t qq = q[m], w = root_for(q[m], n), wi = invmod(w, qq);
     psi_root[m] = (uint32_t)w;
     pw[0] = ipw[0] = 1;
-    for (int e = 1; e < n; ++e) pw[e] = pw[e - 1] * w % qq, ipw[e] = ipw[e - 1] * wi % qq;
+    // without divisions, which were most of a context's creation: x w mod q by the companion of w, and
+    // floor(a 2^32 / q) by floor(2^64 / q), which gives it or one less
+    const uint64_t w_sh = (w << 32) / qq, wi_sh = (wi << 32) / qq, mu = (uint64_t)(((u128)1 << 64) / qq);
+    const auto times = [qq](uint64_t x, uint64_t y, uint64_t y_sh) {
+      const uint64_t r = x * y - (x * y_sh >> 32) * qq;
+      return r >= qq ? r - qq : r;
+    };
+    const auto companion = [qq, mu](uint32_t a) {
+      const uint64_t t = (uint64_t)a << 32, f = (uint64_t)((u128)t * mu >> 64);
+      return (uint32_t)(f + (t - f * qq >= qq));
+    };
+    for (int e = 1; e < n; ++e) pw[e] = times(pw[e - 1], w, w_sh), ipw[e] = times(ipw[e - 1], wi, wi_sh);
     for (int i = 0; i < n; ++i) {
       const uint32_t a = (uint32_t)pw[bitrev(i, logn)], b = (uint32_t)ipw[bitrev(i, logn)];
       h_psi[(size_t)m * n + i] = a;
@@ -142,7 +153,7 @@ int Ring::init(int n_, int k_, const uint32_t *primes, int dev) {
         const int th = (i - n / 2) >> 3, g = i & 7;
         at = n / 2 + (((g >> 2) * (n / 16) + th) << 2) + (g & 3);
       }
-      const uint32_t a_sh = shoup_of(a, (uint32_t)qq), b_sh = shoup_of(b, (uint32_t)qq);
+      const uint32_t a_sh = companion(a), b_sh = companion(b);
       for (int flat = 0; flat < 2; ++flat) {
         uint32_t *f = &tab[2 * (((size_t)2 * flat * k + m) * n + (flat ? i : at))];
         f[0] = a;
