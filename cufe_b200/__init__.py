@@ -72,6 +72,7 @@ def lib():
             "cufe_batch_tune": [vp, i, vp, vp, vp, vp],
             "cufe_decrypt_coef0": [vp, i, vp, i, vp, i, vp, vp, vp, vp],
             "cufe_sample_cpu_map": [vp, i, i, vp, i, vp, vp],
+            "cufe_sample_cpu_map_form": [vp, i, i, i, vp, i, vp, vp],
             "cufe_sample_gpu_map": [vp, i, vp, i, i, vp, vp],
             "cufe_sample_polya": [vp, vp, vp, vp],
             "cufe_ring_create": [C.POINTER(vp), i, i, vp, i],
@@ -407,6 +408,14 @@ class Context:
         ns = nstreams if nstreams is not None else (1 if k is None else len(k) // 32)
         out = _dev((ns, calls, 3, self.n), self.dev) if out is None else out
         _check(lib().cufe_sample_cpu_map(self.h, sig, ns, _ptr(k), calls, _ptr(out), _stream(stream, self.device)), "cufe_sample_cpu_map")
+        return out
+
+    def sample_cpu_map_form(self, form, sig, keys, calls, stream=None):
+        """sample_cpu_map with a given search for the call starts (0 rule, 1 walk, 2 doubling, 3..5 table)"""
+        k = _seeds(keys)
+        out = _dev((len(k) // 32, calls, 3, self.n), self.dev)
+        _check(lib().cufe_sample_cpu_map_form(self.h, form, sig, len(k) // 32, _ptr(k), calls, _ptr(out),
+                                              _stream(stream, self.device)), "cufe_sample_cpu_map_form")
         return out
 
     def sample_gpu_map(self, sig, key, poly0, npolys, out=None, stream=None):

@@ -235,7 +235,13 @@ int cufe_decode(cufe_ctx *h, int count, const uint32_t *d_dy, int ncoeff, uint32
 int cufe_sample_cpu_map(cufe_ctx *h, int sig, int nstreams, const uint8_t *keys, int calls, uint32_t *d_out,
                         void *stream) {
   if (!d_out) return CUFE_ERR_INVALID;
-  CTX_CALL(h, cufe::ctx_sample_cpu_map(h->c, sig, nstreams, keys, calls, d_out, h->c.pick(stream)));
+  CTX_CALL(h, cufe::ctx_sample_cpu_map(h->c, 0, sig, nstreams, keys, calls, d_out, h->c.pick(stream)));
+}
+
+int cufe_sample_cpu_map_form(cufe_ctx *h, int form, int sig, int nstreams, const uint8_t *keys, int calls,
+                             uint32_t *d_out, void *stream) {
+  if (!d_out) return CUFE_ERR_INVALID;
+  CTX_CALL(h, cufe::ctx_sample_cpu_map(h->c, form, sig, nstreams, keys, calls, d_out, h->c.pick(stream)));
 }
 
 int cufe_sample_gpu_map(cufe_ctx *h, int sig, const uint8_t key[32], int poly0, int npolys, uint32_t *d_out,

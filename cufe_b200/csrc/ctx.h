@@ -136,7 +136,7 @@ int ctx_tune_encrypt(Ctx &c, int batch, const uint32_t *d_x, const uint32_t *d_m
                      const uint8_t *seeds3, uint32_t *d_ct, int *choice, float *ms, cudaStream_t s);
 int ctx_tune_decrypt_coef0(Ctx &c, int nct, const uint32_t *d_ct, int nkeys, const uint32_t *d_y, int y_signed,
                            const uint32_t *d_sky, uint32_t *d_out, int *choice, float *ms, cudaStream_t s);
-int ctx_sample_cpu_map(Ctx &c, int sig, int nstreams, const uint8_t *keys, int calls, uint32_t *d_out,
+int ctx_sample_cpu_map(Ctx &c, int form, int sig, int nstreams, const uint8_t *keys, int calls, uint32_t *d_out,
                        cudaStream_t s);
 int ctx_sample_gpu_map(Ctx &c, int sig, const uint8_t *key, int poly0, int npolys, uint32_t *d_out,
                        cudaStream_t s);

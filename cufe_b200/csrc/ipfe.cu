@@ -1613,10 +1613,14 @@ int ctx_decrypt_coef0(Ctx &c, int nct, const uint32_t *d_ct, int nkeys, const ui
                                 d_out, s);
 }
 
-int ctx_sample_cpu_map(Ctx &c, int sig, int nstreams, const uint8_t *keys, int calls, uint32_t *d_out,
+// form 0: the run's own search for its call starts; 1 the walk, 2 doubling, 3 the table of call ends, 4 and 5 the
+// table with windows that lose the overshoot to either side
+int ctx_sample_cpu_map(Ctx &c, int form, int sig, int nstreams, const uint8_t *keys, int calls, uint32_t *d_out,
                        cudaStream_t s) {
-  if (sig < 0 || sig > 2 || nstreams < 1 || calls < 1) return CUFE_ERR_INVALID;
-  const SegSizes z = cpu_map_sizes(nstreams, calls, c.n, sig);
+  if (sig < 0 || sig > 2 || nstreams < 1 || calls < 1 || form < 0 || form > 5) return CUFE_ERR_INVALID;
+  SegSizes z = cpu_map_sizes(nstreams, calls, c.n, sig);
+  if (form && !seg_search(z, form == 1 ? kSearchWalk : form == 2 ? kSearchDoubling : kSearchTable)) return CUFE_ERR_INVALID;
+  if (form > 3) z.end_mean = form == 4 ? 0 : 2;
   const size_t sws = seg_scratch_bytes(z);
   int rc = c.ensure_ws(sws + (size_t)nstreams * 60 * 4 + 512);
   if (rc) return rc;

@@ -1255,6 +1255,7 @@ bool seg_search(SegSizes &z, CallSearch how) {
   if ((how == kSearchTable && !w) || (how == kSearchDoubling && !doubling_ok(z))) return false;
   z.search = how;
   z.end_w = w;
+  z.end_mean = 1;
   return true;
 }
 
@@ -1286,7 +1287,7 @@ SegSizes seg_fill_host(int sig, uint32_t S, const uint32_t *calls, const uint32_
   uint32_t *hn = reinterpret_cast<uint32_t *>(b + L.n), *hc = reinterpret_cast<uint32_t *>(b + L.calls);
   uint64_t *hr = reinterpret_cast<uint64_t *>(b + L.roff), *hco = reinterpret_cast<uint64_t *>(b + L.coff);
   uint64_t *ho = reinterpret_cast<uint64_t *>(b + L.ooff);
-  SegSizes z{S, 0, 0, 0, 0, 0xffffffffu, kSearchWalk, 0};
+  SegSizes z{S, 0, 0, 0, 0, 0xffffffffu, kSearchWalk, 0, 1};
   for (uint32_t i = 0; i < S; ++i) {
     const uint32_t R = cpu_map_refills(calls[i], n[i], sig);
     hn[i] = n[i];
@@ -1308,7 +1309,7 @@ SegSizes seg_fill_host(int sig, uint32_t S, const uint32_t *calls, const uint32_
 
 SegSizes cpu_map_sizes(uint32_t S, uint32_t calls, uint32_t n, int sig) {
   const uint32_t R = cpu_map_refills(calls, n, sig);
-  SegSizes z{S, (uint64_t)S * R, (uint64_t)S * calls, R, calls, n, kSearchWalk, 0};
+  SegSizes z{S, (uint64_t)S * R, (uint64_t)S * calls, R, calls, n, kSearchWalk, 0, 1};
   choose_search(z);
   return z;
 }
@@ -1365,7 +1366,7 @@ int sample_cpu_map_seg(int sig, const SegDev &sg, const SegSizes &z, const uint3
       t.max_tiles = tiles.x;
       t.counts = reinterpret_cast<uint32_t *>(take((size_t)z.nstreams * tiles.x * 4));
       t.W = z.end_w;
-      t.mean = mean_overshoot(sig);
+      t.mean = z.end_mean * mean_overshoot(sig);
       note_launch(), k_tile_counts<<<tiles, 256, 0, s>>>(amask, sg, t.counts, tiles.x);
       note_launch(), k_ends<<<tiles, 256, 0, s>>>(amask, sg, t);
       note_launch(), k_chain<<<z.nstreams, 128, 0, s>>>(amask, sg, t, cstart, d_status);

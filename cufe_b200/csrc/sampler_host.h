@@ -47,7 +47,8 @@ struct SegSizes {
   uint64_t calls;
   uint32_t max_refills, max_calls, min_n;  // over the streams
   CallSearch search;
-  uint32_t end_w;  // words per call of the table of call ends (kSearchTable)
+  uint32_t end_w;     // words per call of the table of call ends (kSearchTable)
+  uint32_t end_mean;  // its windows follow this many times the mean overshoot: 1, or 0 or 2 to lead them astray
 };
 // another search for a run, before its scratch is laid out; false, and no change, where its sizes do not allow
 // it (the walk they always do)

@@ -177,6 +177,12 @@ int cufe_decrypt_coef0_form(cufe_ctx *ctx, int form, int nct, const uint32_t *d_
  * gaussian_sampler_S* calls of n samples (src/gauss.c:789,995,1086): d_out[nstreams][calls][3][n]. */
 int cufe_sample_cpu_map(cufe_ctx *ctx, int sig, int nstreams, const uint8_t *keys, int calls, uint32_t *d_out,
                         void *stream);
+/* The same with a given search for the call starts (tests, comparisons): 0 the run's own choice (see
+ * cufe_sampler_call_search), 1 the walk, 2 doubling, 3 the table of call ends, 4 and 5 the table with windows that
+ * follow none and twice of the mean overshoot, so that its recoveries run; CUFE_ERR_INVALID where the sizes do
+ * not allow it. */
+int cufe_sample_cpu_map_form(cufe_ctx *ctx, int form, int sig, int nstreams, const uint8_t *keys, int calls,
+                             uint32_t *d_out, void *stream);
 /* refills (384-byte AES-CTR blocks of 8 candidates) that the CPU-mapping sampler
  * precomputes per stream for `calls` calls of n samples (sizing and roofline accounting) */
 long long cufe_sampler_refills(int sig, int calls, int n);
