@@ -10,7 +10,8 @@
 // compiler spent one more addition per lookup whenever its address folding did not apply (1,411
 // against 1,039 million instructions for the sigma_3 candidates of four encryptions at n = 4096,
 // l = 784).  Kernels that use the tables therefore take kAesSmemBytes = 192 KiB of dynamic
-// shared memory (it starts below address 0x10000, so it covers the tables) and no static one.
+// shared memory and no static one of 64 KiB; it starts below address 0x10000 then, so it covers the tables,
+// which every such kernel checks before it writes them.
 // Round keys are 60 big-endian words in registers; an all-zero key schedule is valid (the
 // reference CPU path's uninitialised AES contexts).
 #pragma once
@@ -29,9 +30,28 @@ __device__ __forceinline__ uint32_t xtime_u8(uint32_t b) {
   return ((b << 1) ^ ((b & 0x80u) ? 0x1bu : 0u)) & 0xffu;
 }
 
+// whether dynamic shared memory of `bytes` from address `base` holds the tables
+__host__ __device__ constexpr bool aes_tables_fit(uint32_t base, uint32_t bytes) {
+  return base <= kAesTables && bytes >= (uint32_t)kAesTableBytes && base + bytes - kAesTableBytes >= kAesTables;
+}
+static_assert(aes_tables_fit(0, kAesSmemBytes) && aes_tables_fit(0x400, kAesSmemBytes) &&
+                  aes_tables_fit(kAesTables, kAesSmemBytes) && aes_tables_fit(kAesTables, kAesTableBytes),
+              "tables inside");
+static_assert(!aes_tables_fit(kAesTables + 1, kAesSmemBytes) && !aes_tables_fit(0, kAesSmemBytes - 1) &&
+                  !aes_tables_fit(0x400, kAesTableBytes) && !aes_tables_fit(0, 0),
+              "tables outside");
+
 // fill the replicated tables (all threads of the CTA, a multiple of 16; caller syncs): 16 threads
-// write the 256 bytes of one entry of a pair of tables, 16 bytes each
-__device__ __forceinline__ void aes_fill_tables() {
+// write the 256 bytes of one entry of a pair of tables, 16 bytes each.  False, with nothing written and
+// the status set, where the CTA's shared memory does not lie as they need it.
+__device__ __forceinline__ bool aes_fill_tables(uint32_t *status) {
+  extern __shared__ uint32_t smem_u32[];
+  uint32_t bytes;
+  asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(bytes));
+  if (!aes_tables_fit((uint32_t)__cvta_generic_to_shared(smem_u32), bytes)) {
+    if (threadIdx.x == 0) atomicOr(status, kStatusAesTables);
+    return false;
+  }
   const uint32_t tid = threadIdx.x + threadIdx.y * blockDim.x, piece = tid & 15u;
   for (uint32_t x = tid >> 4; x < 256; x += (blockDim.x * blockDim.y) >> 4) {
     const uint32_t s = c_sbox[x], d = xtime_u8(s);
@@ -41,6 +61,7 @@ __device__ __forceinline__ void aes_fill_tables() {
     asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(at), "r"(lo) : "memory");
     asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(at + 65536), "r"(hi) : "memory");
   }
+  return true;
 }
 
 struct AesCtx {

@@ -42,7 +42,8 @@ enum : uint32_t {
   kStatusRefillsExhausted = 2u, // mode A: the precomputed refills did not cover all calls
   kStatusRefillCap = 4u,        // GPU mapping: a thread exceeded kMaxRefillsPerThread refills
   kStatusWideSample = 8u,       // an accepted candidate at or above 2^33 (z = K x + y < 8K keeps it below)
-  kStatusMmaTimeout = 16u,      // a wait for the tensor core gave up (mac.cu)
+  kStatusMmaTimeout = 16u,      // a wait for the tensor core gave up (mac.cu, coef0.cu)
+  kStatusAesTables = 32u,       // shared memory not where the samplers' tables are (aes.cuh)
 };
 
 // ------------------------------------------------------------------ arithmetic

@@ -1012,6 +1012,7 @@ int Ctx::check_status(cudaStream_t s) {
     if (st & 4u) why += " GPU-mapping refill cap reached;";
     if (st & 8u) why += " candidate at or above 2^33;";
     if (st & 16u) why += " a wait for the tensor core gave up;";
+    if (st & 32u) why += " shared memory not where the samplers' tables are;";
     set_last_error(std::string("sampler status ") + std::to_string(st) + ":" + why);
     return CUFE_ERR_SAMPLER;
   }
@@ -1120,7 +1121,7 @@ int ctx_setup_cpu_map_l(Ctx &c, int l, const uint8_t *seed_a, const uint8_t *see
   if (rc) return rc;
   uint32_t *a = d_mpk + (size_t)l * poly;
   rc = sample_cpu_map(0, z, rk + 60, d_msk, sws, c.d_status, c.num_sms, s, e, kSampleCandidates);
-  if (!rc) rc = sample_polya(rk, n, a, second);
+  if (!rc) rc = sample_polya(rk, n, a, c.d_status, second);
   if (!rc) rc = ntt_fwd_shoup_launch(c.ring.args, a, a_sh, 3, second);
   if (!rc) rc = sample_cpu_map(0, z, rk + 60, d_msk, sws, c.d_status, c.num_sms, s, e, kSampleRest);
   if (rc) {
@@ -1650,7 +1651,7 @@ int ctx_sample_polya(Ctx &c, const uint8_t *seed, uint32_t *d_a, cudaStream_t s)
   uint32_t k[60];
   aes_key_expand(seed, k);
   CUFE_CUDA(cudaMemcpyAsync(c.ws, k, sizeof(k), cudaMemcpyHostToDevice, s));
-  return sample_polya(reinterpret_cast<uint32_t *>(c.ws), c.n, d_a, s);
+  return sample_polya(reinterpret_cast<uint32_t *>(c.ws), c.n, d_a, c.d_status, s);
 }
 
 }  // namespace cufe

@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(kCandThreads, 1)
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
   const uint32_t run = ((total + warps - 1) / warps + 31u) & ~31u;
   if (blockIdx.x * run >= total) return;
-  aes_fill_tables();
+  if (!aes_fill_tables(status)) return;
   __syncthreads();
   const AesCtx c = aes_ctx();
   uint32_t rk[60];
@@ -906,7 +906,7 @@ __global__ void __launch_bounds__(kGpuMapThreads, 1)
                     uint32_t group, double kinv, ModArgs m, uint32_t *__restrict__ out, uint32_t *__restrict__ status) {
   const uint32_t T = n / 8, lane = threadIdx.x & 31u;
   if ((uint64_t)blockIdx.x * run >= tasks) return;  // no task for this CTA's first warp, nor for the others
-  aes_fill_tables();
+  if (!aes_fill_tables(status)) return;
   __syncthreads();
   const uint32_t wi = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
   const uint64_t first = (uint64_t)wi * run;
@@ -1035,8 +1035,8 @@ __global__ void __launch_bounds__(kGpuMapThreads, 1)
 
 // sample_polya (src/sample.c:56-128): AES-CTR (nonce 0) bytes, a_i = le64(bytes 8i..8i+7) mod q_j
 __global__ void __launch_bounds__(256) k_polya(const uint32_t *__restrict__ rkey, uint32_t n, ModArgs m,
-                                               uint32_t *__restrict__ a) {
-  aes_fill_tables();
+                                               uint32_t *__restrict__ a, uint32_t *__restrict__ status) {
+  if (!aes_fill_tables(status)) return;
   __syncthreads();
   const AesCtx c = aes_ctx();
   uint32_t rk[60];
@@ -1437,10 +1437,10 @@ int sample_gpu_map(int sig, const uint32_t *d_rkey, uint32_t poly0, uint32_t npo
   return CUFE_OK;
 }
 
-int sample_polya(const uint32_t *d_rkey, uint32_t n, uint32_t *d_a, cudaStream_t s) {
+int sample_polya(const uint32_t *d_rkey, uint32_t n, uint32_t *d_a, uint32_t *d_status, cudaStream_t s) {
   const uint32_t grid = (n / 2 + 255) / 256;
   ProfScope ps("sample_polya", s);
-  note_launch(), k_polya<<<grid, 256, kAesSmemBytes, s>>>(d_rkey, n, mod_args(), d_a);
+  note_launch(), k_polya<<<grid, 256, kAesSmemBytes, s>>>(d_rkey, n, mod_args(), d_a, d_status);
   CUFE_CUDA(cudaGetLastError());
   return CUFE_OK;
 }

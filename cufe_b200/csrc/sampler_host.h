@@ -86,6 +86,6 @@ int sample_gpu_map(int sig, const uint32_t *d_rkey, uint32_t poly0, uint32_t npo
                    uint32_t *d_out, uint32_t *d_status, int num_sms, cudaStream_t s);
 
 // uniform a (sample_polya): d_a[3][n]
-int sample_polya(const uint32_t *d_rkey, uint32_t n, uint32_t *d_a, cudaStream_t s);
+int sample_polya(const uint32_t *d_rkey, uint32_t n, uint32_t *d_a, uint32_t *d_status, cudaStream_t s);
 
 }  // namespace cufe
