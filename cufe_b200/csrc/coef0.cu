@@ -45,9 +45,7 @@ struct Coef0Args {
   int ct_tiles, key_tiles, chunks, poly_chunks, splits;
   uint8_t *pa, *pb;  // packed blocks [tile][m][chunk]
   uint32_t *part;    // [split][m][pair]
-  // reduction of x < 2^51 mod q: (x >> 20) mul >> (32 + sh), mul = floor(2^(52 + sh) / q) of 32 bits, is
-  // floor(x / q) or one less (the cut-off bits are below q / 8)
-  uint32_t mul[3];
+  uint32_t mul[3];  // recip20
   int sh[3];
 };
 
@@ -309,9 +307,8 @@ int coef0_mma_launch(Ctx &c, const SchemeArgs &sa, const DecodeArgs &dd, int nct
   a.pb = a.pa + p.pa;
   a.part = reinterpret_cast<uint32_t *>(a.pb + p.pb);
   for (int j = 0; j < 3; ++j) {
-    const uint64_t q = sa.ra.q[j];
-    for (a.sh[j] = 0; ((1ull << 53) << a.sh[j]) / q < (1ull << 32);) ++a.sh[j];
-    a.mul[j] = (uint32_t)(((1ull << 52) << a.sh[j]) / q);
+    a.mul[j] = recip20(sa.ra.q[j]).mul;
+    a.sh[j] = recip20(sa.ra.q[j]).sh;
   }
   CUFE_CUDA(cudaFuncSetAttribute(k_coef0_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kC0Smem));
   const unsigned rows = (unsigned)p.ct_tiles * kC0Cts + (unsigned)p.key_tiles * kC0Keys;

@@ -1019,6 +1019,7 @@ int Ctx::check_status(cudaStream_t s) {
   return CUFE_OK;
 }
 
+static_assert(recip20_ok(kRefPrimes[0]) && recip20_ok(kRefPrimes[1]) && recip20_ok(kRefPrimes[2]), "recip20");
 static SchemeArgs scheme_args(const Ctx &c) {
   SchemeArgs sa;
   sa.ra = c.ring.args;

@@ -7,7 +7,8 @@
 // product of many keys with v on the tensor cores.  Before, every product was three integer
 // instructions and v was read once per 4 keys (key generation) or per key (decryption).  B200,
 // us per call, before -> now: 1 key at n = 4096, l = 784 277 -> 13; 591 keys at l = 785 2034 -> 70;
-// the decryption of one ciphertext under 591 keys at n = 2048, l = 124 254 -> 100.
+// the decryption of one ciphertext under 591 keys at n = 2048, l = 124 254 -> 100 (60 with its transforms read
+// where they lie and launched at once).
 #include <algorithm>
 
 #include "ctx.h"
@@ -231,10 +232,8 @@ struct MmaArgs {
   const uint32_t *y;
   int y_signed, nkeys, nz, key_tiles, vec;
   uint32_t *out;
-  // Reduction of a sum s, |s| < 2^50 (l <= 1280): with off a multiple of q of at least 2^50 and below
-  // 2^50 + 2^31, x = s + off is in [0, 2^51 + 2^31); its top (x >> 20, 32 bits) times
-  // mul = floor(2^(52 + sh) / q) (32 bits) gives floor(x / q) or one less, since the cut-off bits
-  // are below 2^20 < q / 8 and the rounding of mul below 2^-10.
+  // Reduction of a sum s, |s| < 2^50 (l <= 1280), by recip20: with off a multiple of q of at least 2^50 and
+  // below 2^50 + 2^31, s + off is in [0, 2^51 + 2^31)
   uint64_t off[3];
   uint32_t mul[3];
   int sh[3];
@@ -506,8 +505,8 @@ int mac_launch(Ctx &c, const SchemeArgs &sa, const uint32_t *d_v, size_t vstride
     for (int j = 0; j < 3; ++j) {
       const uint64_t q = sa.ra.q[j];
       a.off[j] = ((1ull << 50) / q + 1) * q;
-      while (((1ull << 53) << a.sh[j]) / q < (1ull << 32)) ++a.sh[j];
-      a.mul[j] = (uint32_t)(((1ull << 52) << a.sh[j]) / q);
+      a.mul[j] = recip20(q).mul;
+      a.sh[j] = recip20(q).sh;
     }
     const long long tiles = (long long)nz * (3 * n / kMmaCols);
     const long long per_key_tile = std::max(1LL, std::min(tiles, (long long)c.num_sms / a.key_tiles));

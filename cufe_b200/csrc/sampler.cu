@@ -1186,7 +1186,7 @@ static uint32_t mean_overshoot(int sig) { return sig == 0 ? 156100u : (sig == 1 
 
 // Refills precomputed for `calls` consecutive calls of n samples.  A call consumes r refills,
 // the first whose accepted total reaches n; E[r] = (n + overshoot) / mu < n / mu + 1 (the
-// overshoot averages below 1.4 samples), and over many calls sum(r) has variance about
+// overshoot averages less than half of mu: mean_overshoot), and over many calls sum(r) has variance about
 // calls n v / mu^3 (renewal count).  The range is calls (n / mu + 1) plus 12 of those
 // standard deviations plus 64.  Against the exact distribution of r (dynamic programming
 // over the measured accept-count histogram), that is at least 13 standard deviations of

@@ -50,6 +50,22 @@ __device__ __forceinline__ void load16_own(const uint32_t *p, uint32_t (&a)[16])
 }
 __device__ __forceinline__ void store16(uint32_t *p, const uint32_t (&a)[16]) { store_vec<16>(p, a); }
 
+// floor(x / q), or one less, for x < 2^51 + 2^31 without a 64-bit multiplication: (x >> 20) mul >> (32 + sh), mul =
+// floor(2^(52 + sh) / q) of 32 bits.  The cut-off bits are worth less than 2^20 / q; the rounding of mul, times
+// x >> 20 < 2^31 + 2^11, less than (1 + 2^-20) / 2^(1 + sh).
+struct Recip20 {
+  uint32_t mul;
+  int sh;
+};
+constexpr Recip20 recip20(uint64_t q) {
+  int sh = 0;
+  while (((1ull << 53) << sh) / q < (1ull << 32)) ++sh;
+  return Recip20{(uint32_t)(((1ull << 52) << sh) / q), sh};
+}
+constexpr bool recip20_ok(uint64_t q) {  // together at most 1/4
+  return ((1ull << 52) << recip20(q).sh) / q < (1ull << 32) && q >= (8ull << 20) && recip20(q).sh >= 3;
+}
+
 struct SchemeArgs {
   RingArgs ra;
   int l;
