@@ -214,20 +214,20 @@ def cpu_baseline_sample(x, y, seeds2, setup_seeds, nproc, steps=2):
 CAND_S3_DRAM_BYTES_PER_REFILL = (1.231872e6 + 530.28736e6) / (16 * 1044352)
 
 
-# algorithmic HBM bytes per launch of each kernel at this workload (batch B)
 def on_main(prof):
     """the kernel groups whose times are device time alone: an encryption's sigma_2 chain runs on a second
     stream, and the events around its groups also span their wait for SMs"""
     return {k: v for k, v in prof.items() if k not in ("sample_cand_s2", "sample_walk")}
 
 
+# algorithmic HBM bytes per launch of each kernel at this workload (batch B)
 def algorithmic_bytes(kernel, B, refills3):
     poly = 3 * N * 4
     return {
         "sample_cand_s3": refills3 * B * 35,           # 8 low words, accept mask, bit-32/sign bytes
         "sample_scatter": refills3 * B * 35 + B * L * poly,  # candidates and masks; f_i residues
         "encrypt_intt": (L + 1) * poly + B * (L * poly + (L + 1) * poly),  # mpk once, f_i, ciphertexts
-        "decrypt_mac": B * (L + 1) * poly + B * poly,    # ciphertexts read, partial sums written
+        "decrypt_mac": B * (L + 1) * poly + B * poly,    # ciphertexts read, sums written
         "decode": B * poly + B * N * 4,
     }.get(kernel)
 
@@ -503,7 +503,7 @@ def gpu_arm(args):
                         "that every encryption carries"},
             "tuning": {"encrypt_instances_per_group": enc_group, "encrypt_ms_by_group": enc_ms,
                        "coef0_form": c0_form, "coef0_ms_by_form": c0_tune_ms,
-                       "coef0_forms": ["per pair", "64x32", "64x64", "32x32", "32x64"],
+                       "coef0_forms": ["per pair", "tensor cores", "64x64", "32x32", "32x64"],
                        "note": "shapes chosen by the library's tuners (cufe_tune_encrypt, cufe_tune_decrypt_coef0) "
                                "on this workload before timing; every form gives the same bits"},
             "e2e": e2e, "gpu_launches": launches, "roofline": roof,
@@ -1114,7 +1114,7 @@ def svm_workload(args):
             "warmup": args.warmup, "ms_per_step": ms / args.steps, "higher_is_better": True, "dtype": "uint32",
             "data": "synthetic", "bit_exact": ok, "sv_keys_s": keys_s,
             "tuning": {"coef0_form": svm_form, "coef0_ms_by_form": svm_form_ms,
-                       "coef0_forms": ["per pair", "64x32", "64x64", "32x32", "32x64"]},
+                       "coef0_forms": ["per pair", "tensor cores", "64x64", "32x32", "32x64"]},
             "config": {"workload": "1,000 test vectors (a1a-shaped) x 500 support vectors, encrypt + predict per step",
                        "n": n, "l": l, "test_vectors": ntest, "support_vectors": nsv},
             "gpu_launches": svm_launches, "kernels_ms": {k: {"launches": v[0], "ms": v[1]} for k, v in sorted(prof.items(), key=lambda kv: -kv[1][1])},

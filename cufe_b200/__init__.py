@@ -355,7 +355,7 @@ class Context:
         return ch.value, list(ms)
 
     def decrypt_coef0_form(self, form, ct, y, sky, y_signed=False, d0=None, out=None, stream=None):
-        """decrypt_coef0 in a given form (0 per pair, 1..4 tile shapes)"""
+        """decrypt_coef0 in a given form (0 per pair, 1 on the tensor cores, 2..4 integer tile shapes)"""
         nct, nkeys = ct.shape[0], y.shape[0]
         out = _dev((nct, nkeys), self.dev) if out is None else out
         _check(lib().cufe_decrypt_coef0_form(self.h, form, nct, _ptr(ct), nkeys, _ptr(y), int(y_signed), _ptr(sky),

@@ -7,7 +7,7 @@
 //    the accepted candidates in order and drops the rest of its last refill.  The stream is
 //    sequential by construction, so it is computed in three parallel phases: (1) every
 //    refill's 8 candidates and accept mask for a generous refill range (the AES work, one
-//    thread per refill), (2) a walk per stream over the accept counts that finds where each
+//    thread per refill), (2) a search per stream over the accept counts that finds where each
 //    call starts (each call starts at a fresh refill), (3) a
 //    scatter of the accepted candidates to their coefficient positions as residues.
 //  * GPU mapping (src/sample_gpu.cu, src/AES.cuh): thread t of polynomial p owns coefficients
