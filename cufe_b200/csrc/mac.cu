@@ -425,6 +425,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
       ch = 0;
       // epilogue: the thread's key (TMEM lane) by 16 coefficients, 8 at a time
       if (live) live = mbar_wait(bar, (uint32_t)(s >> 1) & 1u);
+      __syncwarp();  // the wait's loop may leave a warp's threads apart, and the accumulator loads take whole warps
       umma_fence_after();
       const int z = tile / per_z, col = (tile - z * per_z) * kMmaCols, m = col / n;
       tile += stride;
