@@ -421,6 +421,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
                   umma_smem_desc(stage + 2 * j * kMmaLboB, kMmaLboB), kMmaIdesc, ch > 0 || j > 0);
         umma_commit(bar);
       }
+      __syncwarp();  // thread 0's warp waits for the products only when they have been issued
       if (++ch < chunks) return;
       ch = 0;
       // epilogue: the thread's key (TMEM lane) by 16 coefficients, 8 at a time
