@@ -3,13 +3,14 @@
 // for keys k, RNS moduli m and coefficients j, with v = msk (src/rlwe_sife.c:215-245) or the
 // ciphertexts z (the sum of src/rlwe_sife.c:248-278).
 //
-// Two kernels.  k_mac_few streams v once per KCH keys and is bound by memory; k_mac_mma is the
-// product of many keys with v on the tensor cores.  Before, every product was three integer
+// Three kernels.  k_mac_few streams v once per KCH keys and is bound by memory; k_mac_mma is the
+// product of many keys with v on the tensor cores; k_mac_short takes sums of a few rows.  Before, every product was three integer
 // instructions and v was read once per 4 keys (key generation) or per key (decryption).  B200,
 // us per call, before -> now: 1 key at n = 4096, l = 784 277 -> 13; 591 keys at l = 785 2034 -> 70;
 // the decryption of one ciphertext under 591 keys at n = 2048, l = 124 254 -> 100 (60 with its transforms read
 // where they lie and launched at once).
 #include <algorithm>
+#include <cmath>
 
 #include "ctx.h"
 #include "prof.h"
@@ -197,6 +198,39 @@ __global__ void __launch_bounds__(kFewThreads, KCH == 4 ? 2 : KCH == 2 ? 3 : 4)
   big = __syncthreads_or(big);
   if (!big && few_sums<KCH, false>(a, sa, sm, true)) return;
   few_sums<KCH, true>(a, sa, sm, false);
+}
+
+// ------------------------------------------------------------------ short sums
+
+// A thread sums one coefficient for four keys over all rows: no slices to add up and no packing, so the
+// shortest way through sums of a few rows, whatever the weights (Shoup products of their residues).
+constexpr int kShortRows = 128, kShortKeys = 4;
+__global__ void __launch_bounds__(256) k_mac_short(const __grid_constant__ FewArgs a, const __grid_constant__ SchemeArgs sa) {
+  __shared__ uint2 ys[kShortKeys][kShortRows];  // (y, floor(y 2^32 / q))
+  const int n = sa.ra.n, l = sa.l, z = blockIdx.y / 3, m = blockIdx.y - 3 * z, k0 = blockIdx.z * kShortKeys;
+  const uint32_t q = sa.ra.q[m];
+  const uint64_t mu = sa.mu[m];
+  for (int t = threadIdx.x; t < kShortKeys * l; t += blockDim.x) {
+    const int kk = t / l, i = t - kk * l;
+    const uint32_t w = k0 + kk < a.nkeys ? y_residue(a.y[(size_t)(k0 + kk) * l + i], a.y_signed, q, mu) : 0u;
+    const uint64_t ws = (uint64_t)w << 32, qe = __umul64hi(ws, mu);  // floor(ws / q) or one less
+    ys[kk][i] = make_uint2(w, (uint32_t)qe + (uint32_t)(ws - qe * q >= q));
+  }
+  __syncthreads();
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= n) return;
+  const uint32_t *v = a.v + z * a.vstride + (size_t)m * n + j;
+  uint64_t acc[kShortKeys] = {};
+#pragma unroll 8
+  for (int i = 0; i < l; ++i) {
+    const uint32_t x = __ldg(v + (size_t)i * 3 * n);
+#pragma unroll
+    for (int kk = 0; kk < kShortKeys; ++kk) acc[kk] += shoup_lazy(x, ys[kk][i].x, ys[kk][i].y, q);
+  }
+  uint32_t *o = a.out + ((size_t)(z * (size_t)a.nkeys + k0) * 3 + m) * n + j;
+#pragma unroll
+  for (int kk = 0; kk < kShortKeys; ++kk)
+    if (k0 + kk < a.nkeys) o[(size_t)kk * 3 * n] = mod_u64(acc[kk], mu, q);
 }
 
 // ------------------------------------------------------------------ many keys
@@ -482,27 +516,64 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
 
 }  // namespace
 
-// Which kernel: estimated us on a B200, fitted to the measurements below.  Tensor cores: the CTAs walk
-// their coefficient tiles, 1.25 us per 128 slots and 1.5 per epilogue, whatever the number of keys
-// up to 128 per tile; streamed: v read at about 3.5 TB/s per 4 keys.  One or two keys are always
-// streamed.  us (streamed | tensor cores) at n, l, ciphertexts, keys: 4096, 37, 21, 3: 21 | 78; 2048, 53,
-// 26, 3: 22 | 52; 4096, 123, 36, 4: 70 | 127; 4096, 65, 17, 8: 43 | 66; 4096, 784, 4, 4: 60 | 65; 1024, 100, 30,
-// 6: 32 | 33; 4096, 100, 8, 16: 54 | 36; 4096, 784, 1, 8: 49 | 27; 1024, 40, 1, 32: 26 | 8.
-static bool use_mma(const Ctx &c, int nz, int nkeys) {
-  if (nkeys <= 2 || c.n < kMmaCols || c.l > kMmaMaxL) return false;
-  const int key_tiles = (nkeys + kMmaKeys - 1) / kMmaKeys;
-  const long long tiles = (long long)nz * (3 * c.n / kMmaCols);
-  const long long ctas = std::max(1LL, (long long)c.num_sms / key_tiles), rounds = (tiles + ctas - 1) / ctas;
-  const double mma = 6.0 + (double)rounds * (1.25 * ((c.l + kMmaK - 1) / kMmaK) + 1.5);
-  const double few = ((nkeys + 3) / 4) * (5.0 + (double)nz * c.l * 12.0 * c.n / 3.5e6);
-  return mma < few;
+// Coefficients / 4 of a streamed CTA.  About 64 rows or more per slice; fewer, and so more slices and CTAs, while
+// there are not two CTAs per SM and, with three keys or more, whose slices cost more to add up, more than the eight rows that
+// are in flight at once (1 key at n = 4096, l = 784: 12.5 us with 384 CTAs, 16.6 with 192; 3 keys at l = 8: 6 us in one slice, 10 in 32).
+static int few_lanes(const Ctx &c, int nz, int keys, int groups) {
+  int lanes = 256;
+  while (lanes > 16 && c.l / (kFewThreads / lanes) >= 128) lanes /= 2;
+  lanes = std::min(lanes, c.n / 4);
+  while (lanes > 8 && (keys < 3 || c.l > 8 * (kFewThreads / lanes)) &&
+         (long long)nz * groups * 3 * c.n / (4 * lanes) < 2LL * c.num_sms)
+    lanes /= 2;
+  return lanes;
+}
+
+// Which kernel, of three keys or more (fewer are streamed): the least of these estimates, us on a B200.
+//   streamed: waves of two CTAs per SM, each 5 to 7.5 by its columns and 1.6 per further 8 rows of a slice; and v read at
+//     3.5 TB/s per 4 keys;
+//   tensor cores: the CTAs walk their coefficient tiles, 1.25 per 128 slots and 1.5 per epilogue, whatever
+//     the number of keys up to 128 per tile;
+//   short: 2.85 M products a us behind a latency of the rows; below 32 rows, and in rings below 64.
+// us measured (streamed | tensor cores | short) at n, l, ciphertexts, keys: 4096, 37, 21, 3: 21 | 78; 2048, 53,
+// 26, 3: 22 | 52; 4096, 123, 36, 4: 70 | 127; 4096, 65, 17, 8: 43 | 66; 4096, 784, 4, 4: 60 | 65; 4096, 100, 8, 16:
+// 54 | 36; 4096, 784, 1, 8: 30 | 24; 4096, 100, 1, 12: 11 | 9; 4096, 32, 1, 8: 6 | 9; 1024, 100, 1, 32: 10 | 6; 1024,
+// 8, 1, 16: 7 | 6 | 4; 4096, 8, 1, 16: 7 | 9 | 4; 4096, 16, 1, 64: 12 | 9 | 10; 4096, 8, 1, 600: 46 | 25 | 42.
+enum MacKernel { kMacFew, kMacMma, kMacShort };
+static MacKernel choose_kernel(const Ctx &c, int nz, int nkeys) {
+  if (nkeys < 2) return kMacFew;
+  const int groups = (nkeys + 3) / 4, lanes = few_lanes(c, nz, nkeys, groups), slices = kFewThreads / lanes;
+  const double ctas = (double)nz * groups * 3 * c.n / (4 * lanes), waves = ctas / (2 * c.num_sms);
+  const double per_wave = 5.0 + 2.5 * lanes / 256 + 1.6 * (((c.l + slices - 1) / slices + 7) / 8 - 1);
+  double best = std::max(0.8 + (waves < 4 ? std::ceil(waves) : waves) * per_wave,
+                         5.0 + (double)groups * nz * c.l * 12.0 * c.n / 3.5e6);
+  MacKernel kernel = kMacFew;
+  if (nkeys == 2) best = 4.6;  // streamed in short sums; never on the tensor cores
+  if (nkeys > 2 && c.n >= kMmaCols && c.l <= kMmaMaxL) {
+    const int key_tiles = (nkeys + kMmaKeys - 1) / kMmaKeys;
+    const long long tiles = (long long)nz * (3 * c.n / kMmaCols);
+    const long long each = std::max(1LL, (long long)c.num_sms / key_tiles), rounds = (tiles + each - 1) / each;
+    const double us = 4.0 + (double)rounds * (1.25 * ((c.l + kMmaK - 1) / kMmaK) + 1.5);
+    if (us < best) best = us, kernel = kMacMma;
+  }
+  if ((c.l < 32 || (c.n < kMmaCols && c.l <= kShortRows)) && nz <= 21845 && groups < 65536 &&
+      2.5 + 0.16 * c.l + (double)nz * groups * 12.0 * c.n * (c.l + 7) / 2.85e6 < best)
+    kernel = kMacShort;
+  return kernel;
 }
 
 int mac_launch(Ctx &c, const SchemeArgs &sa, const uint32_t *d_v, size_t vstride, int nz, const uint32_t *d_y,
                int y_signed, int nkeys, uint32_t *d_out, cudaStream_t s) {
   const int n = c.n, l = c.l;
   const int vec = ((reinterpret_cast<uintptr_t>(d_v) | reinterpret_cast<uintptr_t>(d_out)) & 15u) == 0 && vstride % 4 == 0;
-  if (use_mma(c, nz, nkeys)) {
+  const MacKernel kernel = choose_kernel(c, nz, nkeys);
+  if (kernel == kMacShort) {
+    const FewArgs a{d_v, d_y, vstride, d_out, y_signed, nkeys, 0, 0};
+    note_launch(), k_mac_short<<<dim3((n + 255) / 256, 3u * nz, (nkeys + kShortKeys - 1) / kShortKeys), 256, 0, s>>>(a, sa);
+    CUFE_CUDA(cudaGetLastError());
+    return CUFE_OK;
+  }
+  if (kernel == kMacMma) {
     MmaArgs a{d_v, vstride, d_y, y_signed, nkeys, nz, (nkeys + kMmaKeys - 1) / kMmaKeys, vec, d_out, {}};
     for (int j = 0; j < 3; ++j) {
       const uint64_t q = sa.ra.q[j];
@@ -522,12 +593,7 @@ int mac_launch(Ctx &c, const SchemeArgs &sa, const uint32_t *d_v, size_t vstride
   }
   const int kch = nkeys >= 3 ? 4 : nkeys;
   const int groups = (nkeys + kch - 1) / kch;
-  // About 64 rows or more per slice; fewer, and so more slices and CTAs, while there are not two CTAs
-  // per SM (1 key at n = 4096, l = 784: 12.5 us with 384 CTAs, 16.6 with 192).
-  int lanes = 256;
-  while (lanes > 16 && l / (kFewThreads / lanes) >= 128) lanes /= 2;
-  lanes = std::min(lanes, n / 4);
-  while (lanes > 8 && (long long)nz * groups * 3 * n / (4 * lanes) < 2LL * c.num_sms) lanes /= 2;
+  const int lanes = few_lanes(c, nz, nkeys, groups);
   const dim3 grid((unsigned)(3 * n / (4 * lanes)), (unsigned)nz, (unsigned)groups);
   const FewArgs a{d_v, d_y, vstride, d_out, y_signed, nkeys, lanes, vec};
   note_launch();
