@@ -1572,7 +1572,15 @@ int ctx_decrypt_coef0(Ctx &c, int nct, const uint32_t *d_ct, int nkeys, const ui
   // 219 | 26 | 223, 1,000 x 500 8178 | 88 | 1261; n = 4096, l = 784: 64 x 8 33 | 30 | 411
   const long long pairs = (long long)nct * nkeys;
   const bool mma = !d_d0 && coef0_mma_ok(c);
-  if (it == c.coef0_form.end() && nct >= 1 && nkeys >= kCoef0TiledMinKeys && pairs < (mma ? 1024 : 12800)) {
+  // Where the tensor cores cannot have them: 5.2 ns a pair, 5.1 ps a pair and coefficient and 16 ps a pair and
+  // slot of l (whose ciphertext words lie far apart), against a tile's latency, 120 ns a coefficient and 140 a slot, times the
+  // tiles of an SM; tiles where they save a tenth.
+  // us (per pair | tiles), keys x ciphertexts, n = 2048, l = 124: 64 x 32 43 | 218, 200 x 64 219 | 223; n = 16, l = 8: 40 x
+  // 130 43 | 14; n = 256, l = 784: 20 x 600 222 | 157
+  const double rounds = std::max(1.0, 3.0 * ((nct + 63) / 64) * ((nkeys + 31) / 32) / c.num_sms);
+  const bool few = mma ? pairs < 1024
+                       : 0.9 * pairs * (5.2e-3 + 5.1e-6 * c.n + 1.6e-5 * c.l) < (0.12 * c.n + 0.14 * c.l) * rounds;
+  if (it == c.coef0_form.end() && nct >= 1 && nkeys >= kCoef0TiledMinKeys && few && pairs <= 0x7fffffffLL) {
     // many keys, few pairs: per pair, but the decodes by one kernel instead of one thread per CTA
     uint32_t *d0 = d_d0;
     if (!d0) {

@@ -162,7 +162,7 @@ int cufe_decrypt_coef0(cufe_ctx *ctx, int nct, const uint32_t *d_ct, int nkeys, 
  *   cufe_tune_decrypt_coef0: for (nct, nkeys), form 0 = one CTA per (ciphertext, key) pair, 1 = the
  *     product on the tensor cores (with d_d0, rings below 64 or n + l above 8192: the tiled product at
  *     64x32), 2..4 = the tiled product at 64x64, 32x32, 32x64 ciphertexts x keys per CTA (fixed rule:
- *     1 from 1024 pairs, or 12800 where it is the tiled product and there are 32 keys; else form 0);
+ *     1 from 1024 pairs, or with 32 keys where it is the tiled product and by estimate the quicker; else form 0);
  *     choice = the form, ms[5];
  *   cufe_decrypt_coef0_form: cufe_decrypt_coef0 in the given form (tests, comparisons). */
 int cufe_tune_encrypt(cufe_ctx *ctx, int batch, const uint32_t *d_x, const uint32_t *d_mpk, const uint8_t *seeds2,
